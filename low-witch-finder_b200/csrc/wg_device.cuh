@@ -156,13 +156,20 @@ __device__ __forceinline__ uint64_t lcg_long(uint64_t &st) {
     return (hi << 32) + (uint64_t)lo;
 }
 
-// Chunk of the swamp hut in region (rx, rz): spacing 32, separation 8.
+// Chunk of the swamp hut in region (rx, rz): spacing 32, separation 8.  Both draws straight on; the
+// JDK's re-draw (a 31-bit value of 2147483640 or more, 8 in 2^31) starts over with the exact loop.
 __device__ __forceinline__ void hut_chunk(uint64_t seed, int rx, int rz, int salt, int &cx, int &cz) {
-    uint64_t s = (uint64_t)(int64_t)rx * 341873128712ULL + (uint64_t)(int64_t)rz * 132897987541ULL + seed +
-                 (uint64_t)(int64_t)salt;
-    uint64_t st = (s ^ kLcgMul) & kLcgMask;
-    int j = lcg_int(st, 24);
-    int k = lcg_int(st, 24);
+    constexpr uint32_t kLimit = 2147483640u;
+    const uint64_t s = (uint64_t)(int64_t)rx * 341873128712ULL + (uint64_t)(int64_t)rz * 132897987541ULL + seed +
+                       (uint64_t)(int64_t)salt;
+    const uint64_t s1 = (s ^ kLcgMul) * kLcgMul + 0xBULL, s2 = s1 * kLcgMul + 0xBULL;   // low 48 bits matter
+    const uint32_t u1 = (uint32_t)(s1 >> 17) & 0x7FFFFFFFu, u2 = (uint32_t)(s2 >> 17) & 0x7FFFFFFFu;
+    int j = (int)(u1 % 24u), k = (int)(u2 % 24u);
+    if (u1 >= kLimit || u2 >= kLimit) {
+        uint64_t st = (s ^ kLcgMul) & kLcgMask;
+        j = lcg_int(st, 24);
+        k = lcg_int(st, 24);
+    }
     cx = rx * 32 + j;
     cz = rz * 32 + k;
 }

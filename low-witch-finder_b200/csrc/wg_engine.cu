@@ -19,8 +19,41 @@
 
 using namespace wg;
 
-// Regions per unit window: a whole seed when its rect is small, else 2048-region windows.
-uint32_t wg::window_for(uint64_t n_regions) { return n_regions <= 4096 ? (uint32_t)n_regions : 2048u; }
+Tiling wg::tile_rect(uint64_t rw, uint64_t rh, uint64_t target) {
+    constexpr uint64_t kMaxSide = 1023;   // a hut's chunk offset in its tile stays below 2^15
+    target = std::max<uint64_t>(target, 1);
+    uint64_t tw = rw, th = rh;
+    if (rw > target / rh || rw > kMaxSide || rh > kMaxSide) {
+        const uint64_t side = std::max<uint64_t>(1, (uint64_t)std::sqrt((double)target));
+        tw = std::min<uint64_t>({rw, side, kMaxSide});
+        th = std::min<uint64_t>({rh, std::max<uint64_t>(1, target / tw), kMaxSide});
+        tw = std::min<uint64_t>({rw, std::max<uint64_t>(1, target / th), kMaxSide});   // a low rect: wider tiles
+        tw = (rw + (rw + tw - 1) / tw - 1) / ((rw + tw - 1) / tw);                     // of equal size
+        th = (rh + (rh + th - 1) / th - 1) / ((rh + th - 1) / th);
+    }
+    Tiling t;
+    t.tw = (uint32_t)tw;
+    t.th = (uint32_t)th;
+    t.ntx = (uint32_t)((rw + tw - 1) / tw);
+    t.n_win = t.ntx * ((rh + th - 1) / th);
+    return t;
+}
+
+// Whether a request's units take the one-CTA kernel, and its tiles.  Many regions per seed: yes, a
+// tile's two table builds (13,000 warp instructions) are then a small part of it, and the ladder and
+// the entrance gate find the seed's tables built.  Few units for the GPU (sm_count * 3 CTAs are
+// resident): yes too, in tiles small enough to give every CTA one, since the call then takes one
+// build and one evaluation of latency instead of three.  Otherwise 16 units share a CTA.
+static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, bool single_biome, int sm_count, bool &cta) {
+    const uint64_t n_regions = rw * rh, slots = (uint64_t)sm_count * 3;
+    const double total = (double)n_seeds * (double)n_regions;
+    cta = !single_biome && (n_regions >= kUnitCtaRegions || n_seeds <= 4 * slots);
+    if (!cta) return tile_rect(rw, rh, n_regions <= 4096 ? n_regions : 2048);
+    // one tile per resident CTA up to 2,048 regions each, then several waves of larger ones
+    uint64_t target = (uint64_t)(total / (double)slots) + 1;
+    if (target > 2048) target = std::max<uint64_t>(2048, target / 8);
+    return tile_rect(rw, rh, std::min<uint64_t>(std::max<uint64_t>(target, 32), kUnitCtaMax));
+}
 
 // Climate evaluation steps (see ClimateStep): the tiered erosion sequence
 // (engine/tools/lysh/src/noise.c:387-459) followed by plain y=0 DoublePerlin samples of
@@ -143,7 +176,8 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
             "memset hist");
     WG_CUDA(cudaEventRecord(eng->kev[0], eng->stream), "event");
     // one region per unit: the climate tables are built lazily, breadth first
-    if (spot_path(a.jobs != nullptr, a.win, a.codes != nullptr, a.single_biome != 0)) {
+    const bool spots = !a.unit_cta && spot_path(a.jobs != nullptr, (uint64_t)a.tw * a.th, a.codes != nullptr, a.single_biome != 0);
+    if (spots) {
         if (!eng->spot_counts) {
             WG_CUDA(cudaMalloc(&eng->spot_items[0], sizeof(SpotItem) * kSpotUnits), "alloc");
             WG_CUDA(cudaMalloc(&eng->spot_items[1], sizeof(SpotItem) * kSpotUnits), "alloc");
@@ -151,31 +185,40 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
         }
         launch_spot_climate(a, eng->spot_items[0], eng->spot_items[1], eng->spot_counts, kSpotUnits, eng->sm_count,
                             eng->stream);
+    } else if (a.unit_cta) {
+        launch_unit(a, eng->stream);
     } else {
         launch_climate(a, eng->stream);
     }
     WG_CUDA(cudaEventRecord(eng->kev[1], eng->stream), "event");
-    launch_entrance(a, 0, eng->stream);
+    if (!a.unit_cta) launch_entrance(a, 0, eng->stream);
     WG_CUDA(cudaEventRecord(eng->kev[2], eng->stream), "event");
-    launch_ladder(a, 0, eng->stream);
+    if (!a.unit_cta) launch_ladder(a, 0, eng->stream);
     WG_CUDA(cudaEventRecord(eng->kev[3], eng->stream), "event");
     WG_CUDA(cudaGetLastError(), "kernel launch");
-    WG_CUDA(cudaMemcpyAsync(eng->h_counters, eng->counters, sizeof(uint32_t) * CNT_WORDS, cudaMemcpyDeviceToHost,
-                            eng->stream),
-            "copy counters");
-    WG_CUDA(cudaMemcpyAsync(eng->h_hist, eng->hist, sizeof(unsigned long long) * (P1_KINDS + kTiers),
-                            cudaMemcpyDeviceToHost, eng->stream),
-            "copy hist");
-    WG_CUDA(cudaStreamSynchronize(eng->stream), "batch");
+    for (int pass = 0;; pass++) {
+        WG_CUDA(cudaMemcpyAsync(eng->h_counters, eng->counters, sizeof(uint32_t) * CNT_WORDS, cudaMemcpyDeviceToHost,
+                                eng->stream),
+                "copy counters");
+        WG_CUDA(cudaMemcpyAsync(eng->h_hist, eng->hist, sizeof(unsigned long long) * (P1_KINDS + kTiers),
+                                cudaMemcpyDeviceToHost, eng->stream),
+                "copy hist");
+        WG_CUDA(cudaStreamSynchronize(eng->stream), "batch");
+        // candidates past a unit's own list go through the ladder kernel (seldom any)
+        if (!a.unit_cta || pass || !eng->h_counters[CNT_DEEP] || eng->h_counters[CNT_OVERFLOW]) break;
+        launch_ladder(a, 0, eng->stream);
+        WG_CUDA(cudaEventRecord(eng->kev[3], eng->stream), "event");
+        WG_CUDA(cudaGetLastError(), "kernel launch");
+    }
     st.batches++;
     for (int k = 0; k < 3; k++) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, eng->kev[k], eng->kev[k + 1]);
         st.kernel_ms[k] += ms;
-        st.kernel_launches[k]++;
+        if (k == 0 || !a.unit_cta) st.kernel_launches[k]++;
     }
     if (eng->h_counters[CNT_OVERFLOW]) {
-        if (n_units <= 32) return eng->fail(WG_ERR_CAPACITY, "phase-1 work list full even for 32 units");
+        if (n_units <= (a.unit_cta ? 1u : 32u)) return eng->fail(WG_ERR_CAPACITY, "phase-1 work list full even for the smallest batch");
         st.retries++;
         uint32_t half = n_units / 2;
         int rc = run_batch(eng, proto, unit0, half, sink, st);
@@ -187,7 +230,7 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
     st.climate_survivors += eng->h_counters[CNT_SURVIVORS];
     st.rechecks += eng->h_counters[CNT_RECHECK];
     st.records += eng->h_counters[CNT_RECORDS];
-    st.deep_candidates += eng->h_counters[CNT_DEEP];
+    st.deep_candidates += eng->h_counters[CNT_DEEP] + eng->h_counters[CNT_DEEP_UNIT];
     uint32_t nf = eng->h_counters[CNT_FINAL];
     if (nf) {
         if (sink.host) {
@@ -234,14 +277,19 @@ int run_request(wg_engine *eng, const Request &rq, Sink &sink, wg_scan_stats &st
     if (rq.rx1 <= rq.rx0 || rq.rz1 <= rq.rz0 || rq.n_seeds == 0) return eng->fail(WG_ERR_ARG, "empty request");
     const uint64_t rw = (uint64_t)((int64_t)rq.rx1 - rq.rx0), rh = (uint64_t)((int64_t)rq.rz1 - rq.rz0);
     const uint64_t n_regions = rw * rh;
-    const uint32_t win = window_for(n_regions);
-    const uint64_t n_win = (n_regions + win - 1) / win;
+    const bool spot = spot_path(false, n_regions, rq.d_codes != nullptr, rq.opts.single_biome != 0);
+    bool cta = false;
+    const Tiling tiles = spot ? tile_rect(rw, rh, 1) : request_tiles(rw, rh, rq.n_seeds, rq.opts.single_biome != 0, eng->sm_count, cta);
+    const uint64_t n_win = tiles.n_win, win = tiles.win();
     const uint64_t units = rq.n_seeds * n_win;
 
     BatchArgs a = base_args(eng, rq.opts, rq.salt);
+    a.unit_cta = cta ? 1 : 0;
     a.seeds = rq.d_seeds;
     a.gen_base = rq.gen_base;
-    a.win = win;
+    a.tw = tiles.tw;
+    a.th = tiles.th;
+    a.ntx = tiles.ntx;
     a.n_win = n_win;
     a.n_regions = n_regions;
     a.rx0 = rq.rx0;
@@ -257,10 +305,11 @@ int run_request(wg_engine *eng, const Request &rq, Sink &sink, wg_scan_stats &st
     // spots shift the rect by their own regions: only plain requests are proved small
     a.small_coords = !rq.d_spot_s48 && coords_small(std::min(rq.rx0, rq.rz0), std::max(rq.rx1, rq.rz1) - 1ll) ? 1 : 0;
 
-    uint64_t per_batch = std::min<uint64_t>(kMaxUnits, std::max<uint64_t>(32, kWorkPerBatch / win));
-    if (rq.opts.single_biome)  // every region survives the climate stage
+    // the one-CTA kernel keeps no work lists in HBM, so its batches are eight times as large
+    uint64_t per_batch = std::min<uint64_t>(kMaxUnits, std::max<uint64_t>(32, kWorkPerBatch * (cta ? 8 : 1) / win));
+    if (rq.opts.single_biome && !cta)  // every region survives the climate stage
         per_batch = std::min<uint64_t>(per_batch, std::max<uint64_t>(32, kCapSurv / 2 / win));
-    if (spot_path(false, win, rq.d_codes != nullptr, rq.opts.single_biome != 0)) per_batch = kSpotUnits;
+    if (spot) per_batch = kSpotUnits;
     st.scanned = (int64_t)(rq.n_seeds * n_regions);
     // host seeds: the seeds of units [0, units_end) enqueued on the copy stream, ev_up after them
     uint64_t uploaded = 0;

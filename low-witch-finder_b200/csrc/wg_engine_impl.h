@@ -111,8 +111,19 @@ inline bool spot_path(bool jobs, uint64_t win, bool codes, bool single_biome) {
     return !jobs && win == 1 && !codes && !single_biome;
 }
 
-// Regions per unit window: a whole seed when its rect is small, else 2048-region windows.
-uint32_t window_for(uint64_t n_regions);
+// How a rect is cut into units (tiles of regions, wg_phase1.cuh).
+struct Tiling {
+    uint32_t tw = 1, th = 1, ntx = 1;
+    uint64_t n_win = 1;           // tiles per seed
+    uint64_t win() const { return (uint64_t)tw * th; }   // regions per tile at most
+};
+// Tiles of at most `target` regions (at least one), near square, of equal size up to rounding.
+Tiling tile_rect(uint64_t rw, uint64_t rh, uint64_t target);
+
+// Regions per seed from which a unit takes the one-CTA kernel (launch_unit).
+constexpr uint64_t kUnitCtaRegions = 2048;
+// Regions per unit of the one-CTA kernel at most.
+constexpr uint64_t kUnitCtaMax = 1ull << 16;
 
 // Job classes of the autotuner by regions per seed: <= 16, <= 256, <= 4096, more.
 constexpr uint64_t kJobClassMax[4] = {16, 256, 4096, ~0ull};
@@ -121,11 +132,12 @@ inline int job_class(uint64_t n_regions) {
     while (c < 3 && n_regions > kJobClassMax[c]) c++;
     return c;
 }
-// A job's window: the engine's tuned value for its class, else window_for's rule.
-inline uint32_t job_window(const wg_engine *eng, uint64_t n_regions) {
-    const uint32_t w = eng ? eng->tuned_win[job_class(n_regions)] : 0u;
-    if (!w) return window_for(n_regions);
-    return (uint32_t)(n_regions < w ? n_regions : w);
+// Regions per unit of a job: the engine's tuned value for its class, else the whole rect up to
+// 4,096 regions and 16,384-region tiles above.
+inline uint64_t job_window(const wg_engine *eng, uint64_t n_regions) {
+    const uint64_t w = eng ? eng->tuned_win[job_class(n_regions)] : 0u;
+    if (!w) return n_regions <= 4096 ? n_regions : 16384u;
+    return n_regions < w ? n_regions : w;
 }
 
 // One phase-1 request over one rect (wg_engine.cu).

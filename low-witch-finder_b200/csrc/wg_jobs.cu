@@ -30,7 +30,7 @@ constexpr uint64_t kMaxRectSide = 1ull << 24;
 constexpr uint64_t kStageSeeds = 1ull << 21;   // pinned staging for the seeds of small jobs (16 MiB)
 
 bool same_rules(const SchedJob &x, const SchedJob &y) {
-    return x.salt == y.salt && x.opts.mc_1_18_2 == y.opts.mc_1_18_2 && x.opts.single_biome == y.opts.single_biome &&
+    return x.unit_cta == y.unit_cta && x.salt == y.salt && x.opts.mc_1_18_2 == y.opts.mc_1_18_2 && x.opts.single_biome == y.opts.single_biome &&
            x.opts.pre_26_2 == y.opts.pre_26_2 && x.opts.large_biomes == y.opts.large_biomes;
 }
 
@@ -42,8 +42,8 @@ bool candidate_order(const Candidate &x, const Candidate &y) {
 
 // Whether a job's climate coordinates are proved inside maintainPrecision's identity range.
 bool job_small(const SchedJob &j) {
-    const int64_t rh = (int64_t)(j.n_regions / (uint64_t)j.rw);
-    return coords_small(std::min<int64_t>(j.rx0, j.rz0), std::max<int64_t>(j.rx0 + j.rw, j.rz0 + rh) - 1);
+    return coords_small(std::min<int64_t>(j.rx0, j.rz0),
+                        std::max<int64_t>((int64_t)j.rx0 + j.rw, (int64_t)j.rz0 + j.rh) - 1);
 }
 
 }  // namespace
@@ -58,11 +58,12 @@ int sched_job_init(SchedJob &j, const wg_job &spec, const wg_engine *eng) {
     j.rx0 = spec.rx0;
     j.rz0 = spec.rz0;
     j.rw = (int)rw;
+    j.rh = (int)rh;
     j.n_regions = rw * rh;
-    j.win = job_window(eng, j.n_regions);
-    j.n_win = (j.n_regions + j.win - 1) / j.win;
-    if (spec.n_seeds > ~0ull / j.n_win) return WG_ERR_ARG;
-    j.units = spec.n_seeds * j.n_win;
+    j.unit_cta = j.n_regions >= kUnitCtaRegions && !spec.opts.single_biome;
+    j.tiles = tile_rect(rw, rh, std::min<uint64_t>(job_window(eng, j.n_regions), j.unit_cta ? kUnitCtaMax : 4096));
+    if (spec.n_seeds > ~0ull / j.tiles.n_win) return WG_ERR_ARG;
+    j.units = spec.n_seeds * j.tiles.n_win;
     try {
         j.seeds.resize(spec.n_seeds);
     } catch (...) {
@@ -72,6 +73,24 @@ int sched_job_init(SchedJob &j, const wg_job &spec, const wg_engine *eng) {
     else
         for (uint64_t i = 0; i < spec.n_seeds; i++) j.seeds[i] = (int64_t)splitmix64(spec.gen_base + i);
     return WG_OK;
+}
+
+JobGeom job_geom(const SchedJob &j, uint64_t unit0, uint64_t first, uint64_t seed0) {
+    JobGeom g;
+    std::memset(&g, 0, sizeof g);
+    g.unit0 = unit0;
+    g.first = first;
+    g.seed0 = seed0;
+    g.n_win = j.tiles.n_win;
+    g.rx0 = j.rx0;
+    g.rz0 = j.rz0;
+    g.rw = j.rw;
+    g.rh = j.rh;
+    g.tw = j.tiles.tw;
+    g.th = j.tiles.th;
+    g.ntx = j.tiles.ntx;
+    g.max_height = j.max_height;
+    return g;
 }
 
 Scheduler::Scheduler(wg_engine *eng, uint64_t arena_seeds, uint64_t step_work)
@@ -190,7 +209,8 @@ int Scheduler::step(std::vector<SchedJob *> &finished, std::vector<SchedJob *> &
         if (units >= kMaxUnits || budget == 0 || misses >= 64) break;
         if (!same_rules(*j, lead) || (alone && j != alone)) continue;
         uint64_t k = std::min<uint64_t>(j->units - j->dispatched, kMaxUnits - units);
-        uint64_t kb = budget / j->win;
+        const uint64_t win = j->tiles.win();
+        uint64_t kb = budget / win;
         if (kb == 0) {
             if (units) {
                 misses++;
@@ -200,23 +220,11 @@ int Scheduler::step(std::vector<SchedJob *> &finished, std::vector<SchedJob *> &
         }
         misses = 0;
         k = std::min(k, kb);
-        JobGeom g;
-        std::memset(&g, 0, sizeof g);
-        g.unit0 = units;
-        g.first = j->dispatched;
-        g.seed0 = j->arena_off;
-        g.n_win = j->n_win;
-        g.n_regions = j->n_regions;
-        g.win = j->win;
-        g.rx0 = j->rx0;
-        g.rz0 = j->rz0;
-        g.rw = j->rw;
-        g.max_height = j->max_height;
-        table.push_back(g);
+        table.push_back(job_geom(*j, units, j->dispatched, j->arena_off));
         took.push_back(k);
         members.push_back(j);
         units += k;
-        budget -= std::min(budget, k * (uint64_t)j->win);
+        budget -= std::min(budget, k * win);
     }
     // the table: pinned host copy (rewritten only after the batch's closing sync) -> device
     if (table.size() > table_cap_) {
@@ -244,6 +252,7 @@ int Scheduler::step(std::vector<SchedJob *> &finished, std::vector<SchedJob *> &
     a.seeds = d_arena_;
     a.jobs = d_table_;
     a.n_jobs = (uint32_t)table.size();
+    a.unit_cta = lead.unit_cta ? 1 : 0;
     a.small_coords = 1;
     for (const SchedJob *j : members) a.small_coords &= job_small(*j) ? 1 : 0;
     found_.clear();
@@ -356,24 +365,13 @@ int jobs_on_device_queue(wg_engine *eng, std::vector<SchedJob> &js, uint64_t tot
             std::vector<JobGeom> table;
             std::vector<size_t> member;
             uint64_t units = 0;
-            uint32_t min_win = ~0u;
+            uint64_t min_win = ~0ull;
             for (size_t i = lead; i < js.size(); i++) {
                 if (done[i] || !same_rules(js[i], js[lead])) continue;
-                JobGeom g;
-                std::memset(&g, 0, sizeof g);
-                g.unit0 = units;
-                g.seed0 = off[i];
-                g.n_win = js[i].n_win;
-                g.n_regions = js[i].n_regions;
-                g.win = js[i].win;
-                g.rx0 = js[i].rx0;
-                g.rz0 = js[i].rz0;
-                g.rw = js[i].rw;
-                g.max_height = js[i].max_height;
-                table.push_back(g);
+                table.push_back(job_geom(js[i], units, 0, off[i]));
                 member.push_back(i);
                 units += js[i].units;
-                min_win = std::min(min_win, js[i].win);
+                min_win = std::min(min_win, js[i].tiles.win());
                 done[i] = 1;
             }
             e = cudaMemcpyAsync(d_table, table.data(), sizeof(JobGeom) * table.size(), cudaMemcpyHostToDevice,
@@ -386,6 +384,7 @@ int jobs_on_device_queue(wg_engine *eng, std::vector<SchedJob> &js, uint64_t tot
             a.seeds = d_seeds;
             a.jobs = d_table;
             a.n_jobs = (uint32_t)table.size();
+            a.unit_cta = js[lead].unit_cta ? 1 : 0;
             a.small_coords = 1;
             for (size_t k : member) a.small_coords &= job_small(js[k]) ? 1 : 0;
             std::vector<Candidate> found;

@@ -20,10 +20,11 @@ struct SchedJob {
     wg_opts opts{};
     int salt = 0;
     int max_height = 0;
-    int rx0 = 0, rz0 = 0, rw = 0;
+    int rx0 = 0, rz0 = 0, rw = 0, rh = 0;
     std::vector<int64_t> seeds;     // host copy (a generator job is expanded at submit)
-    uint64_t n_regions = 0, n_win = 0, units = 0;
-    uint32_t win = 0;
+    Tiling tiles;
+    uint64_t n_regions = 0, units = 0;
+    bool unit_cta = false;          // its units take the one-CTA kernel
     uint64_t dispatched = 0;        // units handed to batches so far
     uint64_t arena_off = ~0ull;     // first seed in the device seed arena (~0: not admitted)
     std::vector<Candidate> found;   // survivors so far; seed_index = position in the job
@@ -32,13 +33,15 @@ struct SchedJob {
     uint64_t batch_jobs = 0;        // most jobs that shared a batch with this one
     Clock::time_point t_submit, t_start, t_done;
 
-    uint64_t remaining_work() const { return (units - dispatched) * (uint64_t)win; }
+    uint64_t remaining_work() const { return (units - dispatched) * tiles.win(); }
 };
 
 // Fills a SchedJob's geometry and host seeds from a public job description (the window from the
 // engine's tuned settings when eng is given); WG_ERR_ARG if the job is empty or its rect is out
 // of range.
 int sched_job_init(SchedJob &j, const wg_job &spec, const wg_engine *eng);
+// The job-table entry of a job's units from `first` on.
+JobGeom job_geom(const SchedJob &j, uint64_t unit0, uint64_t first, uint64_t seed0);
 
 // Runs the admitted jobs of one engine batch by batch.  Not thread-safe: one thread drives it.
 class Scheduler {

@@ -92,7 +92,9 @@ extern "C" int wg_seed_check_noalloc(const int64_t *d_seeds, uint64_t gen_base, 
     a.gen_base = gen_base;
     a.unit0 = 0;
     a.n_units = n_seeds;
-    a.win = (uint32_t)(rw * rh);
+    a.tw = (uint32_t)rw;
+    a.th = (uint32_t)rh;
+    a.ntx = 1;
     a.n_win = 1;
     a.n_regions = rw * rh;
     a.rx0 = rx0;

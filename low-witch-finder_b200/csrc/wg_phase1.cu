@@ -63,9 +63,6 @@ void upload_tables(const NoiseSpec *specs, const ClimateStep *steps_normal, cons
 // ------------------------------------------------------------------------------------
 // helpers
 // ------------------------------------------------------------------------------------
-// Global seed index and region of a batch-local unit / window offset.
-__device__ __forceinline__ uint64_t unit_seed_index(const BatchArgs &a, uint32_t u) { return (a.unit0 + u) / a.n_win; }
-__device__ __forceinline__ uint64_t unit_window(const BatchArgs &a, uint32_t u) { return (a.unit0 + u) % a.n_win; }
 __device__ __forceinline__ uint64_t seed_value(const BatchArgs &a, uint64_t g) {
     if (a.spot_s48) return ((g & 0xFFFFull) << 48) | ((uint64_t)a.spot_s48[g >> 16] & 0xFFFFFFFFFFFFull);
     return a.seeds ? (uint64_t)a.seeds[g] : splitmix64(a.gen_base + g);
@@ -73,19 +70,34 @@ __device__ __forceinline__ uint64_t seed_value(const BatchArgs &a, uint64_t g) {
 // Rect origin of seed g (shifted to the seed's spot region in spots mode).
 __device__ __forceinline__ int rect_x0(const BatchArgs &a, uint64_t g) { return a.spot_rx ? a.rx0 + a.spot_rx[g >> 16] : a.rx0; }
 __device__ __forceinline__ int rect_z0(const BatchArgs &a, uint64_t g) { return a.spot_rz ? a.rz0 + a.spot_rz[g >> 16] : a.rz0; }
-// Everything about a batch-local unit: its seed, its window and the rect it walks.
+// Everything about a batch-local unit: its seed, and its tile in the rect it walks.
 struct UnitPos {
     uint64_t g;        // global seed index
-    uint64_t rbase;    // first region of the window (index into the rect, rz outer, rx inner)
-    uint32_t len;      // regions in the window
-    int rx0, rz0, rw;  // the rect the window lies in
+    uint64_t rbase;    // index in the rect (rz outer, rx inner) of the tile's first region
+    int rx, rz;        // the tile's first region
+    uint32_t tw, th;   // regions in the tile: tw x th
+    int rw;            // width of the rect
     int max_height;
+    // index in the rect of the region at a tile offset word (dx | dz << 16)
+    __device__ __forceinline__ uint64_t region(uint32_t off) const {
+        return rbase + (uint64_t)(off >> 16) * (uint64_t)rw + (off & 0xFFFFu);
+    }
 };
+__device__ __forceinline__ void unit_tile(UnitPos &p, uint64_t tile, uint32_t tw, uint32_t th, uint32_t ntx, int rx0,
+                                          int rz0, int rw, int rh) {
+    const uint32_t x = (uint32_t)(tile % ntx) * tw, z = (uint32_t)(tile / ntx) * th;
+    p.rx = rx0 + (int)x;
+    p.rz = rz0 + (int)z;
+    p.tw = min(tw, (uint32_t)rw - x);
+    p.th = min(th, (uint32_t)rh - z);
+    p.rw = rw;
+    p.rbase = (uint64_t)z * (uint64_t)rw + x;
+}
 __device__ __forceinline__ UnitPos unit_pos(const BatchArgs &a, uint32_t u) {
     UnitPos p;
+    const uint64_t ul = a.unit0 + u;
     if (a.jobs) {
         // the last table entry whose first global unit is <= this unit
-        const uint64_t ul = a.unit0 + u;
         uint32_t lo = 0, hi = a.n_jobs - 1;
         while (lo < hi) {
             const uint32_t mid = (lo + hi + 1) >> 1;
@@ -95,29 +107,14 @@ __device__ __forceinline__ UnitPos unit_pos(const BatchArgs &a, uint32_t u) {
         const JobGeom &j = a.jobs[lo];
         const uint64_t loc = ul - j.unit0 + j.first;
         p.g = j.seed0 + loc / j.n_win;
-        p.rbase = (loc % j.n_win) * j.win;
-        const uint64_t left = j.n_regions - p.rbase;
-        p.len = (uint32_t)(left < j.win ? left : j.win);
-        p.rx0 = j.rx0;
-        p.rz0 = j.rz0;
-        p.rw = j.rw;
+        unit_tile(p, loc % j.n_win, j.tw, j.th, j.ntx, j.rx0, j.rz0, j.rw, j.rh);
         p.max_height = j.max_height;
         return p;
     }
-    p.g = unit_seed_index(a, u);
-    p.rbase = unit_window(a, u) * a.win;
-    const uint64_t left = a.n_regions - p.rbase;
-    p.len = (uint32_t)(left < a.win ? left : a.win);
-    p.rx0 = rect_x0(a, p.g);
-    p.rz0 = rect_z0(a, p.g);
-    p.rw = a.rw;
+    p.g = ul / a.n_win;
+    unit_tile(p, ul % a.n_win, a.tw, a.th, a.ntx, rect_x0(a, p.g), rect_z0(a, p.g), a.rw, a.rh);
     p.max_height = a.max_height;
     return p;
-}
-// Region (rx, rz) of region index r of a unit's rect (rz outer, rx inner: search.c:148-149).
-__device__ __forceinline__ void unit_region_xz(const UnitPos &p, uint64_t r, int &rx, int &rz) {
-    rz = p.rz0 + (int)(r / (uint64_t)p.rw);
-    rx = p.rx0 + (int)(r % (uint64_t)p.rw);
 }
 
 __device__ __forceinline__ void note_code(const BatchArgs &a, uint64_t g, uint64_t r, int code, int tier) {
@@ -282,11 +279,10 @@ struct ClimateSmem {
     Real wsum[kClimateWarps][kWarpList];
     uint32_t surv[kUnits * kRecordCap];
     uint32_t cnt[kUnits];
-    uint32_t len[kUnits];                      // regions in the unit's window (0: past the batch)
+    uint32_t len[kUnits];                      // regions in the unit's tile (0: past the batch)
     uint64_t g[kUnits], rbase[kUnits], seed[kUnits];   // seed index, first region, world seed
-    uint32_t col0[kUnits];                     // column of the unit's first region in its rect row
-    int row0[kUnits];                          // rz of the unit's first region
-    int rx0u[kUnits];                          // rect x origin of the unit's seed
+    int rx[kUnits], rz[kUnits];                // the tile's first region
+    uint32_t tw[kUnits];                       // the tile's width
     uint32_t rwu[kUnits];                      // rect width of the unit's job
     unsigned int hist[P1_KINDS + kTiers];
     uint32_t grad[kGradWords];
@@ -311,18 +307,32 @@ __device__ void emit_single(const BatchArgs &a, uint32_t u, uint32_t off_in_win)
     }
 }
 
+// The tile offset word of region j (row by row) of unit iu, and its index in the rect.
+template <class Sm>
+__device__ __forceinline__ uint32_t tile_offset(const Sm &S, int iu, uint32_t j) {
+    const uint32_t dz = j / S.tw[iu];
+    return (j - dz * S.tw[iu]) | (dz << 16);
+}
+template <class Sm>
+__device__ __forceinline__ void note_region(const Sm &S, const BatchArgs &a, int iu, uint32_t j, int code, int tier) {
+    if (!a.codes) return;
+    const uint32_t w = tile_offset(S, iu, j);
+    note_code(a, S.g[iu], S.rbase[iu] + (uint64_t)(w >> 16) * S.rwu[iu] + (w & 0xFFFFu), code, tier);
+}
+
 template <class Sm>
 __device__ __forceinline__ void keep_survivor(Sm &S, const BatchArgs &a, int iu, uint32_t j) {
     uint32_t q = atomicAdd(&S.cnt[iu], 1u);
-    if (q < kRecordCap) S.surv[iu * kRecordCap + q] = j;
-    else emit_single(a, blockIdx.x * kUnits + (uint32_t)iu, j);
+    const uint32_t w = tile_offset(S, iu, j);
+    if (q < kRecordCap) S.surv[iu * kRecordCap + q] = w;
+    else emit_single(a, blockIdx.x * kUnits + (uint32_t)iu, w);
 }
 
 template <class Sm>
 __device__ __forceinline__ void climate_reject(Sm &S, const BatchArgs &a, int iu, uint32_t j, int code, int tier) {
     atomicAdd(&S.hist[code], 1u);
     if (tier >= 0) atomicAdd(&S.hist[P1_KINDS + tier], 1u);
-    note_code(a, S.g[iu], S.rbase[iu] + j, code, tier);
+    note_region(S, a, iu, j, code, tier);
 }
 
 // Erosion rejections are counted per thread in registers (16-bit fields, tiers 0-3 and 4-6) and
@@ -346,7 +356,7 @@ template <class Sm>
 __device__ __forceinline__ void erosion_reject(const Sm &S, const BatchArgs &a, TierCounts &tc, int iu, uint32_t j,
                                                int tier) {
     tc.add(tier);
-    note_code(a, S.g[iu], S.rbase[iu] + j, P1_EROSION, tier);
+    note_region(S, a, iu, j, P1_EROSION, tier);
 }
 
 // One y = 0 Perlin sample of climate step k for unit iu at climate point (xc, zc), in FP64 with
@@ -537,20 +547,20 @@ __global__ void __launch_bounds__(kThreadsA, 2) climate_kernel(BatchArgs a) {
     const uint32_t u = blockIdx.x * kUnits + (uint32_t)uu;
     const bool valid = u < a.n_units;
     UnitPos up{};
-    up.rw = 1;
+    up.tw = 1;
     if (valid) up = unit_pos(a, u);
     const uint64_t g = up.g;
     const uint64_t seed = valid ? seed_value(a, g) : 0;
-    const uint32_t len = valid ? up.len : 0;
+    const uint32_t len = valid ? up.tw * up.th : 0;
     if (tid < kUnits) {
         S.cnt[tid] = 0;
         S.len[tid] = len;
         S.g[tid] = g;
         S.rbase[tid] = up.rbase;
         S.seed[tid] = seed;
-        S.col0[tid] = (uint32_t)(up.rbase % (uint64_t)up.rw);
-        S.row0[tid] = up.rz0 + (int)(up.rbase / (uint64_t)up.rw);
-        S.rx0u[tid] = up.rx0;
+        S.rx[tid] = up.rx;
+        S.rz[tid] = up.rz;
+        S.tw[tid] = up.tw;
         S.rwu[tid] = (uint32_t)up.rw;
     }
     TierCounts tc;
@@ -605,9 +615,8 @@ __global__ void __launch_bounds__(kThreadsA, 2) climate_kernel(BatchArgs a) {
             const int qu = q % kUnits;
             const uint32_t j = c0 + (uint32_t)(q / kUnits);
             if (j >= S.len[qu]) continue;
-            const uint32_t t = S.col0[qu] + j;   // region offset from the unit's first row start
-            const uint32_t rw = S.rwu[qu];
-            const int rz = S.row0[qu] + (int)(t / rw), rx = S.rx0u[qu] + (int)(t % rw);
+            const uint32_t w = tile_offset(S, qu, j);
+            const int rz = S.rz[qu] + (int)(w >> 16), rx = S.rx[qu] + (int)(w & 0xFFFFu);
             int cx, cz;
             hut_chunk(S.seed[qu], rx, rz, a.salt, cx, cz);
             S.pos[q] = make_int2(cx, cz);
@@ -1108,7 +1117,7 @@ __device__ __forceinline__ uint64_t spot_point(const BatchArgs &a, uint32_t u, d
     const UnitPos up = unit_pos(a, u);
     const uint64_t seed = seed_value(a, up.g);
     int cx, cz;
-    hut_chunk(seed, up.rx0, up.rz0, a.salt, cx, cz);
+    hut_chunk(seed, up.rx, up.rz, a.salt, cx, cz);
     xc = (cx * 16 + 8) * 0.25;   // exact: an integer over 4
     zc = (cz * 16 + 8) * 0.25;
     return seed;
@@ -1327,7 +1336,7 @@ struct EntranceSmem {
     uint32_t emap[kEntList];              // tile survivor list: record << 16 | index in its record
     uint64_t rseed[kUnits], rg[kUnits], rbase[kUnits];
     uint32_t runit[kUnits], roff[kUnits];
-    int rrx0[kUnits], rrz0[kUnits], rrw[kUnits];   // rect of each record's unit
+    int rrx[kUnits], rrz[kUnits], rrw[kUnits];   // first region of each record's tile, width of its rect
     unsigned int hist[P1_KINDS];
     unsigned int n_list;
     uint32_t grad[kGradWords];
@@ -1436,8 +1445,8 @@ __global__ void __launch_bounds__(kThreadsB, 2) entrance_kernel(BatchArgs a) {
                 S.rbase[rr] = up.rbase;
                 S.runit[rr] = u;
                 S.roff[rr] = off;
-                S.rrx0[rr] = up.rx0;
-                S.rrz0[rr] = up.rz0;
+                S.rrx[rr] = up.rx;
+                S.rrz[rr] = up.rz;
                 S.rrw[rr] = up.rw;
             }
             if (cnt) {
@@ -1467,9 +1476,7 @@ __global__ void __launch_bounds__(kThreadsB, 2) entrance_kernel(BatchArgs a) {
                 const uint32_t em = S.emap[e0 + e];
                 const int r2 = (int)(em >> 16);
                 const uint32_t jr = a.surv_region[S.roff[r2] + (em & 0xFFFFu)];
-                const uint64_t reg = S.rbase[r2] + jr;
-                const int rz = S.rrz0[r2] + (int)(reg / (uint64_t)S.rrw[r2]);
-                const int rx = S.rrx0[r2] + (int)(reg % (uint64_t)S.rrw[r2]);
+                const int rz = S.rrz[r2] + (int)(jr >> 16), rx = S.rrx[r2] + (int)(jr & 0xFFFFu);
                 int cx, cz;
                 hut_chunk(S.rseed[r2], rx, rz, a.salt, cx, cz);
                 S.hx[e] = cx * 16 + 3;
@@ -1588,7 +1595,7 @@ __global__ void __launch_bounds__(kThreadsB, 2) entrance_kernel(BatchArgs a) {
                 else if (ent_v[1] >= 0) code = P1_ENTRANCE_60;
                 if (code >= 0) {
                     atomicAdd(&S.hist[code], 1u);
-                    note_code(a, S.rg[r2], S.rbase[r2] + jr, code, -1);
+                    note_code(a, S.rg[r2], S.rbase[r2] + (uint64_t)(jr >> 16) * (uint64_t)S.rrw[r2] + (jr & 0xFFFFu), code, -1);
                 } else {
                     uint32_t di = atomicAdd(&a.counters[CNT_DEEP], 1u);
                     if (di < a.cap_deep) {
@@ -1641,13 +1648,18 @@ void launch_entrance(const BatchArgs &a, int grid, cudaStream_t s) {
 constexpr int kLadderHeights = 12;   // maxHeight, the y <= 0 ladder (<= 6), y = 10..40
 constexpr int kFloodHeights = 16;
 
-struct LadderSmem {
-    uint8_t perm[256 * kLadderStride];       // slot s, row k at k * kLadderStride + s
-    double org[kSlotsC * 3];
+// A candidate's samples and heights.
+struct LadderVals {
     double val[kSlotsC][kLadderHeights];     // [slot][height index]
     double fval[2][kFloodHeights];           // floodedness samples
     double tun[kLadderHeights];
     int ys[kLadderHeights];
+};
+
+struct LadderSmem {
+    uint8_t perm[256 * kLadderStride];       // slot s, row k at k * kLadderStride + s
+    double org[kSlotsC * 3];
+    LadderVals v;
     uint32_t grad[kGradWords];
 };
 
@@ -1661,12 +1673,182 @@ __device__ __forceinline__ double combine_vals(int noise, const double *v, int s
     return (a + b) * ns.amplitude;
 }
 
+// lysh's ladder for one candidate whose cave tables `src` reads, by all NT threads of the CTA; the
+// survivor, the reject code and the funnel go to the batch.
+template <int NT, class Src>
+__device__ void ladder_candidate(const BatchArgs &a, LadderVals &S, const Src &src, uint64_t seed, uint64_t g,
+                                 uint64_t r, int rx, int rz, int cx, int cz, int mh) {
+    const int t = threadIdx.x;
+    const int large = a.large_biomes ? 1 : 0;
+    const int cont_noise = large ? N_CONTINENTALNESS_LARGE : N_CONTINENTALNESS;
+    // heights: [0] maxHeight, then y = 0, -10, ... >= ladderFloor with maxHeight < y, then
+    // 10..40 (S.ys is rewritten only after the previous candidate's closing barrier)
+    int floor_y = (-40 < mh) ? -40 : mh;
+    if (floor_y < -50) floor_y = -50;
+    int nh = 0;
+    if (t == 0) S.ys[nh] = mh;
+    nh++;
+    for (int y = 0; y >= floor_y; y -= 10)
+        if (mh < y) {
+            if (t == 0) S.ys[nh] = y;
+            nh++;
+        }
+    const int first_pos = nh;
+    for (int y = 10; y <= 40; y += 10) {
+        if (t == 0) S.ys[nh] = y;
+        nh++;
+    }
+    const long long nf_ll = mh > 60 ? 0 : ((long long)60 - mh) / 10 + 1;
+    const int nf = nf_ll > kFloodHeights ? 0 : (int)nf_ll;   // more: sampled one by one at the end
+    const int hut_x = cx * 16, hut_z = cz * 16;
+    const int hx = hut_x + 3, hz = hut_z + 3;
+    __syncthreads();
+    // round 1: per height, rarity .. rough minus spaghetti_3d_1/2 (8 slots), cave_layer and
+    // cave_cheese (16 slots); cave_entrance (6 slots) at y = 10..40; continentalness; flood
+    const int n_a = nh * 24, n_b = (nh - first_pos) * 6, n_c = 18, n_d = nf * 2;
+    for (int k = t; k < n_a + n_b + n_c + n_d; k += NT) {
+        int slot, hi = 0;
+        double px, py, pz;
+        if (k < n_a) {
+            hi = k / 24;
+            const int s24 = k % 24;
+            slot = s24 < 4 ? kBaseRarity + s24 : (s24 < 8 ? kBaseRmod + (s24 - 4) : kBaseLayer + (s24 - 8));
+            const int y = S.ys[hi];
+            if (slot < kBaseRmod || slot >= kBaseLayer) {
+                if (slot < kBaseThickness) {   // rarity at (x*2, y, z*2)
+                    px = (double)(int)((uint32_t)hx * 2u); py = (double)y; pz = (double)(int)((uint32_t)hz * 2u);
+                } else if (slot < kBaseSp1) {  // thickness
+                    px = (double)hx; py = (double)y; pz = (double)hz;
+                } else if (slot < kBaseCheese) {   // cave_layer at (x, y*8, z)
+                    px = (double)hx; py = (double)(int)((uint32_t)y * 8u); pz = (double)hz;
+                } else {                           // cave_cheese at (x, y*2/3, z)
+                    px = (double)hx; py = (double)y * 0.6666666666666666; pz = (double)hz;
+                }
+            } else {                               // roughness modulator / roughness
+                px = (double)hx; py = (double)y; pz = (double)hz;
+            }
+        } else if (k < n_a + n_b) {
+            const int kk = k - n_a;
+            hi = first_pos + kk / 6;
+            slot = kBaseEntrance + kk % 6;
+            const int y = S.ys[hi];
+            px = (double)hx * 0.75; py = (double)y * 0.5; pz = (double)hz * 0.75;
+        } else if (k < n_a + n_b + n_c) {
+            slot = kBaseCont + (k - n_a - n_b);
+            px = (hut_x + 8) / 4.0; py = 0.0; pz = (hut_z + 8) / 4.0;
+        } else {
+            const int kk = k - n_a - n_b - n_c;
+            hi = kk >> 1;
+            slot = kBaseFlood + (kk & 1);
+            px = (double)(hut_x + 3); py = (double)(mh + 10 * hi) * 0.67; pz = (double)(hut_z + 3);
+        }
+        const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
+        const double v = slot_sample(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
+        if (slot >= kBaseFlood) S.fval[slot - kBaseFlood][hi] = v;
+        else S.val[slot][hi] = v;
+    }
+    __syncthreads();
+    if (t < nh) S.tun[t] = tunnel_scale(combine_vals(N_SPAGHETTI_RARITY, &S.val[kBaseRarity][t], kLadderHeights));
+    __syncthreads();
+    // round 2: spaghetti_3d_1 / _2 at (x/e, y/e, z/e)
+    for (int k = t; k < nh * 4; k += NT) {
+        const int hi = k >> 2, slot = kBaseSp1 + (k & 3);
+        const double e = S.tun[hi], y = (double)S.ys[hi];
+        const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
+        S.val[slot][hi] = slot_sample(src, slot, sub, c_noise[noise].lac[p], (double)hx / e, y / e, (double)hz / e);
+    }
+    __syncthreads();
+    if (t == 0) {
+        // lysh_phase1_check_ex from the cave at maxHeight on (phase1.c:149-199)
+        auto spag = [&](int hi) {
+            const double e = S.tun[hi];
+            const double tv = combine_vals(N_SPAGHETTI_THICKNESS, &S.val[kBaseThickness][hi], kLadderHeights);
+            const double h = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
+            const double l = combine_vals(N_SPAGHETTI_1, &S.val[kBaseSp1][hi], kLadderHeights);
+            const double m = fabs(e * l) - h;
+            const double n = combine_vals(N_SPAGHETTI_2, &S.val[kBaseSp2][hi], kLadderHeights);
+            const double o = fabs(e * n) - h;
+            const double pp = clampd(jmax(m, o), -1.0, 1.0);
+            const double mod = combine_vals(N_ROUGHNESS_MODULATOR, &S.val[kBaseRmod][hi], kLadderHeights);
+            const double rgh = combine_vals(N_ROUGHNESS, &S.val[kBaseRough][hi], kLadderHeights);
+            const double qq = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
+            return pp + qq;
+        };
+        auto chz = [&](int hi) {
+            const double layer = combine_vals(N_CAVE_LAYER, &S.val[kBaseLayer][hi], kLadderHeights);
+            const double av = 4.0 * layer * layer;
+            const double raw = combine_vals(N_CAVE_CHEESE, &S.val[kBaseCheese][hi], kLadderHeights);
+            return av + clampd(0.27 + raw, -1.0, 1.0);
+        };
+        int code = P1_ACCEPT;
+        if (spag(0) >= 0 && chz(0) >= 0) code = P1_CAVE_AT_MAXH;
+        if (code == P1_ACCEPT)
+            for (int hi = 1; hi < first_pos; hi++)
+                if (spag(hi) >= 0 && chz(hi) >= 0) {
+                    code = P1_LADDER_NEG;
+                    break;
+                }
+        if (code == P1_ACCEPT)
+            for (int hi = first_pos; hi < nh; hi++) {
+                const int y = S.ys[hi];
+                const double ent = combine_vals(N_CAVE_ENTRANCE, &S.val[kBaseEntrance][hi], kLadderHeights);
+                const double tt = (10.0 + (double)y) / 40.0;
+                const double cl = tt < 0.0 ? 0.3 : (tt > 1.0 ? 0.0 : lerp(tt, 0.3, 0.0));
+                const double cc = ent + 0.37 + cl;
+                if (jmin(cc, spag(hi)) >= 0 && chz(hi) >= 0) {
+                    code = P1_LADDER_POS;
+                    break;
+                }
+            }
+        if (code == P1_ACCEPT && !a.single_biome) {
+            // the y = 0 climate sample equals the 3-D sample at y = 0 bit for bit
+            const double c = combine_vals(cont_noise, &S.val[kBaseCont][0], kLadderHeights);
+            if (c < -0.11) code = P1_CONTINENTALNESS;
+        }
+        if (code == P1_ACCEPT) {
+            if (nf_ll <= kFloodHeights) {
+                for (int fi = 0; fi < nf; fi++)
+                    if (combine_vals(N_FLOODEDNESS, &S.fval[0][fi], kFloodHeights) > 0.41) {
+                        code = P1_FLOODEDNESS;
+                        break;
+                    }
+            } else {
+                for (long long y = mh; y <= 60; y += 10) {
+                    const double f = dbl3d(src, N_FLOODEDNESS, kBaseFlood, (double)(hut_x + 3),
+                                           (double)y * 0.67, (double)(hut_z + 3));
+                    if (f > 0.41) {
+                        code = P1_FLOODEDNESS;
+                        break;
+                    }
+                }
+            }
+        }
+        atomicAdd(&a.hist[code], 1ull);
+        note_code(a, g, r, code, -1);
+        if (code == P1_ACCEPT) {
+            uint32_t oi = atomicAdd(&a.counters[CNT_FINAL], 1u);
+            if (oi < a.cap_out) {
+                Candidate c;
+                c.seed_index = g;
+                c.seed = (int64_t)seed;
+                c.rx = rx;
+                c.rz = rz;
+                c.chunk_x = cx;
+                c.chunk_z = cz;
+                a.out[oi] = c;
+            } else {
+                atomicOr(&a.counters[CNT_OVERFLOW], 4u);
+            }
+        }
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(BatchArgs a) {
     __shared__ __align__(16) LadderSmem S;
     batch_range(a);
     const int t = threadIdx.x;
     const int large = a.large_biomes ? 1 : 0;
-    const int cont_noise = large ? N_CONTINENTALNESS_LARGE : N_CONTINENTALNESS;
     if (a.counters[CNT_OVERFLOW]) return;
     const uint32_t n_deep = min(a.counters[CNT_DEEP], a.cap_deep);
     fill_grad_table(S.grad, t);
@@ -1675,34 +1857,10 @@ __global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(BatchArgs a) {
     for (uint32_t q = blockIdx.x; q < n_deep; q += gridDim.x) {
         const uint32_t u = a.deep[2 * q], jr = a.deep[2 * q + 1];
         const UnitPos up = unit_pos(a, u);
-        const uint64_t g = up.g;
-        const uint64_t r = up.rbase + jr;
-        const uint64_t seed = seed_value(a, g);
-        int rx, rz, cx, cz;
-        unit_region_xz(up, r, rx, rz);
+        const uint64_t seed = seed_value(a, up.g);
+        const int rx = up.rx + (int)(jr & 0xFFFFu), rz = up.rz + (int)(jr >> 16);
+        int cx, cz;
         hut_chunk(seed, rx, rz, a.salt, cx, cz);
-        // heights: [0] maxHeight, then y = 0, -10, ... >= ladderFloor with maxHeight < y, then
-        // 10..40 (S.ys is rewritten only after the previous candidate's closing barrier)
-        const int mh = up.max_height;
-        int floor_y = (-40 < mh) ? -40 : mh;
-        if (floor_y < -50) floor_y = -50;
-        int nh = 0;
-        if (t == 0) S.ys[nh] = mh;
-        nh++;
-        for (int y = 0; y >= floor_y; y -= 10)
-            if (mh < y) {
-                if (t == 0) S.ys[nh] = y;
-                nh++;
-            }
-        const int first_pos = nh;
-        for (int y = 10; y <= 40; y += 10) {
-            if (t == 0) S.ys[nh] = y;
-            nh++;
-        }
-        const long long nf_ll = mh > 60 ? 0 : ((long long)60 - mh) / 10 + 1;
-        const int nf = nf_ll > kFloodHeights ? 0 : (int)nf_ll;   // more: sampled one by one at the end
-        const int hut_x = cx * 16, hut_z = cz * 16;
-        const int hx = hut_x + 3, hz = hut_z + 3;
         perm_blocks_init<kLadderStride, 256 * kLadderStride>(S.perm, 1, t, kThreadsC);
         __syncthreads();
         if (t < kSlotsC) {
@@ -1715,147 +1873,11 @@ __global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(BatchArgs a) {
             S.org[3 * t + 2] = oz;
         }
         __syncthreads();
-        // round 1: per height, rarity .. rough minus spaghetti_3d_1/2 (8 slots), cave_layer and
-        // cave_cheese (16 slots); cave_entrance (6 slots) at y = 10..40; continentalness; flood
-        const int n_a = nh * 24, n_b = (nh - first_pos) * 6, n_c = 18, n_d = nf * 2;
-        for (int k = t; k < n_a + n_b + n_c + n_d; k += kThreadsC) {
-            int slot, hi = 0;
-            double px, py, pz;
-            if (k < n_a) {
-                hi = k / 24;
-                const int s24 = k % 24;
-                slot = s24 < 4 ? kBaseRarity + s24 : (s24 < 8 ? kBaseRmod + (s24 - 4) : kBaseLayer + (s24 - 8));
-                const int y = S.ys[hi];
-                if (slot < kBaseRmod || slot >= kBaseLayer) {
-                    if (slot < kBaseThickness) {   // rarity at (x*2, y, z*2)
-                        px = (double)(int)((uint32_t)hx * 2u); py = (double)y; pz = (double)(int)((uint32_t)hz * 2u);
-                    } else if (slot < kBaseSp1) {  // thickness
-                        px = (double)hx; py = (double)y; pz = (double)hz;
-                    } else if (slot < kBaseCheese) {   // cave_layer at (x, y*8, z)
-                        px = (double)hx; py = (double)(int)((uint32_t)y * 8u); pz = (double)hz;
-                    } else {                           // cave_cheese at (x, y*2/3, z)
-                        px = (double)hx; py = (double)y * 0.6666666666666666; pz = (double)hz;
-                    }
-                } else {                               // roughness modulator / roughness
-                    px = (double)hx; py = (double)y; pz = (double)hz;
-                }
-            } else if (k < n_a + n_b) {
-                const int kk = k - n_a;
-                hi = first_pos + kk / 6;
-                slot = kBaseEntrance + kk % 6;
-                const int y = S.ys[hi];
-                px = (double)hx * 0.75; py = (double)y * 0.5; pz = (double)hz * 0.75;
-            } else if (k < n_a + n_b + n_c) {
-                slot = kBaseCont + (k - n_a - n_b);
-                px = (hut_x + 8) / 4.0; py = 0.0; pz = (hut_z + 8) / 4.0;
-            } else {
-                const int kk = k - n_a - n_b - n_c;
-                hi = kk >> 1;
-                slot = kBaseFlood + (kk & 1);
-                px = (double)(hut_x + 3); py = (double)(mh + 10 * hi) * 0.67; pz = (double)(hut_z + 3);
-            }
-            const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
-            const double v = slot_sample(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
-            if (slot >= kBaseFlood) S.fval[slot - kBaseFlood][hi] = v;
-            else S.val[slot][hi] = v;
-        }
-        __syncthreads();
-        if (t < nh) S.tun[t] = tunnel_scale(combine_vals(N_SPAGHETTI_RARITY, &S.val[kBaseRarity][t], kLadderHeights));
-        __syncthreads();
-        // round 2: spaghetti_3d_1 / _2 at (x/e, y/e, z/e)
-        for (int k = t; k < nh * 4; k += kThreadsC) {
-            const int hi = k >> 2, slot = kBaseSp1 + (k & 3);
-            const double e = S.tun[hi], y = (double)S.ys[hi];
-            const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
-            S.val[slot][hi] = slot_sample(src, slot, sub, c_noise[noise].lac[p], (double)hx / e, y / e, (double)hz / e);
-        }
-        __syncthreads();
-        if (t == 0) {
-            // lysh_phase1_check_ex from the cave at maxHeight on (phase1.c:149-199)
-            auto spag = [&](int hi) {
-                const double e = S.tun[hi];
-                const double tv = combine_vals(N_SPAGHETTI_THICKNESS, &S.val[kBaseThickness][hi], kLadderHeights);
-                const double h = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
-                const double l = combine_vals(N_SPAGHETTI_1, &S.val[kBaseSp1][hi], kLadderHeights);
-                const double m = fabs(e * l) - h;
-                const double n = combine_vals(N_SPAGHETTI_2, &S.val[kBaseSp2][hi], kLadderHeights);
-                const double o = fabs(e * n) - h;
-                const double pp = clampd(jmax(m, o), -1.0, 1.0);
-                const double mod = combine_vals(N_ROUGHNESS_MODULATOR, &S.val[kBaseRmod][hi], kLadderHeights);
-                const double rgh = combine_vals(N_ROUGHNESS, &S.val[kBaseRough][hi], kLadderHeights);
-                const double qq = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
-                return pp + qq;
-            };
-            auto chz = [&](int hi) {
-                const double layer = combine_vals(N_CAVE_LAYER, &S.val[kBaseLayer][hi], kLadderHeights);
-                const double av = 4.0 * layer * layer;
-                const double raw = combine_vals(N_CAVE_CHEESE, &S.val[kBaseCheese][hi], kLadderHeights);
-                return av + clampd(0.27 + raw, -1.0, 1.0);
-            };
-            int code = P1_ACCEPT;
-            if (spag(0) >= 0 && chz(0) >= 0) code = P1_CAVE_AT_MAXH;
-            if (code == P1_ACCEPT)
-                for (int hi = 1; hi < first_pos; hi++)
-                    if (spag(hi) >= 0 && chz(hi) >= 0) {
-                        code = P1_LADDER_NEG;
-                        break;
-                    }
-            if (code == P1_ACCEPT)
-                for (int hi = first_pos; hi < nh; hi++) {
-                    const int y = S.ys[hi];
-                    const double ent = combine_vals(N_CAVE_ENTRANCE, &S.val[kBaseEntrance][hi], kLadderHeights);
-                    const double tt = (10.0 + (double)y) / 40.0;
-                    const double cl = tt < 0.0 ? 0.3 : (tt > 1.0 ? 0.0 : lerp(tt, 0.3, 0.0));
-                    const double cc = ent + 0.37 + cl;
-                    if (jmin(cc, spag(hi)) >= 0 && chz(hi) >= 0) {
-                        code = P1_LADDER_POS;
-                        break;
-                    }
-                }
-            if (code == P1_ACCEPT && !a.single_biome) {
-                // the y = 0 climate sample equals the 3-D sample at y = 0 bit for bit
-                const double c = combine_vals(cont_noise, &S.val[kBaseCont][0], kLadderHeights);
-                if (c < -0.11) code = P1_CONTINENTALNESS;
-            }
-            if (code == P1_ACCEPT) {
-                if (nf_ll <= kFloodHeights) {
-                    for (int fi = 0; fi < nf; fi++)
-                        if (combine_vals(N_FLOODEDNESS, &S.fval[0][fi], kFloodHeights) > 0.41) {
-                            code = P1_FLOODEDNESS;
-                            break;
-                        }
-                } else {
-                    for (long long y = mh; y <= 60; y += 10) {
-                        const double f = dbl3d(src, N_FLOODEDNESS, kBaseFlood, (double)(hut_x + 3),
-                                               (double)y * 0.67, (double)(hut_z + 3));
-                        if (f > 0.41) {
-                            code = P1_FLOODEDNESS;
-                            break;
-                        }
-                    }
-                }
-            }
-            atomicAdd(&a.hist[code], 1ull);
-            note_code(a, g, r, code, -1);
-            if (code == P1_ACCEPT) {
-                uint32_t oi = atomicAdd(&a.counters[CNT_FINAL], 1u);
-                if (oi < a.cap_out) {
-                    Candidate c;
-                    c.seed_index = g;
-                    c.seed = (int64_t)seed;
-                    c.rx = rx;
-                    c.rz = rz;
-                    c.chunk_x = cx;
-                    c.chunk_z = cz;
-                    a.out[oi] = c;
-                } else {
-                    atomicOr(&a.counters[CNT_OVERFLOW], 4u);
-                }
-            }
-        }
-        __syncthreads();
+        ladder_candidate<kThreadsC>(a, S.v, src, seed, up.g, up.region(jr), rx, rz, cx, cz, up.max_height);
     }
 }
+
+#include "wg_unit.cuh"
 
 // grid <= 0: as many blocks as are resident at once (the kernel loops over candidates, so blocks
 // beyond the resident count would only form a second, mostly idle wave)
@@ -1884,6 +1906,7 @@ void prepare_phase1_launches() {
     allow_dynamic_smem(climate_kernel<false, false>, sizeof(ClimateSmem<false>), g_smem_done64);
     allow_dynamic_smem(entrance_kernel<false>, sizeof(EntranceSmem), g_smem_done_ent);
     allow_dynamic_smem(entrance_kernel<true>, sizeof(EntranceSmem), g_smem_done_ent32);
+    prepare_unit_launches();
     ladder_geometry();
 }
 

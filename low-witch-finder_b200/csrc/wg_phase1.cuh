@@ -59,6 +59,7 @@ enum : int {
     CNT_FINAL,         // phase-1 survivors
     CNT_OVERFLOW,      // bit 0 records/survivors, bit 1 deep list, bit 2 final list
     CNT_RECHECK,       // FP32 noise core: gate decisions re-taken in FP64 (value inside the error band)
+    CNT_DEEP_UNIT,     // deep candidates the unit kernel finished itself
     CNT_WORDS = 8
 };
 
@@ -70,10 +71,9 @@ struct Candidate {
     int32_t chunk_x, chunk_z;
 };
 
-// Work is cut into "units": unit u of a request is (seed u / n_win, region window
-// u % n_win); a window is `win` consecutive regions of the rect (rz outer, rx inner).  One
-// lane of the climate kernel owns one unit, so a request with few seeds and a huge rect
-// (a whole-world scan of one seed) fills the GPU as well as many seeds x 9x9 regions.
+// Work is cut into "units": unit u of a request is (seed u / n_win, tile u % n_win); a tile is a
+// tw x th block of the rect's regions (the last ones of a row or column smaller), tiles row by row.
+// A region inside its unit is one word, its offset in the tile: dx | dz << 16.
 //
 // Jobs mode flattens many Seed Check jobs, each with its own rect and floor, into one batch:
 // entry k of the job table covers the global units [unit0, next entry's unit0) and maps them
@@ -82,12 +82,10 @@ struct JobGeom {
     uint64_t unit0;        // first global unit of this entry (entries sorted by unit0, none empty)
     uint64_t first;        // the job's unit index of that first unit
     uint64_t seed0;        // global seed index of the job's seed 0 (index into BatchArgs::seeds)
-    uint64_t n_win;        // windows per seed of the job
-    uint64_t n_regions;    // regions per seed (rw * rh)
-    uint32_t win;          // regions per window
-    int32_t rx0, rz0, rw;  // the job's region rect origin and width
+    uint64_t n_win;        // tiles per seed of the job
+    int32_t rx0, rz0, rw, rh;   // the job's region rect
+    uint32_t tw, th, ntx;  // tile size in regions, tiles per row of the rect
     int32_t max_height;    // the job's gate floor
-    int32_t pad;
 };
 static_assert(sizeof(JobGeom) == 64, "job table entry layout");
 
@@ -97,8 +95,8 @@ struct BatchArgs {
     uint64_t gen_base;
     uint64_t unit0;               // global index of the batch's first unit
     uint32_t n_units;             // units in this batch
-    uint32_t win;                 // regions per window
-    uint64_t n_win;               // windows per seed
+    uint32_t tw, th, ntx;         // tile size in regions, tiles per row of the rect
+    uint64_t n_win;               // tiles per seed
     uint64_t n_regions;           // regions per seed (rw * rh)
     int rx0, rz0, rw, rh;         // region rect origin and size
     int salt;
@@ -113,8 +111,8 @@ struct BatchArgs {
     uint32_t *rec_unit;           // [cap_rec] batch-local unit of each record
     uint32_t *rec_off;            // [cap_rec] first entry in surv_region
     uint32_t *rec_cnt;            // [cap_rec]
-    uint32_t *surv_region;        // [cap_surv] region offset inside the unit's window
-    uint32_t *deep;               // [cap_deep * 2] (batch-local unit, region offset)
+    uint32_t *surv_region;        // [cap_surv] region offset in the unit's tile (dx | dz << 16)
+    uint32_t *deep;               // [cap_deep * 2] (batch-local unit, region offset in its tile)
     Candidate *out;               // [cap_out] phase-1 survivors of this batch
     uint32_t cap_rec, cap_surv, cap_deep, cap_out;
     uint32_t *counters;           // [CNT_WORDS], zeroed per batch
@@ -132,6 +130,8 @@ struct BatchArgs {
     // max_height per job; seeds from `seeds`); unit0 .. unit0 + n_units are global units of it.
     const JobGeom *jobs = nullptr;
     uint32_t n_jobs = 0;
+
+    int unit_cta = 0;             // one CTA per unit runs all of phase 1 (launch_unit) instead of the three kernels
 
     // Optional device work queue (wg_queue.cu): when set, the batch's unit0 and n_units are read
     // from dyn[0], dyn[1] at kernel start instead of the fields above (a graph replays the same
@@ -167,9 +167,9 @@ struct F32Bands {
     float r_lo[4], r_hi[4];
 };
 
-// Bound on |FP32 Perlin sample - exact sample| of perlin_y0_f32 (wg_device.cuh), in units of
-// 2^-24; derived operation by operation in the comment above perlin_y0_f32.
-constexpr double kPerlinF32ErrUlps = 44.0;
+// Bound on |FP32 Perlin sample - exact sample| in units of 2^-24: 44 for perlin_y0_f32 (derived in
+// the comment above it) and unit_sample_f32, 45 for lat_sample (wg_unit.cuh).
+constexpr double kPerlinF32ErrUlps = 48.0;
 // The same bound for the 3-D sample perlin_3d_f32 (the cave noises of the entrance kernel).
 constexpr double kPerlin3dF32ErrUlps = 60.0;
 enum : int { ACT_NONE = 0, ACT_TIER, ACT_TIER_LAST, ACT_END_SUB_A, ACT_TEMPERATURE, ACT_RIDGE };
@@ -199,6 +199,8 @@ void upload_tables(const NoiseSpec *specs, const ClimateStep *steps_normal, cons
 void launch_climate(const BatchArgs &a, cudaStream_t s);
 void launch_entrance(const BatchArgs &a, int grid, cudaStream_t s);
 void launch_ladder(const BatchArgs &a, int grid, cudaStream_t s);
+// All of phase 1, one CTA per unit; deep candidates past a CTA's own list go to the ladder kernel's.
+void launch_unit(const BatchArgs &a, cudaStream_t s);
 // Sets the kernels' shared-memory limits and the ladder's resident-block count on the current
 // device, so that the launch functions make no further runtime calls (a stream capture may follow).
 void prepare_phase1_launches();

@@ -60,7 +60,7 @@ __global__ void queue_plan_kernel(QueueState *q, const JobGeom *jobs, uint32_t *
     uint32_t e = entry_of(jobs, q->n_jobs, u0);
     while (u0 + n < q->total && n < q->max_units) {
         const uint64_t end = e + 1 < q->n_jobs ? jobs[e + 1].unit0 : q->total;
-        const uint64_t per = jobs[e].win;
+        const uint64_t per = (uint64_t)jobs[e].tw * jobs[e].th;
         uint64_t k = (q->budget - work) / per;
         if (k == 0) {
             if (n) break;
@@ -98,7 +98,7 @@ __global__ void queue_commit_kernel(QueueState *q, const uint32_t *counters, con
             base = q->n_out;
             q->n_out += nf;
             q->climate_survivors += counters[CNT_SURVIVORS];
-            q->deep += counters[CNT_DEEP];
+            q->deep += counters[CNT_DEEP] + counters[CNT_DEEP_UNIT];
             q->rechecks += counters[CNT_RECHECK];
             q->records += counters[CNT_RECORDS];
             q->cursor += q->dyn[1];
@@ -185,8 +185,12 @@ int run_queue(wg_engine *eng, const BatchArgs &proto, uint64_t total_units, uint
         QUEUE_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed),
                    "capture");
         queue_plan_kernel<<<1, 32, 0, s>>>(R.q, proto.jobs, a.counters, a.hist);
-        launch_climate(a, s);
-        launch_entrance(a, 0, s);
+        if (a.unit_cta) {
+            launch_unit(a, s);
+        } else {
+            launch_climate(a, s);
+            launch_entrance(a, 0, s);
+        }
         launch_ladder(a, 0, s);
         queue_commit_kernel<<<1, 256, 0, s>>>(R.q, a.counters, a.hist, a.out, R.out, R.cap, cond);
         cudaGraph_t captured = nullptr;

@@ -1,0 +1,48 @@
+"""GPU: the one-CTA-per-unit phase-1 kernel (few seeds or many regions per seed), verdict by verdict
+against the C restatement.
+
+The sizes are where its tiles and blocks can go wrong: one region, blocks of 32 regions a side exactly
+full and one over, rects one region wide and longer than a tile's largest side (1,023), a tile cut off
+at the rect's edge, the world border, and coordinates beyond the FP32 core's range.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+RECTS = [(0, 1, 0, 1), (-16, 16, -16, 16), (5, 38, -7, 26), (0, 1, -530, 570), (-40, 61, 3, 5), (-70, 70, -1, 30),
+         (58540, 58594, -58594, -58550), (3_000_000, 3_000_040, -3_000_033, -3_000_000)]
+
+
+@pytest.mark.parametrize("core", ["fp32", "fp64", "fp32_recheck_all"])
+@pytest.mark.parametrize("version,preset", [("1.19.x~26.1", "NORMAL"), ("26.2", "LARGE_BIOMES"), ("1.18.2", "NORMAL")])
+@pytest.mark.parametrize("rect", RECTS)
+def test_codes_equal_the_oracle(engine, port, bind_mod, core, version, preset, rect):
+    rules = bind_mod.rules(version, preset)
+    seeds = [1473884015873122059, -7, 3]
+    engine.set_noise_core(core)
+    try:
+        codes, tiers = engine.phase1_codes(seeds=seeds, rect=rect, max_height=-50, version=version, preset=preset)
+    finally:
+        engine.set_noise_core("fp32")
+    for i, s in enumerate(seeds):
+        c, t, _, _ = port.phase1_rect(s, rules, -50, rect)
+        assert np.array_equal(codes[i], c)
+        assert np.array_equal(tiers[i], t)
+
+
+def test_survivors_equal_the_list_kernels(engine, wg):
+    """A rect of many regions per seed (one CTA per tile) against the same regions in strips of few per
+    seed run as jobs (the list kernels), at a relaxed floor so that there are survivors."""
+    seeds = wg.splitmix64_array(77, 6)
+    whole = engine.seed_check(seeds=seeds, rect=(-100, 100, -100, 100), max_height=40)
+    assert len(whole.candidates)
+    jobs = [{"seeds": seeds, "rect": (x, x + 20, z, z + 20), "max_height": 40} for x in range(-100, 100, 20)
+            for z in range(-100, 100, 20)]
+    per, st = engine.seed_check_jobs(jobs)
+    parts = np.sort(np.concatenate(per), order=["seed_index", "rz", "rx"])
+    assert np.array_equal(parts, whole.candidates)
+    assert st["reject_hist"] == whole.stats["reject_hist"]
+    assert st["tier_hist"] == whole.stats["tier_hist"]
