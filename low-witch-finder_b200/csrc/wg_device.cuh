@@ -218,6 +218,16 @@ __device__ __forceinline__ void perm_blocks_init(uint8_t *base, int nblocks, int
 // the four steps' draws are taken again one by one with the exact rejection loop.  Either way the
 // draws, and so the table, are those of the step-by-step shuffle; the common path is straight-line
 // code in which the next draws overlap the swaps.
+struct ShuffleDraws {
+    Xr32 q;
+    uint32_t j[4];
+};
+// Four draws one by one with the exact rejection loop, out of line (never taken in most launches).
+static __device__ __noinline__ ShuffleDraws shuffle_slow(Xr32 q, uint32_t b0) {
+    ShuffleDraws d{q, {0, 0, 0, 0}};
+    for (int s = 0; s < 4; s++) d.j[s] = d.q.bounded(b0 - (uint32_t)s);
+    return d;
+}
 template <int STRIDE>
 __device__ __forceinline__ void perlin_shuffle(uint8_t *t, Xr r, double &ox, double &oy, double &oz) {
     ox = xr_double(r) * 256.0;
@@ -231,11 +241,12 @@ __device__ __forceinline__ void perlin_shuffle(uint8_t *t, Xr r, double &ox, dou
         const uint32_t x0 = q.next32(), x1 = q.next32(), x2 = q.next32(), x3 = q.next32();
         uint32_t j0 = __umulhi(x0, b0), j1 = __umulhi(x1, b1), j2 = __umulhi(x2, b2), j3 = __umulhi(x3, b3);
         if ((x0 * b0 < b0) | (x1 * b1 < b1) | (x2 * b2 < b2) | (x3 * b3 < b3)) {
-            q = q0;
-            j0 = q.bounded(b0);
-            j1 = q.bounded(b1);
-            j2 = q.bounded(b2);
-            j3 = q.bounded(b3);
+            const ShuffleDraws d = shuffle_slow(q0, b0);
+            q = d.q;
+            j0 = d.j[0];
+            j1 = d.j[1];
+            j2 = d.j[2];
+            j3 = d.j[3];
         }
         const uint32_t js[4] = {j0, j1, j2, j3};
 #pragma unroll
@@ -461,17 +472,13 @@ __device__ __forceinline__ void fill_grad_table_f32(GradF *gf, int tid) {
     }
 }
 
-// One Perlin sampler at y = 0 in the FP32 core; hyf / fyf are rn(hy) and rn(fade(hy)) of the
-// table's y origin fraction, jy its floor.  x, z are the FP64 sampling coordinates.  The corner
-// values are paired along z, (v.0, v.1), so the x and y lerps and both fades run two lanes per
-// instruction; every lane performs the operations the bound above counts.
+// One Perlin sampler at y = 0 in the FP32 core, in lattice cell (i, k) at fractions (g, l); hyf / fyf are
+// rn(hy) and rn(fade(hy)) of the table's y origin fraction, jy its floor.  The corner values are paired
+// along z, (v.0, v.1), so the x and y lerps and both fades run two lanes per instruction; every lane
+// performs the operations the bound above counts.
 template <class T>
-__device__ __forceinline__ float perlin_y0_f32(const T &P, double ox, double oz, int jy, float hyf, float fyf,
-                                               double x, double z) {
-    const double d = x + ox, f = z + oz;
-    const double fd = floor(d), ff = floor(f);
-    const int i = (int)fd, k = (int)ff;
-    const float g = __double2float_rn(d - fd), l = __double2float_rn(f - ff);
+__device__ __forceinline__ float perlin_y0_cell_f32(const T &P, int i, int jy, int k, float g, float l, float hyf,
+                                                    float fyf) {
     const F2 gl = f2(g, l);
     float g1, l1;
     f2_split(f2_add(gl, f2(-1.0f, -1.0f)), g1, l1);   // g - 1, l - 1
@@ -496,6 +503,15 @@ __device__ __forceinline__ float perlin_y0_f32(const T &P, double ox, double oz,
     float y0, y1;
     f2_split(lerp_f32x2(f2(fyf, fyf), x0, x1), y0, y1);
     return lerp_f32(fz, y0, y1);
+}
+
+// The same at the FP64 sampling coordinates x, z.
+template <class T>
+__device__ __forceinline__ float perlin_y0_f32(const T &P, double ox, double oz, int jy, float hyf, float fyf,
+                                               double x, double z) {
+    const double d = x + ox, f = z + oz;
+    const double fd = floor(d), ff = floor(f);
+    return perlin_y0_cell_f32(P, (int)fd, jy, (int)ff, __double2float_rn(d - fd), __double2float_rn(f - ff), hyf, fyf);
 }
 
 // fade_f32 on one lane: 1/2 + s (15/8 + s^2 (6 s^2 - 5)), s = t - 1/2 (fade_f32x2's operations)

@@ -39,15 +39,19 @@ Tiling wg::tile_rect(uint64_t rw, uint64_t rh, uint64_t target) {
     return t;
 }
 
+bool wg::few_units(uint64_t n_seeds, double n_regions, int sm_count, bool fp32) {
+    return (double)n_seeds <= (fp32 ? 6.0 : 3.0) * sm_count * (1.0 + n_regions / 1024.0);
+}
+
 // Whether a request's units take the one-CTA kernel, and its tiles.  Many regions per seed: yes, a
 // tile's two table builds (13,000 warp instructions) are then a small part of it, and the ladder and
-// the entrance gate find the seed's tables built.  Few units for the GPU (sm_count * 3 CTAs are
-// resident): yes too, in tiles small enough to give every CTA one, since the call then takes one
-// build and one evaluation of latency instead of three.  Otherwise 16 units share a CTA.
-static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, bool single_biome, int sm_count, bool &cta) {
-    const uint64_t n_regions = rw * rh, slots = (uint64_t)sm_count * 3;
+// the entrance gate find the seed's tables built.  Few units (few_units): yes too, in tiles small
+// enough to give every one of the sm_count * 3 resident CTAs one, since the call then takes one build
+// and one evaluation of latency instead of three.  Otherwise 16 units share a CTA.
+static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, const wg_engine *eng, bool single_biome, bool &cta) {
+    const uint64_t n_regions = rw * rh, slots = (uint64_t)eng->sm_count * 3;
     const double total = (double)n_seeds * (double)n_regions;
-    cta = !single_biome && (n_regions >= kUnitCtaRegions || n_seeds <= 4 * slots);
+    cta = !single_biome && (n_regions >= kUnitCtaRegions || few_units(n_seeds, (double)n_regions, eng->sm_count, eng->fp32_core != 0));
     if (!cta) return tile_rect(rw, rh, n_regions <= 4096 ? n_regions : 2048);
     // one tile per resident CTA up to 2,048 regions each, then several waves of larger ones
     uint64_t target = (uint64_t)(total / (double)slots) + 1;
@@ -112,6 +116,7 @@ void wg::build_climate_steps(const NoiseSpec *specs, int erosion, int temperatur
         mag += std::fabs(c);
         err += std::fabs(c) * (eps + vmax * u) + vmax * u * mag;
         s.cf = (float)c;
+        s.fstep = (uint64_t)(4.0 * s.sc * s.lac * 72057594037927936.0);
         s.err = (float)(2.0 * err + 1e-10);
         if (s.act == ACT_TIER || s.act == ACT_TIER_LAST) {
             const double center = s.thr / s.amp, half = 2.0 * err + 1e-10;
@@ -171,12 +176,19 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
     BatchArgs a = proto;
     a.unit0 = unit0;
     a.n_units = n_units;
+    const bool spots = !a.unit_cta && spot_path(a.jobs != nullptr, (uint64_t)a.tw * a.th, a.codes != nullptr, a.single_biome != 0);
+    const bool lists = !spots && list_path(a, n_units);
+    if (lists) {
+        int rc = list_buffers(eng);
+        if (rc) return rc;
+        a.lists[0] = eng->lists[0];
+        a.lists[1] = eng->lists[1];
+    }
     WG_CUDA(cudaMemsetAsync(eng->counters, 0, sizeof(uint32_t) * CNT_WORDS, eng->stream), "memset counters");
     WG_CUDA(cudaMemsetAsync(eng->hist, 0, sizeof(unsigned long long) * (P1_KINDS + kTiers), eng->stream),
             "memset hist");
     WG_CUDA(cudaEventRecord(eng->kev[0], eng->stream), "event");
     // one region per unit: the climate tables are built lazily, breadth first
-    const bool spots = !a.unit_cta && spot_path(a.jobs != nullptr, (uint64_t)a.tw * a.th, a.codes != nullptr, a.single_biome != 0);
     if (spots) {
         if (!eng->spot_counts) {
             WG_CUDA(cudaMalloc(&eng->spot_items[0], sizeof(SpotItem) * kSpotUnits), "alloc");
@@ -187,6 +199,8 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
                             eng->stream);
     } else if (a.unit_cta) {
         launch_unit(a, eng->stream);
+    } else if (lists) {
+        launch_lists(a, eng->stream);
     } else {
         launch_climate(a, eng->stream);
     }
@@ -227,9 +241,9 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
     }
     for (int i = 0; i < P1_KINDS; i++) st.reject_hist[i] += (int64_t)eng->h_hist[i];
     for (int i = 0; i < kTiers; i++) st.tier_hist[i] += (int64_t)eng->h_hist[P1_KINDS + i];
-    st.climate_survivors += eng->h_counters[CNT_SURVIVORS];
+    st.climate_survivors += climate_survivors(eng->h_counters);
     st.rechecks += eng->h_counters[CNT_RECHECK];
-    st.records += eng->h_counters[CNT_RECORDS];
+    st.records += climate_records(eng->h_counters);
     st.deep_candidates += eng->h_counters[CNT_DEEP] + eng->h_counters[CNT_DEEP_UNIT];
     uint32_t nf = eng->h_counters[CNT_FINAL];
     if (nf) {
@@ -270,7 +284,27 @@ BatchArgs base_args(wg_engine *eng, const wg_opts &opts, int salt) {
     a.cap_out = kCapOut;
     a.counters = eng->counters;
     a.hist = eng->hist;
+    a.lists[2] = RegionList{eng->rec_unit, eng->rec_off, eng->rec_cnt, eng->surv, nullptr, kCapRec, kCapSurv, CNT_RECORDS};
     return a;
+}
+
+int list_buffers(wg_engine *eng) {
+    if (eng->list_block) return WG_OK;
+    const size_t rec = sizeof(uint32_t) * kCapRec, reg = sizeof(uint32_t) * kCapSurv, one = 3 * rec + 2 * reg;
+    WG_CUDA(cudaMalloc(&eng->list_block, 2 * one), "alloc lists");
+    for (int k = 0; k < 2; k++) {
+        char *p = static_cast<char *>(eng->list_block) + k * one;
+        RegionList &L = eng->lists[k];
+        L.unit = reinterpret_cast<uint32_t *>(p);
+        L.off = reinterpret_cast<uint32_t *>(p + rec);
+        L.rcnt = reinterpret_cast<uint32_t *>(p + 2 * rec);
+        L.surv = reinterpret_cast<uint32_t *>(p + 3 * rec);
+        L.pay = reinterpret_cast<float *>(p + 3 * rec + reg);
+        L.cap_rec = kCapRec;
+        L.cap_surv = kCapSurv;
+        L.cnt = 0;
+    }
+    return WG_OK;
 }
 
 int run_request(wg_engine *eng, const Request &rq, Sink &sink, wg_scan_stats &st) {
@@ -279,7 +313,7 @@ int run_request(wg_engine *eng, const Request &rq, Sink &sink, wg_scan_stats &st
     const uint64_t n_regions = rw * rh;
     const bool spot = spot_path(false, n_regions, rq.d_codes != nullptr, rq.opts.single_biome != 0);
     bool cta = false;
-    const Tiling tiles = spot ? tile_rect(rw, rh, 1) : request_tiles(rw, rh, rq.n_seeds, rq.opts.single_biome != 0, eng->sm_count, cta);
+    const Tiling tiles = spot ? tile_rect(rw, rh, 1) : request_tiles(rw, rh, rq.n_seeds, eng, rq.opts.single_biome != 0, cta);
     const uint64_t n_win = tiles.n_win, win = tiles.win();
     const uint64_t units = rq.n_seeds * n_win;
 
@@ -483,6 +517,7 @@ void wg_engine_close(wg_engine *eng) {
     cudaFree(eng->counters);
     cudaFree(eng->hist);
     cudaFree(eng->d_seed_list);
+    cudaFree(eng->list_block);
     cudaFree(eng->spot_items[0]);
     cudaFree(eng->spot_items[1]);
     cudaFree(eng->spot_counts);

@@ -44,6 +44,8 @@ struct wg_engine {
     int64_t *d_seed_list = nullptr;
     uint64_t d_seed_cap = 0;
     // breadth-first climate stage of one-region batches: two item lists and their counts
+    wg::RegionList lists[2] = {};         // the list kernels' alternating lists, in one block
+    void *list_block = nullptr;
     wg::SpotItem *spot_items[2] = {nullptr, nullptr};
     uint32_t *spot_counts = nullptr;
 
@@ -120,8 +122,13 @@ struct Tiling {
 // Tiles of at most `target` regions (at least one), near square, of equal size up to rounding.
 Tiling tile_rect(uint64_t rw, uint64_t rh, uint64_t target);
 
-// Regions per seed from which a unit takes the one-CTA kernel (launch_unit).
-constexpr uint64_t kUnitCtaRegions = 2048;
+// Regions per seed from which a unit takes the one-CTA kernel (launch_unit) however many seeds there
+// are: 8,192 seeds x 2,025 regions take it 1.73 ms and the list kernels 1.41; 3,552 x 4,096 1.07 and 1.99.
+constexpr uint64_t kUnitCtaRegions = 3072;
+// Whether so few units are better off with one CTA each (one wave of sm_count * 3 CTAs takes 70 to
+// 150 us, the fused kernels 100 to 200 whatever the number): 81 regions, 888 seeds 154 us and 162 fused,
+// 1,332 183 and 164; 1,024 regions, 1,776 seeds 337 and 367, 3,552 582 and 477.  FP64 units take longer.
+bool few_units(uint64_t n_seeds, double n_regions, int sm_count, bool fp32);
 // Regions per unit of the one-CTA kernel at most.
 constexpr uint64_t kUnitCtaMax = 1ull << 16;
 
@@ -162,6 +169,17 @@ struct Sink {            // where phase-1 survivors go after each batch
     uint64_t found = 0;
 };
 
+// Units per batch from which the list kernels run the climate and first entrance stages.  Below, their
+// seven builds in a row outweigh their higher rate (9 x 9 regions, fused and list kernels: 16,384 seeds
+// 358 and 391 us, 24,576 482 and 467, 131,072 2,030 and 1,650; 1 x 2 regions: 228 and 270, 296 and 297,
+// 1,048 and 679).
+constexpr uint32_t kListUnits = 24576;
+// Allocates the list kernels' lists once per engine.
+int list_buffers(wg_engine *eng);
+// Whether a batch of n_units units takes the list kernels.
+inline bool list_path(const BatchArgs &a, uint32_t n_units) {
+    return !a.unit_cta && a.fp32_core == 1 && a.small_coords && !a.single_biome && n_units >= kListUnits;
+}
 // The BatchArgs fields every batch of an engine shares (work lists, counters, rules, salt).
 BatchArgs base_args(wg_engine *eng, const wg_opts &opts, int salt);
 // Runs units [unit0, unit0 + n_units) of `proto` (three kernels, one sync), halving on overflow.

@@ -40,6 +40,11 @@ bool candidate_order(const Candidate &x, const Candidate &y) {
     return x.rx < y.rx;
 }
 
+// Whether a batch of so few units takes the one-CTA kernel.
+bool small_batch(const wg_engine *eng, const SchedJob &lead, uint64_t units, uint64_t work) {
+    return !lead.opts.single_biome && few_units(units, (double)work / (double)units, eng->sm_count, eng->fp32_core != 0);
+}
+
 // Whether a job's climate coordinates are proved inside maintainPrecision's identity range.
 bool job_small(const SchedJob &j) {
     return coords_small(std::min<int64_t>(j.rx0, j.rz0),
@@ -252,7 +257,7 @@ int Scheduler::step(std::vector<SchedJob *> &finished, std::vector<SchedJob *> &
     a.seeds = d_arena_;
     a.jobs = d_table_;
     a.n_jobs = (uint32_t)table.size();
-    a.unit_cta = lead.unit_cta ? 1 : 0;
+    a.unit_cta = lead.unit_cta || small_batch(eng_, lead, units, step_work_ - budget) ? 1 : 0;
     a.small_coords = 1;
     for (const SchedJob *j : members) a.small_coords &= job_small(*j) ? 1 : 0;
     found_.clear();
@@ -364,13 +369,14 @@ int jobs_on_device_queue(wg_engine *eng, std::vector<SchedJob> &js, uint64_t tot
             // one table: the lead's rule set
             std::vector<JobGeom> table;
             std::vector<size_t> member;
-            uint64_t units = 0;
+            uint64_t units = 0, work = 0;
             uint64_t min_win = ~0ull;
             for (size_t i = lead; i < js.size(); i++) {
                 if (done[i] || !same_rules(js[i], js[lead])) continue;
                 table.push_back(job_geom(js[i], units, 0, off[i]));
                 member.push_back(i);
                 units += js[i].units;
+                work += js[i].units * js[i].tiles.win();
                 min_win = std::min(min_win, js[i].tiles.win());
                 done[i] = 1;
             }
@@ -384,7 +390,7 @@ int jobs_on_device_queue(wg_engine *eng, std::vector<SchedJob> &js, uint64_t tot
             a.seeds = d_seeds;
             a.jobs = d_table;
             a.n_jobs = (uint32_t)table.size();
-            a.unit_cta = js[lead].unit_cta ? 1 : 0;
+            a.unit_cta = js[lead].unit_cta || small_batch(eng, js[lead], units, work) ? 1 : 0;
             a.small_coords = 1;
             for (size_t k : member) a.small_coords &= job_small(js[k]) ? 1 : 0;
             std::vector<Candidate> found;

@@ -85,7 +85,11 @@ struct UnitPos {
 };
 __device__ __forceinline__ void unit_tile(UnitPos &p, uint64_t tile, uint32_t tw, uint32_t th, uint32_t ntx, int rx0,
                                           int rz0, int rw, int rh) {
-    const uint32_t x = (uint32_t)(tile % ntx) * tw, z = (uint32_t)(tile / ntx) * th;
+    uint32_t x = 0, z = 0;
+    if (tile) {   // a rect of one tile takes no division
+        x = (uint32_t)(tile % ntx) * tw;
+        z = (uint32_t)(tile / ntx) * th;
+    }
     p.rx = rx0 + (int)x;
     p.rz = rz0 + (int)z;
     p.tw = min(tw, (uint32_t)rw - x);
@@ -95,7 +99,7 @@ __device__ __forceinline__ void unit_tile(UnitPos &p, uint64_t tile, uint32_t tw
 }
 __device__ __forceinline__ UnitPos unit_pos(const BatchArgs &a, uint32_t u) {
     UnitPos p;
-    const uint64_t ul = a.unit0 + u;
+    const uint64_t ul = batch_unit0(a) + u;
     if (a.jobs) {
         // the last table entry whose first global unit is <= this unit
         uint32_t lo = 0, hi = a.n_jobs - 1;
@@ -106,13 +110,14 @@ __device__ __forceinline__ UnitPos unit_pos(const BatchArgs &a, uint32_t u) {
         }
         const JobGeom &j = a.jobs[lo];
         const uint64_t loc = ul - j.unit0 + j.first;
-        p.g = j.seed0 + loc / j.n_win;
-        unit_tile(p, loc % j.n_win, j.tw, j.th, j.ntx, j.rx0, j.rz0, j.rw, j.rh);
+        const uint64_t k = j.n_win == 1 ? loc : loc / j.n_win;
+        p.g = j.seed0 + k;
+        unit_tile(p, loc - k * j.n_win, j.tw, j.th, j.ntx, j.rx0, j.rz0, j.rw, j.rh);
         p.max_height = j.max_height;
         return p;
     }
-    p.g = ul / a.n_win;
-    unit_tile(p, ul % a.n_win, a.tw, a.th, a.ntx, rect_x0(a, p.g), rect_z0(a, p.g), a.rw, a.rh);
+    p.g = a.n_win == 1 ? ul : ul / a.n_win;
+    unit_tile(p, ul - p.g * a.n_win, a.tw, a.th, a.ntx, rect_x0(a, p.g), rect_z0(a, p.g), a.rw, a.rh);
     p.max_height = a.max_height;
     return p;
 }
@@ -514,12 +519,12 @@ __device__ void climate_rest(Sm &S, const BatchArgs &a, TierCounts &tc, uint32_t
 // order and decides exactly as the FP64 path does.  So every decision, and with it the reject
 // codes, tier histogram and survivor set, equals the FP64 path's.
 template <bool F32, bool SMALL>
-__global__ void __launch_bounds__(kThreadsA, 2) climate_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(kThreadsA, 2) climate_kernel(const __grid_constant__ BatchArgs a) {
     using Real = typename ClimateSmem<F32>::Real;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     ClimateSmem<F32> &S = *reinterpret_cast<ClimateSmem<F32> *>(smem_raw);
-    batch_range(a);
-    if (blockIdx.x * kUnits >= a.n_units) return;   // past this batch (a launch sized for a larger one)
+    const uint32_t n_units = batch_units(a);
+    if (blockIdx.x * kUnits >= n_units) return;   // past this batch (a launch sized for a larger one)
     const int tid = threadIdx.x;
     const int my_slot = tid / kUnits, uu = tid % kUnits;
     const int large = a.large_biomes ? 1 : 0;
@@ -545,7 +550,7 @@ __global__ void __launch_bounds__(kThreadsA, 2) climate_kernel(BatchArgs a) {
     }
 
     const uint32_t u = blockIdx.x * kUnits + (uint32_t)uu;
-    const bool valid = u < a.n_units;
+    const bool valid = u < n_units;
     UnitPos up{};
     up.tw = 1;
     if (valid) up = unit_pos(a, u);
@@ -1402,10 +1407,10 @@ __device__ __forceinline__ int free_slot(int i) { return i < kBaseSp1 ? i : i + 
 // times the amplitude; caves.c:83-113).  Entrance(60) is computed for every survivor but only
 // decides those with Entrance(50) < 0, as in lysh.
 template <bool F32>
-__global__ void __launch_bounds__(kThreadsB, 2) entrance_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(kThreadsB, 2) entrance_kernel(const __grid_constant__ BatchArgs a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     EntranceSmem &S = *reinterpret_cast<EntranceSmem *>(smem_raw);
-    batch_range(a);
+    const uint32_t n_units = batch_units(a);
     const int tid = threadIdx.x;
     const int my_slot = tid / kUnits, rr = tid % kUnits;
     const bool all_rechecks = F32 && a.fp32_core == 2;   // every FP32 decision re-taken in FP64 (a check mode)
@@ -1435,7 +1440,7 @@ __global__ void __launch_bounds__(kThreadsB, 2) entrance_kernel(BatchArgs a) {
         if (ri < n_rec) {
             const uint32_t u = a.rec_unit[ri], off = a.rec_off[ri];
             cnt = a.rec_cnt[ri];
-            if (u >= a.n_units || off >= a.cap_surv || cnt > a.cap_surv - off || cnt > kRecordCap) cnt = 0;
+            if (u >= n_units || off >= a.cap_surv || cnt > a.cap_surv - off || cnt > kRecordCap) cnt = 0;
             const UnitPos up = unit_pos(a, u);
             const uint64_t g = up.g;
             const uint64_t seed = seed_value(a, g);
@@ -1844,9 +1849,8 @@ __device__ void ladder_candidate(const BatchArgs &a, LadderVals &S, const Src &s
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(const __grid_constant__ BatchArgs a) {
     __shared__ __align__(16) LadderSmem S;
-    batch_range(a);
     const int t = threadIdx.x;
     const int large = a.large_biomes ? 1 : 0;
     if (a.counters[CNT_OVERFLOW]) return;
@@ -1878,6 +1882,7 @@ __global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(BatchArgs a) {
 }
 
 #include "wg_unit.cuh"
+#include "wg_lists.cuh"
 
 // grid <= 0: as many blocks as are resident at once (the kernel loops over candidates, so blocks
 // beyond the resident count would only form a second, mostly idle wave)
@@ -1907,6 +1912,7 @@ void prepare_phase1_launches() {
     allow_dynamic_smem(entrance_kernel<false>, sizeof(EntranceSmem), g_smem_done_ent);
     allow_dynamic_smem(entrance_kernel<true>, sizeof(EntranceSmem), g_smem_done_ent32);
     prepare_unit_launches();
+    prepare_list_launches();
     ladder_geometry();
 }
 

@@ -60,7 +60,31 @@ enum : int {
     CNT_OVERFLOW,      // bit 0 records/survivors, bit 1 deep list, bit 2 final list
     CNT_RECHECK,       // FP32 noise core: gate decisions re-taken in FP64 (value inside the error band)
     CNT_DEEP_UNIT,     // deep candidates the unit kernel finished itself
-    CNT_WORDS = 8
+    // records and regions of the list kernels' stages (a pair each: n, n + 1), by what they passed
+    CNT_EROSION_LIST = 8,
+    CNT_TEMP_LIST = 10,
+    CNT_CLIMATE_LIST = 12,
+    CNT_SCALED_LIST = 14,
+    CNT_ENTRANCE_LIST = 16,
+    CNT_WORDS = 20
+};
+
+// Climate survivors and their records in a batch's counters: the list kernels count them as a list, the
+// other paths in CNT_SURVIVORS / CNT_RECORDS (which the list kernels use for what the entrance kernel gets).
+__host__ __device__ inline uint32_t climate_survivors(const uint32_t *c) {
+    return c[CNT_CLIMATE_LIST + 1] ? c[CNT_CLIMATE_LIST + 1] : c[CNT_SURVIVORS];
+}
+__host__ __device__ inline uint32_t climate_records(const uint32_t *c) {
+    return c[CNT_CLIMATE_LIST] ? c[CNT_CLIMATE_LIST] : c[CNT_RECORDS];
+}
+
+// Regions that passed a stage, grouped in records of one unit each (device pointers).
+struct RegionList {
+    uint32_t *unit, *off, *rcnt;   // per record: batch-local unit, first region, regions (<= 32)
+    uint32_t *surv;                // per region: its offset in the unit's tile (dx | dz << 16)
+    float *pay;                    // per region: the value a later stage needs, or null
+    uint32_t cap_rec, cap_surv;
+    int cnt;                       // its counters
 };
 
 // Final phase-1 survivor; the layout of wg_candidate in include/witchgpu.h.
@@ -131,6 +155,7 @@ struct BatchArgs {
     const JobGeom *jobs = nullptr;
     uint32_t n_jobs = 0;
 
+    RegionList lists[3];          // list kernels: two that alternate, and the entrance kernel's input (rec_*, surv_region)
     int unit_cta = 0;             // one CTA per unit runs all of phase 1 (launch_unit) instead of the three kernels
 
     // Optional device work queue (wg_queue.cu): when set, the batch's unit0 and n_units are read
@@ -141,15 +166,10 @@ struct BatchArgs {
 };
 
 // The batch range of a launch: dyn when set, else the launch's own fields.
-__device__ __forceinline__ void batch_range(BatchArgs &a) {
-    if (a.dyn) {
-        a.unit0 = a.dyn[0];
-        a.n_units = (uint32_t)a.dyn[1];
-    }
-}
+__device__ __forceinline__ uint64_t batch_unit0(const BatchArgs &a) { return a.dyn ? a.dyn[0] : a.unit0; }
+__device__ __forceinline__ uint32_t batch_units(const BatchArgs &a) { return a.dyn ? (uint32_t)a.dyn[1] : a.n_units; }
 
-// One evaluation step of the climate state machine (a single y=0 Perlin sample).  The last
-// four fields serve the FP32 noise core: cf = (float)(c1 * c2), and for a tier step the band
+// One evaluation step of the climate state machine (a single y=0 Perlin sample).  cf to err serve the FP32 noise core: cf = (float)(c1 * c2), and for a tier step the band
 // [lo, hi) of partial sums (in sum space, i.e. before the amplitude) inside which an FP32
 // partial sum cannot decide the tier; err is the bound on |FP32 partial sum - FP64 partial sum|
 // after this step.
@@ -157,6 +177,7 @@ struct ClimateStep {
     double sc, lac, c1, c2, thr, amp;
     int slot, act, tier, pad;
     float cf, lo, hi, err;
+    uint64_t fstep;   // 4 sc lac 2^56: the 8.56 fixed-point step of one chunk (wg_unit.cuh)
 };
 
 // Undecidable bands of the FP32 core for the temperature and ridge gates, in sum space
@@ -199,6 +220,9 @@ void upload_tables(const NoiseSpec *specs, const ClimateStep *steps_normal, cons
 void launch_climate(const BatchArgs &a, cudaStream_t s);
 void launch_entrance(const BatchArgs &a, int grid, cudaStream_t s);
 void launch_ladder(const BatchArgs &a, int grid, cudaStream_t s);
+// The climate gates and the first entrance tests as list kernels (FP32 core, small coordinates, no
+// SINGLE_BIOME); what stays open is the entrance kernel's input.
+void launch_lists(const BatchArgs &a, cudaStream_t s);
 // All of phase 1, one CTA per unit; deep candidates past a CTA's own list go to the ladder kernel's.
 void launch_unit(const BatchArgs &a, cudaStream_t s);
 // Sets the kernels' shared-memory limits and the ladder's resident-block count on the current

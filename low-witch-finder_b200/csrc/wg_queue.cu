@@ -97,10 +97,10 @@ __global__ void queue_commit_kernel(QueueState *q, const uint32_t *counters, con
             nf = counters[CNT_FINAL];
             base = q->n_out;
             q->n_out += nf;
-            q->climate_survivors += counters[CNT_SURVIVORS];
+            q->climate_survivors += climate_survivors(counters);
             q->deep += counters[CNT_DEEP] + counters[CNT_DEEP_UNIT];
             q->rechecks += counters[CNT_RECHECK];
-            q->records += counters[CNT_RECORDS];
+            q->records += climate_records(counters);
             q->cursor += q->dyn[1];
             q->slices++;
             if (q->budget < q->max_budget) q->budget = min(q->max_budget, q->budget * 2);
@@ -167,6 +167,13 @@ int run_queue(wg_engine *eng, const BatchArgs &proto, uint64_t total_units, uint
     a.unit0 = 0;
     a.n_units = max_units;   // the launch geometry; the slice range comes from dyn
     a.dyn = R.q->dyn;
+    const bool lists = list_path(a, max_units);
+    if (lists) {
+        int rc = list_buffers(eng);
+        if (rc) return rc;
+        a.lists[0] = eng->lists[0];
+        a.lists[1] = eng->lists[1];
+    }
     prepare_phase1_launches();
 
     cudaGraph_t graph = nullptr;
@@ -188,7 +195,8 @@ int run_queue(wg_engine *eng, const BatchArgs &proto, uint64_t total_units, uint
         if (a.unit_cta) {
             launch_unit(a, s);
         } else {
-            launch_climate(a, s);
+            if (lists) launch_lists(a, s);
+            else launch_climate(a, s);
             launch_entrance(a, 0, s);
         }
         launch_ladder(a, 0, s);

@@ -541,12 +541,11 @@ __device__ __forceinline__ bool unit_cave_at(const SrcUnit &src, double *v, int 
 // One CTA per unit.  F32: the FP32 noise core with the block lattices (small coordinates only), else
 // FP64 samples throughout, in the reference's order.
 template <bool F32>
-__global__ void __launch_bounds__(kUThreads, 3) unit_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constant__ BatchArgs a) {
     using Real = typename UnitSmem<F32>::Real;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     UnitSmem<F32> &S = *reinterpret_cast<UnitSmem<F32> *>(smem_raw);
-    batch_range(a);
-    if (blockIdx.x >= a.n_units) return;
+    if (blockIdx.x >= batch_units(a)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned below = (1u << lane) - 1u;
     const int large = a.large_biomes ? 1 : 0;
@@ -604,7 +603,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(BatchArgs a) {
             const double xc = (U.ucx * 16 + 8) * 0.25, zc = (U.ucz * 16 + 8) * 0.25;
             S.fx[lane] = to_fixed(keep_precision((xc * sc) * lac) + ox);
             S.fz[lane] = to_fixed(keep_precision((zc * sc) * lac) + oz);
-            S.fstep[lane] = (uint64_t)(4.0 * sc * lac * 72057594037927936.0);
+            S.fstep[lane] = c_steps[large][lane].fstep;
             if (lane < kLatTables) {
                 S.w0[lane] = __double2float_rn(1.0 - fy);
                 S.w1[lane] = __double2float_rn(fy);

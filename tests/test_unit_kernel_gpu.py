@@ -46,3 +46,19 @@ def test_survivors_equal_the_list_kernels(engine, wg):
     assert np.array_equal(parts, whole.candidates)
     assert st["reject_hist"] == whole.stats["reject_hist"]
     assert st["tier_hist"] == whole.stats["tier_hist"]
+
+
+@pytest.mark.parametrize("version,preset", [("1.19.x~26.1", "NORMAL"), ("26.2", "LARGE_BIOMES"), ("1.18.2", "NORMAL")])
+@pytest.mark.parametrize("n,rect", [(24576, (-4, 5, -4, 5)), (24579, (0, 1, 0, 3)), (25001, (7, 17, -30, -21)),
+                                    (24577, (58585, 58594, -58594, -58574))])
+def test_list_kernels_codes_equal_the_fp64_core(engine, version, preset, n, rect):
+    """From 24,576 units of few regions on, the FP32 core takes the list kernels and the FP64 core the
+    fused ones: every verdict equal, at unit counts that leave groups of units and records part full."""
+    a = engine.phase1_codes(gen=(n, n), rect=rect, max_height=-50, version=version, preset=preset)
+    engine.set_noise_core("fp64")
+    try:
+        b = engine.phase1_codes(gen=(n, n), rect=rect, max_height=-50, version=version, preset=preset)
+    finally:
+        engine.set_noise_core("fp32")
+    assert np.array_equal(a[0], b[0])
+    assert np.array_equal(a[1], b[1])
