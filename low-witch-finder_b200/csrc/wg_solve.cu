@@ -13,8 +13,8 @@
 //     bits (state bits 17..19 of the region's first two draws) and whose equation bits
 //     0 .. 3 + m are already zero; key = (cx, cz) mod 2^(4+m), which fixes those bits;
 //   * chain: per task (region, offset) one warp, each lane lifts the upper 28 state bits of one
-//     list entry.  When v2(cx) != v2(cz) each equation bit has one solution and the lift runs
-//     four bits per step (lift_chunks); when v2(cx) == v2(cz) state bit j does not reach
+//     list entry.  When v2(cx) != v2(cz) each equation bit has one solution and the lift is a
+//     fixed-point iteration (lift); when v2(cx) == v2(cz) state bit j does not reach
 //     equation bit j - 16 + m, so a nibble of the equation has 0 to 16 solutions and the lift is
 //     a depth-first search over nibbles (lift_eq).  Past equation bit 31 the remaining top bits
 //     are enumerated and every completion is checked in full (48-bit carver state, hut offsets
@@ -45,7 +45,6 @@ constexpr uint32_t kListCap = 1536;     // t20 entries per (group, key) list (me
 constexpr uint32_t kGroupsPerBatch = 16;
 constexpr uint32_t kHitCap = 1u << 20;
 constexpr int kChainThreads = 256;
-constexpr int kLiftTable = 8 * 16 * 16;    // nibble lift table (bytes)
 constexpr int kEqTable = 8 * 16 * 16 * 2;  // nibble solution masks of the v2(cx) == v2(cz) lift (bytes)
 
 // One group slot of a batch: its regions, offsets, key table and first task.
@@ -138,17 +137,15 @@ __device__ __forceinline__ void emit_hit(const ChainTask &T, uint64_t S, SolveHi
     else atomicOr(&cnt[SCNT_OVERFLOW], 2ull);
 }
 
-// v2(cx) != v2(cz), four state bits per step.  Divide the equation by 2^m and call "o" the term
-// whose multiplier is odd after that (cx h2 if v2(cx) = m, else cz h4) and "e" the other.  With
-// z = o (the odd term's value) as the unknown instead of the upper state bits u: 16 u =
-// (z - o0) / (odd multiplier) = V, and e = Kq + rho z with rho = (even multiplier) / (odd
-// multiplier), an even number.  The equation z ^ (Kq + rho z) ^ Y = 0, where Y = (S ^ X) >> m
-// holds u only as V << 16 (bits known from lower nibbles), is triangular in z nibble by nibble:
-// nibble k solves zk ^ ((Aq_k + rho zk) mod 16) = Y_k, Aq = Kq + rho z<k, one lookup in a
-// 2,048-entry table [rho mod 16 / 2][Aq_k][Y_k].  The top m bits of u are free.
-struct ChunkTask {
-    uint32_t inv, rho, coef_o_x;   // 1 / odd multiplier, rho, 1 if the odd term is cx h2
-    const uint8_t *row;            // table row for rho mod 16
+// v2(cx) != v2(cz).  Divide the equation by 2^m and call "o" the term whose multiplier is odd after that
+// (cx h2 if v2(cx) = m, else cz h4) and "e" the other.  With z = o (the odd term's value) as the unknown
+// instead of the upper state bits u: 16 u = (z - o0) / (odd multiplier) = V, and e = Kq + rho z with
+// rho = (even multiplier) / (odd multiplier), an even number.  The equation z ^ (Kq + rho z) ^ Y = 0, where
+// Y = (S ^ X) >> m holds u only as V << 16 (bits known from lower ones), is a fixed point z = Y ^ (Kq + rho z)
+// whose right side's bit j reads z's bits below j - d + 1 only, d = v2(rho): every step settles d more
+// bits (lift).  The top m bits of u are free.
+struct ChunkTask {   // of the equal class's search
+    uint32_t inv, rho;   // 1 / odd multiplier, rho
 };
 
 __device__ __forceinline__ uint32_t inverse_u32(uint32_t a) {   // a odd
@@ -158,44 +155,84 @@ __device__ __forceinline__ uint32_t inverse_u32(uint32_t a) {   // a odd
     return x;
 }
 
-// Full check of t = t20 | u << 20 (u: 28 bits).  The 48-bit carver state from 32-bit words: the
-// draws' low words h2, h4 move by (A^2 << 4) u and (A^4 << 4) u; only the low 16 bits of the high
-// words h1, h3 reach bit 47 of a, b, and those are bits 16..31 of A t + C, A^3 t + K3, which the
-// state's low word alone decides.
-__device__ __forceinline__ void check_u(const ChainTask &T, uint32_t t20, uint32_t h2, uint32_t h4, uint32_t u,
-                                        SolveHitDev *hits, uint32_t cap, unsigned long long *cnt) {
-    const uint32_t t32 = t20 | (u << 20);
-    const uint32_t h2u = h2 + (uint32_t)(kA2 << 4) * u, h4u = h4 + (uint32_t)(kA4 << 4) * u;
-    const uint32_t h1lo = (((uint32_t)kA * t32 + (uint32_t)kC) >> 16) & 0xFFFFu;
-    const uint32_t h3lo = (((uint32_t)kA3 * t32 + (uint32_t)kK3) >> 16) & 0xFFFFu;
-    const uint64_t a = ((uint64_t)h1lo << 32) + (uint64_t)(int64_t)(int32_t)h2u;
-    const uint64_t b = ((uint64_t)h3lo << 32) + (uint64_t)(int64_t)(int32_t)h4u;
+// A state whose 48 carver bits match so far (1 in 65,536 of the checked): the whole check, out of line.
+__device__ __noinline__ void check_state(const ChainTask &T, uint32_t t32, uint32_t u, SolveHitDev *hits, uint32_t cap,
+                                         unsigned long long *cnt) {
     const uint64_t S = ((((uint64_t)(u >> 12)) << 32) | t32) ^ (kA & kM48);
-    const uint64_t carver =
-        ((uint64_t)((int64_t)T.cx * (int64_t)a) ^ (uint64_t)((int64_t)T.cz * (int64_t)b) ^ S) & kM48;
-    if (carver != T.X) return;
     if (solve_check(S, T.cx, T.cz, T.X, T.creg, T.ox, T.oz)) emit_hit(T, S, hits, cap, cnt);
 }
 
-__device__ void lift_chunks(const ChainTask &T, const ChunkTask &N, uint32_t t20, SolveHitDev *hits, uint32_t cap,
-                             unsigned long long *cnt) {
-    const uint32_t cx = (uint32_t)T.cx, cz = (uint32_t)T.cz, m = (uint32_t)T.m;
-    const uint32_t h2 = (uint32_t)((((kA2 * t20) + kK2) & kM48) >> 16);
-    const uint32_t h4 = (uint32_t)((((kA4 * t20) + kK4) & kM48) >> 16);
-    const uint32_t P = cx * h2, Q = cz * h4;
-    const uint32_t o0 = (N.coef_o_x ? P : Q) >> m, e0 = (N.coef_o_x ? Q : P) >> m;
-    const uint32_t s0 = t20 ^ (uint32_t)kA, x32 = (uint32_t)T.X;
-    const uint32_t kq = e0 - N.rho * o0;
-    uint32_t z = o0 & 15u;   // nibble 0 is o0's: u only enters from bit 4 (16 u)
+// Check of t = t20 | u << 20 (u: 28 bits), whose low 32 carver bits the lift has solved (at m > 0 all but what
+// the enumerated top bits decide).  The draws' low words h2, h4 move by (A^2 << 4) u and (A^4 << 4) u; bits
+// 32..47 of cx a, with a = (h1 << 32) + (signed) h2, are those of the signed high product cx h2 plus cx h1,
+// where only the low 16 bits of h1 count, and those are bits 16..31 of A t + C, which the state's low
+// word alone decides (h3 likewise, A^3 t + K3).
+__device__ __forceinline__ void check_u(const ChainTask &T, uint32_t t20, uint32_t h2, uint32_t h4, uint32_t u,
+                                        SolveHitDev *hits, uint32_t cap, unsigned long long *cnt) {
+    const uint32_t t32 = t20 + (u << 20);
+    const uint32_t h2u = h2 + (uint32_t)(kA2 << 4) * u, h4u = h4 + (uint32_t)(kA4 << 4) * u;
+    const uint32_t h1 = ((uint32_t)kA * t32 + (uint32_t)kC) >> 16, h3 = ((uint32_t)kA3 * t32 + (uint32_t)kK3) >> 16;
+    const uint32_t x = (uint32_t)__mulhi(T.cx, (int)h2u) + (uint32_t)T.cx * h1;
+    const uint32_t z = (uint32_t)__mulhi(T.cz, (int)h4u) + (uint32_t)T.cz * h3;
+    const uint32_t top = x ^ z ^ (u >> 12) ^ (uint32_t)((kA ^ T.X) >> 32);
+    if ((top & 0xFFFFu) == 0) check_state(T, t32, u, hits, cap, cnt);
+}
+
+// Lifts the task's list entries, lanes over the list, D bits of z a step (D <= v2(rho)).  Y's bits below
+// 16 - m do not depend on u, and V's bits below j are settled once z's are (V is z's difference times an
+// odd number), so V is formed twice, when z's low 16 bits are known and, for m > 0, again at 20: bits
+// 16..19 of Y read V's bits m .. 3 + m (<= 7), those above read its bits up to 15 + m (<= 19).  M0: m = 0;
+// OX: the odd term is cx h2.  A step is two instructions, one on each integer pipe; a nibble looked up
+// in a table took ten.  Half of an odd-class plan's tasks have D = 1 (28 steps), a quarter D = 2 (14).
+// Measured, 2.4e10 entries (32 groups of the odd class at regime 22), wall: by the table 178 ms, V formed
+// twice and the check above on 16 bits 153 ms, the steps 124 ms, M0 and OX split off and the list prefetched 102 ms (FMA-heavy pipe 71 % busy, ALU 50 %, issue 62 %).
+template <int D, bool M0, bool OX>
+__device__ __forceinline__ void lift(const ChainTask &T, uint32_t inv, uint32_t rho, const uint32_t *list, uint32_t n,
+                                     SolveHitDev *hits, uint32_t cap, unsigned long long *cnt) {
+    const uint32_t m = M0 ? 0u : (uint32_t)T.m;
+    const uint32_t sc = (uint32_t)kA ^ (uint32_t)T.X, umask = (1u << (28 - m)) - 1u;
+    const uint32_t *p = list + (threadIdx.x & 31), *const end = list + n;
+    uint32_t next = p < end ? *p : 0u;
+    for (; p < end; p += 32) {
+        const uint32_t t20 = next;
+        if (p + 32 < end) next = p[32];   // the next entry's load runs during this one's lift
+        const uint32_t h2 = (uint32_t)((kA2 * t20 + kK2) >> 16), h4 = (uint32_t)((kA4 * t20 + kK4) >> 16);
+        const uint32_t P = (uint32_t)T.cx * h2, Q = (uint32_t)T.cz * h4;
+        const uint32_t o0 = (OX ? P : Q) >> m, e0 = (OX ? Q : P) >> m;
+        const uint32_t sx = t20 ^ sc, kq = e0 - rho * o0;
+        uint32_t z = o0;   // its bits 0..3 are right: u only enters from bit 4 (16 u)
+        uint32_t Y = sx >> m;
+        auto settle = [&](int bits) {   // `bits` more bits of z
 #pragma unroll
-    for (int k = 4; k < 32; k += 4) {
-        const uint32_t V = (z - o0) * N.inv;
-        const uint32_t Y = ((s0 ^ (V << 16)) ^ x32) >> m;
-        const uint32_t Aq = kq + N.rho * z;
-        z |= (uint32_t)N.row[(((Aq >> k) & 15u) << 4) | ((Y >> k) & 15u)] << k;
+            for (int q = 0; q < (bits + D - 1) / D; q++) z = Y ^ (kq + rho * z);
+        };
+        settle(12);
+        Y = (sx ^ (((z - o0) * inv) << 16)) >> m;
+        if (M0) {
+            settle(16);
+        } else {
+            settle(4);
+            Y = (sx ^ (((z - o0) * inv) << 16)) >> m;
+            settle(12);
+        }
+        const uint32_t u0 = ((z - o0) * inv) >> 4;
+        if (M0) {
+            check_u(T, t20, h2, h4, u0, hits, cap, cnt);
+        } else {
+            for (uint32_t f = 0; f < (1u << m); f++) check_u(T, t20, h2, h4, (u0 & umask) | (f << (28 - m)), hits, cap, cnt);
+        }
     }
-    const uint32_t u0 = (((z - o0) * N.inv) >> 4) & ((1u << (28 - m)) - 1u);
-    for (uint32_t f = 0; f < (1u << m); f++) check_u(T, t20, h2, h4, u0 | (f << (28 - m)), hits, cap, cnt);
+}
+template <int D>
+__device__ __forceinline__ void lift_list(const ChainTask &T, bool ox, uint32_t inv, uint32_t rho, const uint32_t *list,
+                                          uint32_t n, SolveHitDev *hits, uint32_t cap, unsigned long long *cnt) {
+    if (T.m) {
+        if (ox) lift<D, false, true>(T, inv, rho, list, n, hits, cap, cnt);
+        else lift<D, false, false>(T, inv, rho, list, n, hits, cap, cnt);
+    } else {
+        if (ox) lift<D, true, true>(T, inv, rho, list, n, hits, cap, cnt);
+        else lift<D, true, false>(T, inv, rho, list, n, hits, cap, cnt);
+    }
 }
 
 // v2(cx) == v2(cz): the same substitution with o = cx h2 leaves rho = (cz A^4) / (cx A^2) odd, and
@@ -364,12 +401,12 @@ __global__ void __launch_bounds__(kChainThreads, EQ ? 4 : 6) solve_chain_kernel(
     const int2 *__restrict__ offsets, const uint32_t *__restrict__ keymap, const uint32_t *__restrict__ lists,
     const uint32_t *__restrict__ counts, const uint8_t *__restrict__ nib, uint64_t X, SolveHitDev *hits,
     uint32_t hit_cap, unsigned long long *cnt) {
-    // the class's table: the nibble lift's (2 KB) or the solution masks (4 KB, after it in `nib`)
-    constexpr int kTab = EQ ? kEqTable : kLiftTable;
-    __shared__ __align__(16) uint8_t tab[kTab];
-    const uint8_t *src = nib + (EQ ? kLiftTable : 0);
-    for (int i = threadIdx.x; i < kTab / 16; i += kChainThreads) ((uint4 *)tab)[i] = ((const uint4 *)src)[i];
-    __syncthreads();
+    // the equal class's solution masks (4 KB)
+    __shared__ __align__(16) uint8_t tab[EQ ? kEqTable : 16];
+    if constexpr (EQ) {
+        for (int i = threadIdx.x; i < kEqTable / 16; i += kChainThreads) ((uint4 *)tab)[i] = ((const uint4 *)nib)[i];
+        __syncthreads();
+    }
     const uint16_t *eqtab = reinterpret_cast<const uint16_t *>(tab);
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t)gridDim.x * (kChainThreads / 32);
@@ -407,20 +444,19 @@ __global__ void __launch_bounds__(kChainThreads, EQ ? 4 : 6) solve_chain_kernel(
         if constexpr (EQ) {
             ChunkTask N;
             const uint32_t co = ((uint32_t)T.cx * (uint32_t)kA2) >> T.m, ce = ((uint32_t)T.cz * (uint32_t)kA4) >> T.m;
-            N.coef_o_x = 1u;
             N.inv = inverse_u32(co);
             N.rho = ce * N.inv;
-            N.row = nullptr;
             eq_task(T, N, eqtab + ((N.rho & 15u) >> 1) * 256, list, n, hits, hit_cap, cnt);
         } else {
-            ChunkTask N;
+            const bool ox = vx < vz;
             const uint32_t cxa = (uint32_t)T.cx * (uint32_t)kA2, cza = (uint32_t)T.cz * (uint32_t)kA4;
-            N.coef_o_x = vx < vz ? 1u : 0u;
-            const uint32_t co = (N.coef_o_x ? cxa : cza) >> T.m, ce = (N.coef_o_x ? cza : cxa) >> T.m;
-            N.inv = inverse_u32(co);
-            N.rho = ce * N.inv;
-            N.row = tab + ((N.rho & 15u) >> 1) * 256;
-            for (uint32_t i = lane; i < n; i += 32) lift_chunks(T, N, list[i], hits, hit_cap, cnt);
+            const uint32_t inv = inverse_u32((ox ? cxa : cza) >> T.m), rho = ((ox ? cza : cxa) >> T.m) * inv;
+            switch (min(v2_of(rho), 4)) {   // the same in the whole warp
+                case 1: lift_list<1>(T, ox, inv, rho, list, n, hits, hit_cap, cnt); break;
+                case 2: lift_list<2>(T, ox, inv, rho, list, n, hits, hit_cap, cnt); break;
+                case 3: lift_list<3>(T, ox, inv, rho, list, n, hits, hit_cap, cnt); break;
+                default: lift_list<4>(T, ox, inv, rho, list, n, hits, hit_cap, cnt); break;
+            }
         }
     }
     if (lane == 0 && lifted) atomicAdd(&cnt[SCNT_CANDIDATES], lifted);
@@ -433,7 +469,7 @@ __global__ void __launch_bounds__(kChainThreads, EQ ? 4 : 6) solve_chain_kernel(
 // ---------------------------------------------------------------------------------------------
 struct SolveState {
     uint32_t *hq = nullptr, *hq_off = nullptr;   // region states q0 (mod 2^20) grouped by hut key
-    uint8_t *nib = nullptr;   // [rho mod 16 / 2][a][y] -> x with x ^ ((a + rho x) mod 16) = y (rho even), then the odd-rho masks
+    uint8_t *nib = nullptr;   // [rho mod 16 / 2][a][y] -> mask of x with x ^ ((a + rho x) mod 16) = y, rho odd
     SolveSlot *slots = nullptr;
     SolveKey *keys = nullptr;
     uint32_t *keymap = nullptr, *lists = nullptr, *counts = nullptr;
@@ -495,19 +531,13 @@ int solve_state(wg_engine *eng, SolveState **out) {
         SOLVE_CUDA(cudaMalloc(&s->cnt, sizeof(unsigned long long) * SCNT_WORDS), "solver counters");
         SOLVE_CUDA(cudaMemcpy(s->hq, list.data(), sizeof(uint32_t) << 20, cudaMemcpyHostToDevice), "solver tables");
         SOLVE_CUDA(cudaMemcpy(s->hq_off, off.data(), sizeof(uint32_t) * 65, cudaMemcpyHostToDevice), "solver tables");
-        // the nibble step's solutions, by search: x ^ ((a + 2r x) mod 16) is a bijection of x
-        std::vector<uint8_t> nib(kLiftTable + kEqTable, 0);
-        for (int r = 0; r < 8; r++)
-            for (int a = 0; a < 16; a++)
-                for (int x = 0; x < 16; x++) nib[r * 256 + a * 16 + (x ^ ((a + 2 * r * x) & 15))] = (uint8_t)x;
-        // and the masks of x with x ^ ((a + rho x) mod 16) = y for odd rho = 2r + 1
+        // the masks of x with x ^ ((a + rho x) mod 16) = y for odd rho = 2r + 1, by search
         std::vector<uint16_t> eqm(kEqTable / 2, 0);
         for (int r = 0; r < 8; r++)
             for (int a = 0; a < 16; a++)
                 for (int x = 0; x < 16; x++) eqm[r * 256 + a * 16 + (x ^ ((a + (2 * r + 1) * x) & 15))] |= (uint16_t)(1u << x);
-        std::memcpy(nib.data() + kLiftTable, eqm.data(), kEqTable);
-        SOLVE_CUDA(cudaMalloc(&s->nib, kLiftTable + kEqTable), "solver tables");
-        SOLVE_CUDA(cudaMemcpy(s->nib, nib.data(), kLiftTable + kEqTable, cudaMemcpyHostToDevice), "solver tables");
+        SOLVE_CUDA(cudaMalloc(&s->nib, kEqTable), "solver tables");
+        SOLVE_CUDA(cudaMemcpy(s->nib, eqm.data(), kEqTable, cudaMemcpyHostToDevice), "solver tables");
     }
     *out = eng->solve;
     return WG_OK;
