@@ -1386,6 +1386,14 @@ __device__ __forceinline__ double slot_sample(const Src &src, int slot, int sub,
     return src.p3(slot, keep_precision(px * l), keep_precision(py * l), keep_precision(pz * l));
 }
 
+// The same out of line, for code that takes it at several places: the ladder and the unit kernel cycle
+// through more code than the instruction cache holds as it is.
+template <class Src>
+__device__ __noinline__ double slot_sample_call(const Src src, int slot, int sub, double l, double px, double py,
+                                                double pz) {
+    return slot_sample(src, slot, sub, l, px, py, pz);
+}
+
 // DoublePerlin value from its per-octave samples stored at val[base .. base + 2 np).
 __device__ __forceinline__ double combine(const EntranceSmem &S, int noise, int base, int h, int e) {
     const NoiseSpec &ns = c_noise[noise];
@@ -1669,7 +1677,7 @@ struct LadderSmem {
 };
 
 // Octave-sum of noise `noise` (slots base .. base + 2 np) over stored samples v[slot * stride].
-__device__ __forceinline__ double combine_vals(int noise, const double *v, int stride) {
+__device__ __noinline__ double combine_vals(int noise, const double *v, int stride) {
     const NoiseSpec &ns = c_noise[noise];
     const int np = ns.npresent;
     double a = 0.0, b = 0.0;
@@ -1681,7 +1689,7 @@ __device__ __forceinline__ double combine_vals(int noise, const double *v, int s
 // lysh's ladder for one candidate whose cave tables `src` reads, by all NT threads of the CTA; the
 // survivor, the reject code and the funnel go to the batch.
 template <int NT, class Src>
-__device__ void ladder_candidate(const BatchArgs &a, LadderVals &S, const Src &src, uint64_t seed, uint64_t g,
+__device__ __noinline__ void ladder_candidate(const BatchArgs &a, LadderVals &S, const Src &src, uint64_t seed, uint64_t g,
                                  uint64_t r, int rx, int rz, int cx, int cz, int mh) {
     const int t = threadIdx.x;
     const int large = a.large_biomes ? 1 : 0;
@@ -1748,7 +1756,7 @@ __device__ void ladder_candidate(const BatchArgs &a, LadderVals &S, const Src &s
             px = (double)(hut_x + 3); py = (double)(mh + 10 * hi) * 0.67; pz = (double)(hut_z + 3);
         }
         const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
-        const double v = slot_sample(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
+        const double v = slot_sample_call(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
         if (slot >= kBaseFlood) S.fval[slot - kBaseFlood][hi] = v;
         else S.val[slot][hi] = v;
     }
@@ -1760,7 +1768,7 @@ __device__ void ladder_candidate(const BatchArgs &a, LadderVals &S, const Src &s
         const int hi = k >> 2, slot = kBaseSp1 + (k & 3);
         const double e = S.tun[hi], y = (double)S.ys[hi];
         const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
-        S.val[slot][hi] = slot_sample(src, slot, sub, c_noise[noise].lac[p], (double)hx / e, y / e, (double)hz / e);
+        S.val[slot][hi] = slot_sample_call(src, slot, sub, c_noise[noise].lac[p], (double)hx / e, y / e, (double)hz / e);
     }
     __syncthreads();
     if (t == 0) {
@@ -1819,8 +1827,11 @@ __device__ void ladder_candidate(const BatchArgs &a, LadderVals &S, const Src &s
                     }
             } else {
                 for (long long y = mh; y <= 60; y += 10) {
-                    const double f = dbl3d(src, N_FLOODEDNESS, kBaseFlood, (double)(hut_x + 3),
-                                           (double)y * 0.67, (double)(hut_z + 3));
+                    double pair[2];
+                    for (int q = 0; q < 2; q++)
+                        pair[q] = slot_sample_call(src, kBaseFlood + q, q, c_noise[N_FLOODEDNESS].lac[0],
+                                                   (double)(hut_x + 3), (double)y * 0.67, (double)(hut_z + 3));
+                    const double f = combine_vals(N_FLOODEDNESS, pair, 1);
                     if (f > 0.41) {
                         code = P1_FLOODEDNESS;
                         break;

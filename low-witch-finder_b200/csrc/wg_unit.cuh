@@ -115,7 +115,7 @@ __device__ __forceinline__ uint64_t to_fixed(double v) {
 // with the fixed-point coordinates: the fractions lie within u of the exact ones, G - 1 and L - 1
 // are exact, so a corner dot stays within 3 u and the bound above perlin_y0_f32 holds).
 template <bool F32>
-__device__ __noinline__ float unit_sample_f32(const UnitSmem<F32> &S, int k, uint32_t dx, uint32_t dz) {
+__device__ __forceinline__ float unit_sample_f32(const UnitSmem<F32> &S, int k, uint32_t dx, uint32_t dz) {
     const uint8_t *P = S.tab + (kUClim + k) * kUPitch;
     const uint64_t step = S.fstep[k];
     const uint32_t hx = fixed_hi(S.fx[k], step, dx), hz = fixed_hi(S.fz[k], step, dz);
@@ -503,7 +503,7 @@ __device__ __forceinline__ bool unit_cave_at(const SrcUnit &src, double *v, int 
     // cheese 14, then spaghetti_3d_1 2, spaghetti_3d_2 2 at the scaled point
     auto sample = [&](int slot, double px, double py, double pz) {
         const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
-        return slot_sample(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
+        return slot_sample_call(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
     };
     const double x = (double)hx, y = (double)mh, z = (double)hz;
     if (lane < 24) {
