@@ -39,6 +39,64 @@ struct WalkGeom {
     int rx0, rw, rz0, rh, strips;
 };
 
+// The start test of one region, in 32-bit words of the 48-bit LCG arithmetic (nothing above bit 47 matters, so
+// no state is masked).  The integer pipes bound the walk (issue 72 %, FMA-heavy 75 %, ALU 62 % busy), so its
+// instructions per region count: 83 with 64-bit states masked after every step, 61 now.  One structure seed
+// over the whole world (1.37e10 regions) 42.2 -> 31.2 ms.  Tables of the multiples j a and m b in shared
+// memory instead of the wide multiplies: 31.1 ms, not kept.
+constexpr uint64_t kRegionMulX = 341873128712ull, kRegionMulZ = 132897987541ull;
+constexpr uint32_t kMulLo = 0xDEECE66Du, kMulHi = 5u;   // kDeepMul
+static_assert((((uint64_t)kMulHi << 32) | kMulLo) == kDeepMul, "LCG multiplier words");
+constexpr uint32_t kHutDrawLimit = 2147483640u;   // nextInt(24) re-draws a 31-bit value at or above this
+constexpr uint32_t kStartHiBound = 268435;        // floor(0.004 * 2^53 / 2^27): the start test's 26-bit first draw
+constexpr uint32_t kStartTop16 = kStartHiBound >> 10;   // a start's state has its bits 32..47 at most this
+
+struct StartCtx {
+    uint64_t s48;
+    uint64_t a, b;           // the structure seed's two nextLong() draws
+    uint64_t sx;             // s48 ^ kDeepMul
+};
+__device__ __forceinline__ StartCtx start_ctx(uint64_t s48) {
+    const DeepCtx c = deep_ctx(s48);
+    return StartCtx{c.s48, (uint64_t)c.a, (uint64_t)c.b, c.s48 ^ kDeepMul};
+}
+// s * kDeepMul + 11 from the words of s.
+__device__ __forceinline__ uint64_t lcg_words(uint32_t lo, uint32_t hi) {
+    const uint64_t w = (uint64_t)lo * kMulLo + 11u;
+    return ((uint64_t)((uint32_t)(w >> 32) + lo * kMulHi + hi * kMulLo) << 32) | (uint32_t)w;
+}
+// The rare rest: a hut draw in the re-draw range (8 in 2^31), or a first draw on the start bound itself.
+__device__ __noinline__ bool start_exact(uint64_t s48, int64_t a, int64_t b, int rx, int rz, int &cx, int &cz,
+                                         uint64_t &carver) {
+    hut_chunk(s48, rx, rz, 14357620, cx, cz);
+    const DeepCtx c{s48, a, b};
+    carver = deep_carver(c, cx, cz);
+    return deep_is_start(carver);
+}
+// Whether region (rx, rz)'s hut chunk is a mineshaft start; rs = the region's seed (before setSeed's xor),
+// px = 32 rx a, pz = 32 rz b.  Its chunk and carver state are set when it is.
+__device__ __forceinline__ bool region_start(const StartCtx &c, uint64_t rs, uint64_t px, uint64_t pz, int rx, int rz,
+                                             int &cx, int &cz, uint64_t &carver) {
+    const uint64_t s1 = lcg_words((uint32_t)rs ^ kMulLo, (uint32_t)(rs >> 32) ^ kMulHi);
+    const uint64_t s2 = lcg_words((uint32_t)s1, (uint32_t)(s1 >> 32));
+    const uint32_t u1 = (uint32_t)(s1 >> 17) & 0x7FFFFFFFu, u2 = (uint32_t)(s2 >> 17) & 0x7FFFFFFFu;
+    const uint32_t j = u1 % 24u, m = u2 % 24u;
+    const uint64_t x = px + (uint64_t)j * (uint32_t)c.a, z = pz + (uint64_t)m * (uint32_t)c.b;
+    const uint32_t lo = (uint32_t)x ^ (uint32_t)z ^ (uint32_t)c.sx;
+    const uint32_t hi = ((uint32_t)(x >> 32) + j * (uint32_t)(c.a >> 32)) ^ ((uint32_t)(z >> 32) + m * (uint32_t)(c.b >> 32)) ^
+                        (uint32_t)(c.sx >> 32);
+    const uint64_t w = (uint64_t)lo * kMulLo + 11u;
+    const uint32_t top = ((uint32_t)(w >> 32) + lo * kMulHi + hi * kMulLo) & 0xFFFFu;
+    if (top > kStartTop16 && max(u1, u2) < kHutDrawLimit) return false;
+    const uint32_t hi26 = (top << 10) | ((uint32_t)w >> 22);   // nextDouble()'s first draw
+    if (hi26 == kStartHiBound || max(u1, u2) >= kHutDrawLimit)
+        return start_exact(c.s48, (int64_t)c.a, (int64_t)c.b, rx, rz, cx, cz, carver);
+    cx = rx * 32 + (int)j;
+    cz = rz * 32 + (int)m;
+    carver = (((uint64_t)(hi ^ kMulHi) << 32) | (lo ^ kMulLo)) & kDeepMask48;
+    return hi26 < kStartHiBound;
+}
+
 template <class F>
 __device__ __forceinline__ void walk_task(const WalkGeom &G, uint64_t t, F &&on_start) {
     const int strip = (int)(t % (uint64_t)G.strips);
@@ -47,14 +105,19 @@ __device__ __forceinline__ void walk_task(const WalkGeom &G, uint64_t t, F &&on_
     const uint64_t i = rest / (uint64_t)G.rh;
     if (i >= G.n_seeds) return;
     const uint64_t s48 = (G.s48s ? (uint64_t)G.s48s[i] : G.s48_base + i) & kDeepMask48;
-    const DeepCtx c = deep_ctx(s48);
+    const StartCtx c = start_ctx(s48);
     const int rz = G.rz0 + row;
     const int xa = G.rx0 + strip * kDeepCols, xb = min(G.rx0 + G.rw, xa + kDeepCols);
+    uint64_t rs = (uint64_t)(int64_t)xa * kRegionMulX + (uint64_t)(int64_t)rz * kRegionMulZ + s48 + 14357620ull;
+    uint64_t px = (uint64_t)((int64_t)xa * 32) * c.a;
+    const uint64_t pz = (uint64_t)((int64_t)rz * 32) * c.b;
+#pragma unroll 4
     for (int rx = xa; rx < xb; rx++) {
         int cx, cz;
-        hut_chunk(s48, rx, rz, 14357620, cx, cz);
-        const uint64_t carver = deep_carver(c, cx, cz);
-        if (deep_is_start(carver)) on_start(i, s48, rx, rz, cx, cz, carver);
+        uint64_t carver;
+        if (region_start(c, rs, px, pz, rx, rz, cx, cz, carver)) on_start(i, s48, rx, rz, cx, cz, carver);
+        rs += kRegionMulX;
+        px += 32ull * c.a;
     }
 }
 
@@ -143,10 +206,6 @@ __global__ void __launch_bounds__(kDeepThreads) walk_write_kernel(WalkGeom G, ui
 // ------------------------------------------------------------------------------------
 constexpr int kSweepRows = 64;
 constexpr uint64_t kSweepPassTasks = 1ull << 24;
-constexpr uint64_t kRegionMulX = 341873128712ull, kRegionMulZ = 132897987541ull;
-constexpr uint32_t kHutDrawLimit = 2147483640u;   // nextInt(24) re-draws a 31-bit value at or above this
-constexpr uint64_t kStartHiBound = 268435;        // floor(0.004 * 2^53 / 2^27): the start test's first draw
-
 struct SweepMatch {
     uint64_t seed_index;
     int64_t s48;
@@ -163,10 +222,16 @@ struct SweepGeom {
     const uint64_t *keys;                // catalogued layouts, sorted ascending
     const uint32_t *vals;
     uint32_t n_keys;
+    const uint32_t *filter;              // kFilterBits bits: set where a layout has these low bits
 };
 
+// One bit per value of a layout's low 16 bits: a start (0.4 % of the regions) that no layout of the
+// catalogue resembles takes one load instead of the binary search, which ran in 12 % of the warps' steps.
+constexpr uint32_t kFilterBits = 1u << 16;
 // Index of carver in the sorted catalogue, or -1.
 __device__ __forceinline__ int catalogue_find(const SweepGeom &G, uint64_t carver) {
+    const uint32_t f = (uint32_t)carver & (kFilterBits - 1u);
+    if (!((G.filter[f >> 5] >> (f & 31u)) & 1u)) return -1;
     uint32_t lo = 0, hi = G.n_keys;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
@@ -174,15 +239,6 @@ __device__ __forceinline__ int catalogue_find(const SweepGeom &G, uint64_t carve
         else hi = mid;
     }
     return (lo < G.n_keys && G.keys[lo] == carver) ? (int)lo : -1;
-}
-
-// nextInt(24) of a java.util.Random state right after setSeed: the state after the draw, the value
-// in v; false when the 31-bit draw falls in the re-draw range (the caller takes the exact path).
-__device__ __forceinline__ bool draw24(uint64_t &st, int &v) {
-    st = deep_step(st);
-    const uint32_t u = (uint32_t)(st >> 17);
-    v = (int)(u % 24u);
-    return u < kHutDrawLimit;
 }
 
 __global__ void __launch_bounds__(kDeepThreads) sweep_kernel(SweepGeom G, uint64_t t0, uint64_t n_tasks,
@@ -199,31 +255,17 @@ __global__ void __launch_bounds__(kDeepThreads) sweep_kernel(SweepGeom G, uint64
         const int seg = (int)(rest % (uint64_t)G.segs);
         i = rest / (uint64_t)G.segs;
         const uint64_t s48 = (G.s48s ? (uint64_t)G.s48s[i] : G.s48_base + i) & kDeepMask48;
-        const DeepCtx c = deep_ctx(s48);
+        const StartCtx c = start_ctx(s48);
         const int rx = G.rx0 + col;
         const int za = G.rz0 + seg * kSweepRows, zb = min(G.rz0 + G.rh, za + kSweepRows);
-        // region seed (low 48 bits suffice: setSeed masks to 48 bits) and the carver's row terms
         uint64_t rs = (uint64_t)(int64_t)rx * kRegionMulX + (uint64_t)(int64_t)za * kRegionMulZ + s48 + 14357620ull;
-        const uint64_t px = (uint64_t)((int64_t)rx * 32) * (uint64_t)c.a;
-        uint64_t pz = (uint64_t)((int64_t)za * 32) * (uint64_t)c.b;
-#pragma unroll 4   // rows are independent apart from the two running sums: four in flight (4 structure seeds over the whole world: 156.5 vs 159.9 ms)
+        const uint64_t px = (uint64_t)((int64_t)rx * 32) * c.a;
+        uint64_t pz = (uint64_t)((int64_t)za * 32) * c.b;
+#pragma unroll 4   // rows are independent apart from the two running sums
         for (int rz = za; rz < zb; rz++) {
-            uint64_t st = (rs ^ kDeepMul) & kDeepMask48;
-            int j, m;
-            const bool ok1 = draw24(st, j), ok2 = draw24(st, m);
-            int cx = rx * 32 + j, cz = rz * 32 + m;
+            int cx, cz;
             uint64_t carver;
-            if (ok1 && ok2) {
-                carver = ((px + (uint64_t)(int64_t)j * (uint64_t)c.a) ^ (pz + (uint64_t)(int64_t)m * (uint64_t)c.b) ^ s48) &
-                         kDeepMask48;
-            } else {   // a re-draw: the exact placement
-                hut_chunk(s48, rx, rz, 14357620, cx, cz);
-                carver = deep_carver(c, cx, cz);
-            }
-            const uint64_t s1 = deep_step((carver ^ kDeepMul) & kDeepMask48);
-            const uint64_t hi = s1 >> 22;
-            const bool start = hi < kStartHiBound || (hi == kStartHiBound && deep_is_start(carver));
-            if (start) {
+            if (region_start(c, rs, px, pz, rx, rz, cx, cz, carver)) {
                 n_starts++;
                 const int at = catalogue_find(G, carver);
                 if (at >= 0) {
@@ -232,7 +274,7 @@ __global__ void __launch_bounds__(kDeepThreads) sweep_kernel(SweepGeom G, uint64
                 }
             }
             rs += kRegionMulZ;
-            pz += 32ull * (uint64_t)c.b;
+            pz += 32ull * c.b;
         }
     }
     // starts per structure seed: one warp sum when the warp's lanes share a seed (lanes past the
@@ -264,7 +306,7 @@ struct WalkState {
     uint64_t cap_s48 = 0, cap_out = 0;
     // forward sweep: catalogue, per-seed start counts, matches
     uint64_t *keys = nullptr;
-    uint32_t *vals = nullptr;
+    uint32_t *vals = nullptr, *filter = nullptr;
     unsigned long long *starts = nullptr, *n_match = nullptr;
     SweepMatch *match = nullptr;
     uint64_t cap_keys = 0, cap_starts = 0;
@@ -281,6 +323,7 @@ void walk_release(wg_engine *eng) {
     cudaFree(w->total);
     cudaFree(w->keys);
     cudaFree(w->vals);
+    cudaFree(w->filter);
     cudaFree(w->starts);
     cudaFree(w->n_match);
     cudaFree(w->match);
@@ -362,7 +405,11 @@ extern "C" int wg_deep_sweep(wg_engine *eng, const uint64_t *layouts, const uint
     if (!w.match) {
         DEEP_CUDA(cudaMalloc(&w.match, sizeof(SweepMatch) * kSweepMatchCap), "sweep matches");
         DEEP_CUDA(cudaMalloc(&w.n_match, sizeof(unsigned long long)), "sweep matches");
+        DEEP_CUDA(cudaMalloc(&w.filter, kFilterBits / 8), "sweep filter");
     }
+    std::vector<uint32_t> filter(kFilterBits / 32, 0u);
+    for (const uint64_t k : keys) filter[(k & (kFilterBits - 1u)) >> 5] |= 1u << (k & 31u);
+    DEEP_CUDA(cudaMemcpyAsync(w.filter, filter.data(), kFilterBits / 8, cudaMemcpyHostToDevice, st), "upload");
     DEEP_CUDA(cudaMemcpyAsync(w.keys, keys.data(), sizeof(uint64_t) * keys.size(), cudaMemcpyHostToDevice, st), "upload");
     DEEP_CUDA(cudaMemcpyAsync(w.vals, vals.data(), sizeof(uint32_t) * vals.size(), cudaMemcpyHostToDevice, st), "upload");
     rc = upload_seeds(eng, w, s48, n);
@@ -381,6 +428,7 @@ extern "C" int wg_deep_sweep(wg_engine *eng, const uint64_t *layouts, const uint
     G.keys = w.keys;
     G.vals = w.vals;
     G.n_keys = (uint32_t)keys.size();
+    G.filter = w.filter;
     const uint64_t n_tasks = n * (uint64_t)G.segs * (uint64_t)G.rw;
     for (uint64_t t0 = 0; t0 < n_tasks; t0 += kSweepPassTasks) {
         const uint64_t m = std::min<uint64_t>(kSweepPassTasks, n_tasks - t0);
