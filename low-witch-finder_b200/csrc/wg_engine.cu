@@ -178,11 +178,14 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
     a.n_units = n_units;
     const bool spots = !a.unit_cta && spot_path(a.jobs != nullptr, (uint64_t)a.tw * a.th, a.codes != nullptr, a.single_biome != 0);
     const bool lists = !spots && list_path(a, n_units);
-    if (lists) {
+    // one-region units: their climate stage is its own, the cave gate's list kernels from kSpotListUnits on
+    const bool spot_lists = spots && a.fp32_core == 1 && n_units >= kSpotListUnits;
+    if (lists || spot_lists) {
         int rc = list_buffers(eng);
         if (rc) return rc;
         a.lists[0] = eng->lists[0];
         a.lists[1] = eng->lists[1];
+        if (spot_lists) a.lists[0].cnt = CNT_CLIMATE_LIST;
     }
     WG_CUDA(cudaMemsetAsync(eng->counters, 0, sizeof(uint32_t) * CNT_WORDS, eng->stream), "memset counters");
     WG_CUDA(cudaMemsetAsync(eng->hist, 0, sizeof(unsigned long long) * (P1_KINDS + kTiers), eng->stream),

@@ -174,6 +174,8 @@ struct Sink {            // where phase-1 survivors go after each batch
 // 358 and 391 us, 24,576 482 and 467, 131,072 2,030 and 1,650; 1 x 2 regions: 228 and 270, 296 and 297,
 // 1,048 and 679).
 constexpr uint32_t kListUnits = 24576;
+// The same for the cave gate of one-region units, 1.7 % of which reach it.
+constexpr uint32_t kSpotListUnits = 1u << 19;
 // Allocates the list kernels' lists once per engine.
 int list_buffers(wg_engine *eng);
 // Whether a batch of n_units units takes the list kernels.

@@ -718,23 +718,34 @@ static void prepare_list_launches() {
     }
 }
 
+static RegionList stage_list(const BatchArgs &a, int list, int cnt) {
+    RegionList L = a.lists[list];
+    L.cnt = cnt;
+    return L;
+}
+
+// The first entrance tests for the climate survivors in lists[0].
+static void launch_cave_lists(const BatchArgs &a, cudaStream_t s) {
+    prepare_list_launches();
+    const int gate = g_list_sms * g_gate_per_sm;
+    const RegionList none{}, open = stage_list(a, 2, CNT_RECORDS);
+    gate_kernel<G_SCALED><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 0, CNT_CLIMATE_LIST),
+                                                                    stage_list(a, 1, CNT_SCALED_LIST), open);
+    gate_kernel<G_ENTRANCE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 1, CNT_SCALED_LIST),
+                                                                      stage_list(a, 0, CNT_ENTRANCE_LIST), open);
+    gate_kernel<G_ROUGH><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 0, CNT_ENTRANCE_LIST), none, open);
+}
+
 // The climate and entrance stages of a batch: grids of the resident CTAs, whose warps take groups of
 // units or records in turn.  lists[0], lists[1] alternate; lists[2] is the entrance kernel's input.
 void launch_lists(const BatchArgs &a, cudaStream_t s) {
     prepare_list_launches();
     const int gate = g_list_sms * g_gate_per_sm;
-    auto from = [&](int list, int cnt) {
-        RegionList L = a.lists[list];
-        L.cnt = cnt;
-        return L;
-    };
     BatchArgs b = a;
     b.lists[0].cnt = CNT_EROSION_LIST;
     erosion_kernel<<<g_list_sms * g_ero_per_sm, kEThreads, sizeof(ErosionSmem), s>>>(b);
-    const RegionList none{}, open = from(2, CNT_RECORDS);
-    gate_kernel<G_TEMPERATURE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, from(0, CNT_EROSION_LIST), from(1, CNT_TEMP_LIST), none);
-    gate_kernel<G_RIDGE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, from(1, CNT_TEMP_LIST), from(0, CNT_CLIMATE_LIST), none);
-    gate_kernel<G_SCALED><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, from(0, CNT_CLIMATE_LIST), from(1, CNT_SCALED_LIST), open);
-    gate_kernel<G_ENTRANCE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, from(1, CNT_SCALED_LIST), from(0, CNT_ENTRANCE_LIST), open);
-    gate_kernel<G_ROUGH><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, from(0, CNT_ENTRANCE_LIST), none, open);
+    const RegionList none{};
+    gate_kernel<G_TEMPERATURE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 0, CNT_EROSION_LIST), stage_list(a, 1, CNT_TEMP_LIST), none);
+    gate_kernel<G_RIDGE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 1, CNT_TEMP_LIST), stage_list(a, 0, CNT_CLIMATE_LIST), none);
+    launch_cave_lists(a, s);
 }

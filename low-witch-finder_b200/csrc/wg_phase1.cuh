@@ -233,7 +233,6 @@ size_t climate_smem_bytes(bool fp32_core);
 // two item lists of `cap` entries (counts: 2 words, device); climate survivors become records.
 void launch_spot_climate(const BatchArgs &a, SpotItem *list0, SpotItem *list1, uint32_t *counts, uint32_t cap,
                          int sm_count, cudaStream_t s);
-size_t spot_smem_bytes();
 size_t entrance_smem_bytes();
 // The FP32 core's error probe: noise `noise` (NoiseId) of seed d_seeds[b] at y = 0 and the n_points
 // (x, z) of d_xz, FP32 core -> d_out32[b * n_points + i], FP64 -> d_out64[...].
