@@ -1453,12 +1453,16 @@ struct LadderVals {
     double fval[2][kFloodHeights];           // floodedness samples
     double tun[kLadderHeights];
     int ys[kLadderHeights];
+    uint32_t fails;                          // bit h: cave at height index h; kFailCont, kFailFlood
 };
+constexpr uint32_t kFailCont = 1u << 16, kFailFlood = 1u << 17;
 
 struct LadderSmem {
     uint8_t perm[256 * kLadderStride];       // slot s, row k at k * kLadderStride + s
     double org[kSlotsC * 3];
     LadderVals v;
+    double first[28];                        // the first test's samples
+    bool cave;
     uint32_t grad[kGradWords];
 };
 
@@ -1485,7 +1489,10 @@ __device__ __noinline__ void ladder_candidate(const BatchArgs &a, LadderVals &S,
     int floor_y = (-40 < mh) ? -40 : mh;
     if (floor_y < -50) floor_y = -50;
     int nh = 0;
-    if (t == 0) S.ys[nh] = mh;
+    if (t == 0) {
+        S.ys[nh] = mh;
+        S.fails = 0;
+    }
     nh++;
     for (int y = 0; y >= floor_y; y -= 10)
         if (mh < y) {
@@ -1557,71 +1564,56 @@ __device__ __noinline__ void ladder_candidate(const BatchArgs &a, LadderVals &S,
         S.val[slot][hi] = slot_sample_call(src, slot, sub, c_noise[noise].lac[p], (double)hx / e, y / e, (double)hz / e);
     }
     __syncthreads();
-    if (t == 0) {
-        // lysh_phase1_check_ex from the cave at maxHeight on (phase1.c:149-199)
-        auto spag = [&](int hi) {
-            const double e = S.tun[hi];
-            const double tv = combine_vals(N_SPAGHETTI_THICKNESS, &S.val[kBaseThickness][hi], kLadderHeights);
-            const double h = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
-            const double l = combine_vals(N_SPAGHETTI_1, &S.val[kBaseSp1][hi], kLadderHeights);
-            const double m = fabs(e * l) - h;
-            const double n = combine_vals(N_SPAGHETTI_2, &S.val[kBaseSp2][hi], kLadderHeights);
-            const double o = fabs(e * n) - h;
-            const double pp = clampd(jmax(m, o), -1.0, 1.0);
-            const double mod = combine_vals(N_ROUGHNESS_MODULATOR, &S.val[kBaseRmod][hi], kLadderHeights);
-            const double rgh = combine_vals(N_ROUGHNESS, &S.val[kBaseRough][hi], kLadderHeights);
-            const double qq = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
-            return pp + qq;
-        };
-        auto chz = [&](int hi) {
-            const double layer = combine_vals(N_CAVE_LAYER, &S.val[kBaseLayer][hi], kLadderHeights);
-            const double av = 4.0 * layer * layer;
-            const double raw = combine_vals(N_CAVE_CHEESE, &S.val[kBaseCheese][hi], kLadderHeights);
-            return av + clampd(0.27 + raw, -1.0, 1.0);
-        };
-        int code = P1_ACCEPT;
-        if (spag(0) >= 0 && chz(0) >= 0) code = P1_CAVE_AT_MAXH;
-        if (code == P1_ACCEPT)
-            for (int hi = 1; hi < first_pos; hi++)
-                if (spag(hi) >= 0 && chz(hi) >= 0) {
-                    code = P1_LADDER_NEG;
-                    break;
-                }
-        if (code == P1_ACCEPT)
-            for (int hi = first_pos; hi < nh; hi++) {
-                const int y = S.ys[hi];
-                const double ent = combine_vals(N_CAVE_ENTRANCE, &S.val[kBaseEntrance][hi], kLadderHeights);
-                const double tt = (10.0 + (double)y) / 40.0;
-                const double cl = tt < 0.0 ? 0.3 : (tt > 1.0 ? 0.0 : lerp(tt, 0.3, 0.0));
-                const double cc = ent + 0.37 + cl;
-                if (jmin(cc, spag(hi)) >= 0 && chz(hi) >= 0) {
-                    code = P1_LADDER_POS;
-                    break;
-                }
-            }
-        if (code == P1_ACCEPT && !a.single_biome) {
-            // the y = 0 climate sample equals the 3-D sample at y = 0 bit for bit
-            const double c = combine_vals(cont_noise, &S.val[kBaseCont][0], kLadderHeights);
-            if (c < -0.11) code = P1_CONTINENTALNESS;
+    // Every verdict of the ladder by its own thread: one per height, one for the continentalness, one per
+    // flood height; then the first of them in lysh's order (phase1.c:149-199).
+    if (t < nh) {
+        const double e = S.tun[t];
+        const double tv = combine_vals(N_SPAGHETTI_THICKNESS, &S.val[kBaseThickness][t], kLadderHeights);
+        const double h = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
+        const double l = combine_vals(N_SPAGHETTI_1, &S.val[kBaseSp1][t], kLadderHeights);
+        const double m = fabs(e * l) - h;
+        const double n = combine_vals(N_SPAGHETTI_2, &S.val[kBaseSp2][t], kLadderHeights);
+        const double o = fabs(e * n) - h;
+        const double pp = clampd(jmax(m, o), -1.0, 1.0);
+        const double mod = combine_vals(N_ROUGHNESS_MODULATOR, &S.val[kBaseRmod][t], kLadderHeights);
+        const double rgh = combine_vals(N_ROUGHNESS, &S.val[kBaseRough][t], kLadderHeights);
+        const double qq = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
+        double cave = pp + qq;
+        if (t >= first_pos) {
+            const double ent = combine_vals(N_CAVE_ENTRANCE, &S.val[kBaseEntrance][t], kLadderHeights);
+            const double tt = (10.0 + (double)S.ys[t]) / 40.0;
+            const double cl = tt < 0.0 ? 0.3 : (tt > 1.0 ? 0.0 : lerp(tt, 0.3, 0.0));
+            cave = jmin(ent + 0.37 + cl, cave);
         }
-        if (code == P1_ACCEPT) {
-            if (nf_ll <= kFloodHeights) {
-                for (int fi = 0; fi < nf; fi++)
-                    if (combine_vals(N_FLOODEDNESS, &S.fval[0][fi], kFloodHeights) > 0.41) {
-                        code = P1_FLOODEDNESS;
-                        break;
-                    }
-            } else {
-                for (long long y = mh; y <= 60; y += 10) {
-                    double pair[2];
-                    for (int q = 0; q < 2; q++)
-                        pair[q] = slot_sample_call(src, kBaseFlood + q, q, c_noise[N_FLOODEDNESS].lac[0],
-                                                   (double)(hut_x + 3), (double)y * 0.67, (double)(hut_z + 3));
-                    const double f = combine_vals(N_FLOODEDNESS, pair, 1);
-                    if (f > 0.41) {
-                        code = P1_FLOODEDNESS;
-                        break;
-                    }
+        if (cave >= 0) {
+            const double layer = combine_vals(N_CAVE_LAYER, &S.val[kBaseLayer][t], kLadderHeights);
+            const double av = 4.0 * layer * layer;
+            const double raw = combine_vals(N_CAVE_CHEESE, &S.val[kBaseCheese][t], kLadderHeights);
+            if (av + clampd(0.27 + raw, -1.0, 1.0) >= 0) atomicOr(&S.fails, 1u << t);
+        }
+    } else if (t == 16 && !a.single_biome) {
+        // the y = 0 climate sample equals the 3-D sample at y = 0 bit for bit
+        if (combine_vals(cont_noise, &S.val[kBaseCont][0], kLadderHeights) < -0.11) atomicOr(&S.fails, kFailCont);
+    } else if (t >= 32 && t < 32 + nf) {
+        if (combine_vals(N_FLOODEDNESS, &S.fval[0][t - 32], kFloodHeights) > 0.41) atomicOr(&S.fails, kFailFlood);
+    }
+    __syncthreads();
+    if (t == 0) {
+        const uint32_t f = S.fails, neg = (1u << first_pos) - 2u, pos = (1u << nh) - (1u << first_pos);
+        int code = f & 1u ? P1_CAVE_AT_MAXH
+                   : f & neg ? P1_LADDER_NEG
+                   : f & pos ? P1_LADDER_POS
+                   : f & kFailCont ? P1_CONTINENTALNESS
+                   : f & kFailFlood ? P1_FLOODEDNESS : P1_ACCEPT;
+        if (code == P1_ACCEPT && nf_ll > kFloodHeights) {
+            for (long long y = mh; y <= 60; y += 10) {
+                double pair[2];
+                for (int q = 0; q < 2; q++)
+                    pair[q] = slot_sample_call(src, kBaseFlood + q, q, c_noise[N_FLOODEDNESS].lac[0],
+                                               (double)(hut_x + 3), (double)y * 0.67, (double)(hut_z + 3));
+                if (combine_vals(N_FLOODEDNESS, pair, 1) > 0.41) {
+                    code = P1_FLOODEDNESS;
+                    break;
                 }
             }
         }
@@ -1644,6 +1636,51 @@ __device__ __noinline__ void ladder_candidate(const BatchArgs &a, LadderVals &S,
         }
     }
     __syncthreads();
+}
+
+// The ladder's first test for one candidate, by one warp: cave at maxHeight (spaghetti and cheese
+// both >= 0), where 92 % of the candidates end.  v: kMhSamples doubles of the warp's.
+constexpr int kMhSamples = 28;   // spaghetti (12) and cheese (16) samples of one height
+template <class Src>
+__device__ __forceinline__ bool cave_at_max_height(const Src &src, double *v, int hx, int hz, int mh, int large) {
+    const int lane = threadIdx.x & 31;
+    // samples in the order rarity 2, thickness 2, roughness modulator 2, roughness 2, layer 2,
+    // cheese 14, then spaghetti_3d_1 2, spaghetti_3d_2 2 at the scaled point
+    auto sample = [&](int slot, double px, double py, double pz) {
+        const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
+        return slot_sample_call(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
+    };
+    const double x = (double)hx, y = (double)mh, z = (double)hz;
+    if (lane < 24) {
+        const int slot = lane < 4 ? kBaseRarity + lane : (lane < 8 ? kBaseRmod + (lane - 4) : kBaseLayer + (lane - 8));
+        double px = x, py = y, pz = z;
+        if (lane < 2) {
+            px = (double)(int)((uint32_t)hx * 2u);
+            pz = (double)(int)((uint32_t)hz * 2u);
+        } else if (lane >= 10) {
+            py = y * 0.6666666666666666;
+        } else if (lane >= 8) {
+            py = (double)(int)((uint32_t)mh * 8u);
+        }
+        v[lane] = sample(slot, px, py, pz);
+    }
+    __syncwarp();
+    const double e = tunnel_scale(combine_vals(N_SPAGHETTI_RARITY, v, 1));
+    if (lane < 4) v[24 + lane] = sample(kBaseSp1 + lane, x / e, y / e, z / e);
+    __syncwarp();
+    const double tv = combine_vals(N_SPAGHETTI_THICKNESS, v + 2, 1);
+    const double h = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
+    const double m = fabs(e * combine_vals(N_SPAGHETTI_1, v + 24, 1)) - h;
+    const double o = fabs(e * combine_vals(N_SPAGHETTI_2, v + 26, 1)) - h;
+    const double p = clampd(jmax(m, o), -1.0, 1.0);
+    const double mod = combine_vals(N_ROUGHNESS_MODULATOR, v + 4, 1), rgh = combine_vals(N_ROUGHNESS, v + 6, 1);
+    const double q = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
+    const double layer = combine_vals(N_CAVE_LAYER, v + 8, 1);
+    const double av = 4.0 * layer * layer;
+    const double raw = combine_vals(N_CAVE_CHEESE, v + 10, 1);
+    const bool cave = p + q >= 0 && av + clampd(0.27 + raw, -1.0, 1.0) >= 0;
+    __syncwarp();   // v is free for the warp's next candidate
+    return cave;
 }
 
 __global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(const __grid_constant__ BatchArgs a) {
@@ -1674,7 +1711,23 @@ __global__ void __launch_bounds__(kThreadsC, 10) ladder_kernel(const __grid_cons
             S.org[3 * t + 2] = oz;
         }
         __syncthreads();
-        ladder_candidate<kThreadsC>(a, S.v, src, seed, up.g, up.region(jr), rx, rz, cx, cz, up.max_height);
+        // With more candidates than CTAs, 92 % of them end at a first test of 28 samples by one warp (8.9 ->
+        // 8.0 ms per 2^24 seeds x 9 x 9); with fewer the test only delays the ladder (4,096 seeds: 35 -> 41 us).
+        if (t == 0) S.cave = false;
+        if (n_deep > gridDim.x && t < 32) {
+            const bool cave = cave_at_max_height(src, S.first, cx * 16 + 3, cz * 16 + 3, up.max_height, large);
+            if (t == 0) {
+                S.cave = cave;
+                if (cave) {
+                    atomicAdd(&a.hist[P1_CAVE_AT_MAXH], 1ull);
+                    note_code(a, up.g, up.region(jr), P1_CAVE_AT_MAXH, -1);
+                }
+            }
+        }
+        __syncthreads();
+        if (!S.cave)
+            ladder_candidate<kThreadsC>(a, S.v, src, seed, up.g, up.region(jr), rx, rz, cx, cz, up.max_height);
+        __syncthreads();   // S.cave and the tables are free for the next candidate
     }
 }
 

@@ -38,7 +38,6 @@ constexpr int kList = kBlock * kBlock / kUWarps;   // a warp's regions of a bloc
 constexpr int kPoolFull = kUWarps * 64;       // pooled regions that start a drain: two full rounds a warp
 constexpr int kPool = kPoolFull + kBlock * kBlock;
 constexpr int kUSurv = kUThreads + kUWarps * kList;   // what waited and one drain's
-constexpr int kMhSamples = 28;                // spaghetti (12) and cheese (16) samples of one height
 constexpr int kUDeep = 256;                   // deep candidates finished here; more go to the ladder kernel's list
 static_assert(kUClim + kSlotsA <= kUTabs, "climate tables overlay ladder tables");
 
@@ -495,49 +494,6 @@ __device__ __noinline__ double unit_quick(const UnitSmem<F32> &S, int noise, int
     }
 }
 
-// The ladder's first test for one candidate, by one warp: cave at maxHeight (spaghetti and cheese
-// both >= 0), where 92 % of the candidates end.  v: kMhSamples doubles of the warp's.
-__device__ __forceinline__ bool unit_cave_at(const SrcUnit &src, double *v, int hx, int hz, int mh, int large) {
-    const int lane = threadIdx.x & 31;
-    // samples in the order rarity 2, thickness 2, roughness modulator 2, roughness 2, layer 2,
-    // cheese 14, then spaghetti_3d_1 2, spaghetti_3d_2 2 at the scaled point
-    auto sample = [&](int slot, double px, double py, double pz) {
-        const int noise = c_slot_c[large][slot][0], sub = c_slot_c[large][slot][1], p = c_slot_c[large][slot][2];
-        return slot_sample_call(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
-    };
-    const double x = (double)hx, y = (double)mh, z = (double)hz;
-    if (lane < 24) {
-        const int slot = lane < 4 ? kBaseRarity + lane : (lane < 8 ? kBaseRmod + (lane - 4) : kBaseLayer + (lane - 8));
-        double px = x, py = y, pz = z;
-        if (lane < 2) {
-            px = (double)(int)((uint32_t)hx * 2u);
-            pz = (double)(int)((uint32_t)hz * 2u);
-        } else if (lane >= 10) {
-            py = y * 0.6666666666666666;
-        } else if (lane >= 8) {
-            py = (double)(int)((uint32_t)mh * 8u);
-        }
-        v[lane] = sample(slot, px, py, pz);
-    }
-    __syncwarp();
-    const double e = tunnel_scale(combine_vals(N_SPAGHETTI_RARITY, v, 1));
-    if (lane < 4) v[24 + lane] = sample(kBaseSp1 + lane, x / e, y / e, z / e);
-    __syncwarp();
-    const double tv = combine_vals(N_SPAGHETTI_THICKNESS, v + 2, 1);
-    const double h = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
-    const double m = fabs(e * combine_vals(N_SPAGHETTI_1, v + 24, 1)) - h;
-    const double o = fabs(e * combine_vals(N_SPAGHETTI_2, v + 26, 1)) - h;
-    const double p = clampd(jmax(m, o), -1.0, 1.0);
-    const double mod = combine_vals(N_ROUGHNESS_MODULATOR, v + 4, 1), rgh = combine_vals(N_ROUGHNESS, v + 6, 1);
-    const double q = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
-    const double layer = combine_vals(N_CAVE_LAYER, v + 8, 1);
-    const double av = 4.0 * layer * layer;
-    const double raw = combine_vals(N_CAVE_CHEESE, v + 10, 1);
-    const bool cave = p + q >= 0 && av + clampd(0.27 + raw, -1.0, 1.0) >= 0;
-    __syncwarp();   // v is free for the warp's next candidate
-    return cave;
-}
-
 // One CTA per unit.  F32: the FP32 noise core with the block lattices (small coordinates only), else
 // FP64 samples throughout, in the reference's order.
 template <bool F32>
@@ -871,7 +827,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
         const SrcUnit src{S.tab, S.org, S.grad};
         for (uint32_t q = (uint32_t)warp; q < n_deep; q += kUWarps) {   // S.und is empty here
             const uint32_t e = S.deep[q];
-            const bool cave = unit_cave_at(src, S.mh[warp], (U.ucx + (int)(e & 0xFFFFu)) * 16 + 3,
+            const bool cave = cave_at_max_height(src, S.mh[warp], (U.ucx + (int)(e & 0xFFFFu)) * 16 + 3,
                                            (U.ucz + (int)(e >> 16)) * 16 + 3, U.up.max_height, large);
             if (lane == 0) {
                 if (cave) {
