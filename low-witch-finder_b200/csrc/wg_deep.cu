@@ -514,7 +514,10 @@ extern "C" int wg_deep_starts(wg_engine *eng, const int64_t *s48, int64_t s48_ba
     DEEP_CUDA(cudaStreamSynchronize(st), "deep starts");
     if (found > dcap && cap > dcap) return eng->fail(WG_ERR_CAPACITY, "deep starts: more than 2^24 hits in one call");
     const uint64_t nw = std::min<uint64_t>(cap, found);
-    if (nw) DEEP_CUDA(cudaMemcpy(out, w.out, sizeof(DeepHit) * nw, cudaMemcpyDeviceToHost), "copy hits");
+    if (nw) {
+        const int rc = copy_result(eng, out, w.out, sizeof(DeepHit) * nw);
+        if (rc) return rc;
+    }
     if (n_out) *n_out = found;
     return WG_OK;
 }

@@ -3,11 +3,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/witchgpu.h"
@@ -187,9 +189,7 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
         a.lists[1] = eng->lists[1];
         if (spot_lists) a.lists[0].cnt = CNT_CLIMATE_LIST;
     }
-    WG_CUDA(cudaMemsetAsync(eng->counters, 0, sizeof(uint32_t) * CNT_WORDS, eng->stream), "memset counters");
-    WG_CUDA(cudaMemsetAsync(eng->hist, 0, sizeof(unsigned long long) * (P1_KINDS + kTiers), eng->stream),
-            "memset hist");
+    WG_CUDA(cudaMemsetAsync(eng->counters, 0, kCountBytes, eng->stream), "memset counters");   // and the funnel behind them
     WG_CUDA(cudaEventRecord(eng->kev[0], eng->stream), "event");
     // one region per unit: the climate tables are built lazily, breadth first
     if (spots) {
@@ -208,31 +208,34 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
         launch_climate(a, eng->stream);
     }
     WG_CUDA(cudaEventRecord(eng->kev[1], eng->stream), "event");
-    if (!a.unit_cta) launch_entrance(a, 0, eng->stream);
-    WG_CUDA(cudaEventRecord(eng->kev[2], eng->stream), "event");
-    if (!a.unit_cta) launch_ladder(a, 0, eng->stream);
-    WG_CUDA(cudaEventRecord(eng->kev[3], eng->stream), "event");
+    if (!a.unit_cta) {
+        launch_entrance(a, 0, eng->stream);
+        WG_CUDA(cudaEventRecord(eng->kev[2], eng->stream), "event");
+        launch_ladder(a, 0, eng->stream);
+        WG_CUDA(cudaEventRecord(eng->kev[3], eng->stream), "event");
+    }
     WG_CUDA(cudaGetLastError(), "kernel launch");
+    bool ladder = !a.unit_cta;
     for (int pass = 0;; pass++) {
-        WG_CUDA(cudaMemcpyAsync(eng->h_counters, eng->counters, sizeof(uint32_t) * CNT_WORDS, cudaMemcpyDeviceToHost,
-                                eng->stream),
+        WG_CUDA(cudaMemcpyAsync(eng->h_counters, eng->counters, kCountBytes, cudaMemcpyDeviceToHost, eng->stream),
                 "copy counters");
-        WG_CUDA(cudaMemcpyAsync(eng->h_hist, eng->hist, sizeof(unsigned long long) * (P1_KINDS + kTiers),
-                                cudaMemcpyDeviceToHost, eng->stream),
-                "copy hist");
+        WG_CUDA(cudaEventRecord(eng->ev1, eng->stream), "event");   // the end of the last batch's device work
         WG_CUDA(cudaStreamSynchronize(eng->stream), "batch");
         // candidates past a unit's own list go through the ladder kernel (seldom any)
-        if (!a.unit_cta || pass || !eng->h_counters[CNT_DEEP] || eng->h_counters[CNT_OVERFLOW]) break;
+        if (ladder || pass || !eng->h_counters[CNT_DEEP] || eng->h_counters[CNT_OVERFLOW]) break;
+        WG_CUDA(cudaEventRecord(eng->kev[2], eng->stream), "event");
         launch_ladder(a, 0, eng->stream);
         WG_CUDA(cudaEventRecord(eng->kev[3], eng->stream), "event");
         WG_CUDA(cudaGetLastError(), "kernel launch");
+        ladder = true;
     }
     st.batches++;
-    for (int k = 0; k < 3; k++) {
+    for (int k = 0; k < 3; k++) {   // climate (or unit), entrance, ladder: those this batch launched
+        if (k == 1 ? a.unit_cta != 0 : (k == 2 && !ladder)) continue;
         float ms = 0.f;
         cudaEventElapsedTime(&ms, eng->kev[k], eng->kev[k + 1]);
         st.kernel_ms[k] += ms;
-        if (k == 0 || !a.unit_cta) st.kernel_launches[k]++;
+        st.kernel_launches[k]++;
     }
     if (eng->h_counters[CNT_OVERFLOW]) {
         if (n_units <= (a.unit_cta ? 1u : 32u)) return eng->fail(WG_ERR_CAPACITY, "phase-1 work list full even for the smallest batch");
@@ -289,6 +292,55 @@ BatchArgs base_args(wg_engine *eng, const wg_opts &opts, int salt) {
     a.hist = eng->hist;
     a.lists[2] = RegionList{eng->rec_unit, eng->rec_off, eng->rec_cnt, eng->surv, nullptr, kCapRec, kCapSurv, CNT_RECORDS};
     return a;
+}
+
+int copy_result(wg_engine *eng, void *dst, const void *src, size_t bytes) {
+    constexpr int kPieces = (int)(kStageBytes / kStagePiece), kThreads = 4;
+    static_assert(kPieces <= 8, "one event per piece in flight");
+    const size_t want = std::min(kStageBytes, (bytes + kStagePiece - 1) / kStagePiece * kStagePiece);
+    if (bytes >= (1u << 20) && want > eng->stage_bytes) {
+        cudaFreeHost(eng->stage);
+        eng->stage = nullptr;
+        eng->stage_bytes = 0;
+        if (cudaMallocHost(&eng->stage, want) == cudaSuccess) eng->stage_bytes = want;
+        else cudaGetLastError();   // no pinned memory: the plain copy below
+        for (cudaEvent_t &e : eng->stage_ev)
+            if (!e) WG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    }
+    if (bytes < (1u << 20) || !eng->stage_bytes) {
+        WG_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost), "copy result");
+        return WG_OK;
+    }
+    for (size_t at = 0; at < bytes; at += eng->stage_bytes) {
+        const size_t round = std::min(eng->stage_bytes, bytes - at);
+        const int n = (int)((round + kStagePiece - 1) / kStagePiece);
+        auto size_of = [&](int p) { return std::min(kStagePiece, round - (size_t)p * kStagePiece); };
+        for (int p = 0; p < n; p++) {
+            const size_t o = (size_t)p * kStagePiece;
+            WG_CUDA(cudaMemcpyAsync(eng->stage + o, static_cast<const char *>(src) + at + o, size_of(p),
+                                    cudaMemcpyDeviceToHost, eng->stream),
+                    "copy result");
+            WG_CUDA(cudaEventRecord(eng->stage_ev[p], eng->stream), "event");
+        }
+        std::atomic<int> next{0}, failed{(int)cudaSuccess};
+        auto take = [&] {
+            for (int p = next++; p < n; p = next++) {
+                const cudaError_t e = cudaEventSynchronize(eng->stage_ev[p]);
+                if (e != cudaSuccess) failed = (int)e;
+                else std::memcpy(static_cast<char *>(dst) + at + (size_t)p * kStagePiece, eng->stage + (size_t)p * kStagePiece, size_of(p));
+            }
+        };
+        std::thread helpers[kThreads - 1];
+        try {
+            for (int h = 0; h < std::min(kThreads, n) - 1; h++) helpers[h] = std::thread(take);
+        } catch (const std::exception &) {   // no more threads: this one takes the rest
+        }
+        take();
+        for (std::thread &t : helpers)
+            if (t.joinable()) t.join();
+        if (failed != (int)cudaSuccess) return eng->fail(WG_ERR_CUDA, "copy result", (cudaError_t)failed.load());
+    }
+    return WG_OK;
 }
 
 int list_buffers(wg_engine *eng) {
@@ -493,10 +545,11 @@ int wg_engine_open(int device, wg_engine **out) {
         WG_CUDA(cudaMalloc(&eng->surv, sizeof(uint32_t) * kCapSurv), "alloc");
         WG_CUDA(cudaMalloc(&eng->deep, sizeof(uint32_t) * 2 * kCapDeep), "alloc");
         WG_CUDA(cudaMalloc(&eng->out, sizeof(Candidate) * kCapOut), "alloc");
-        WG_CUDA(cudaMalloc(&eng->counters, sizeof(uint32_t) * CNT_WORDS), "alloc");
-        WG_CUDA(cudaMalloc(&eng->hist, sizeof(unsigned long long) * (P1_KINDS + kTiers)), "alloc");
-        WG_CUDA(cudaMallocHost(&eng->h_counters, sizeof(uint32_t) * CNT_WORDS), "alloc");
-        WG_CUDA(cudaMallocHost(&eng->h_hist, sizeof(unsigned long long) * (P1_KINDS + kTiers)), "alloc");
+        // the counters and, behind them, the funnel: one block, cleared and read back at once
+        WG_CUDA(cudaMalloc(&eng->counters, kCountBytes), "alloc");
+        eng->hist = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(eng->counters) + kHistOffset);
+        WG_CUDA(cudaMallocHost(&eng->h_counters, kCountBytes), "alloc");
+        eng->h_hist = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(eng->h_counters) + kHistOffset);
         return WG_OK;
     }();
     if (rc) {
@@ -518,7 +571,6 @@ void wg_engine_close(wg_engine *eng) {
     cudaFree(eng->deep);
     cudaFree(eng->out);
     cudaFree(eng->counters);
-    cudaFree(eng->hist);
     cudaFree(eng->d_seed_list);
     cudaFree(eng->list_block);
     cudaFree(eng->spot_items[0]);
@@ -530,7 +582,9 @@ void wg_engine_close(wg_engine *eng) {
     queue_release(eng);
     finish_release(eng);
     cudaFreeHost(eng->h_counters);
-    cudaFreeHost(eng->h_hist);
+    cudaFreeHost(eng->stage);
+    for (cudaEvent_t e : eng->stage_ev)
+        if (e) cudaEventDestroy(e);
     if (eng->ev0) cudaEventDestroy(eng->ev0);
     if (eng->ev1) cudaEventDestroy(eng->ev1);
     for (int k = 0; k < 4; k++)
@@ -623,9 +677,7 @@ int wg_seed_check(wg_engine *eng, const int64_t *seeds, uint64_t gen_base, uint6
     WG_CUDA(cudaEventRecord(eng->ev0, eng->stream), "event");
     rc = run_request(eng, rq, sink, st);
     if (rc) return rc;
-    WG_CUDA(cudaEventRecord(eng->ev1, eng->stream), "event");
-    WG_CUDA(cudaEventSynchronize(eng->ev1), "event");
-    float ms = 0.f;
+    float ms = 0.f;   // ev1: after the last batch, which is over
     cudaEventElapsedTime(&ms, eng->ev0, eng->ev1);
     std::sort(found.begin(), found.end(), [](const Candidate &x, const Candidate &y) {
         if (x.seed_index != y.seed_index) return x.seed_index < y.seed_index;
@@ -673,8 +725,10 @@ int wg_seed_check_device(wg_engine *eng, const int64_t *d_seeds, uint64_t gen_ba
     WG_CUDA(cudaEventRecord(eng->ev0, eng->stream), "event");
     int rc = run_request(eng, rq, sink, st);
     if (rc) return rc;
-    WG_CUDA(cudaEventRecord(eng->ev1, eng->stream), "event");
-    WG_CUDA(cudaEventSynchronize(eng->ev1), "event");
+    if (sink.found) {   // the copies of survivors into the caller's buffer
+        WG_CUDA(cudaEventRecord(eng->ev1, eng->stream), "event");
+        WG_CUDA(cudaEventSynchronize(eng->ev1), "event");
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, eng->ev0, eng->ev1);
     if (n_out) *n_out = sink.found;

@@ -38,8 +38,12 @@ struct wg_engine {
     wg::Candidate *out = nullptr;
     uint32_t *counters = nullptr;
     unsigned long long *hist = nullptr;
-    uint32_t *h_counters = nullptr;         // pinned
-    unsigned long long *h_hist = nullptr;   // pinned
+    uint32_t *h_counters = nullptr;         // pinned; h_hist lies behind it
+    unsigned long long *h_hist = nullptr;
+    // pinned staging of large results (copy_result), kept at its largest size up to kStageBytes
+    char *stage = nullptr;
+    size_t stage_bytes = 0;
+    cudaEvent_t stage_ev[8] = {};
     cudaEvent_t kev[4] = {nullptr, nullptr, nullptr, nullptr};   // around the three kernels of a batch
     int64_t *d_seed_list = nullptr;
     uint64_t d_seed_cap = 0;
@@ -95,6 +99,17 @@ namespace wg {
 // index i.  Asynchronous on eng->stream.
 int p2_prepare_chunks(wg_engine *eng, const std::vector<uint64_t> &seeds, int large, const std::vector<int> &world,
                       const std::vector<int> &cx, const std::vector<int> &cz);
+
+// The counters' and the funnel's block.
+constexpr size_t kHistOffset = 128, kCountBytes = kHistOffset + sizeof(unsigned long long) * (P1_KINDS + kTiers);
+static_assert(sizeof(uint32_t) * CNT_WORDS <= kHistOffset, "the funnel lies behind the counters");
+
+// Copies a result from device memory, complete on eng->stream, to the caller's pageable memory.  From
+// 1 MiB on through pinned staging in pieces, several threads copying pieces out (and taking the page
+// faults of a fresh buffer) while later ones are on the bus.  A walk's 268k start chunks (10.7 MB) into
+// a fresh buffer, whole call: 2.65-2.95 ms with one cudaMemcpy, 2.5 ms so; 8 threads 2.7 ms.
+constexpr size_t kStageBytes = 16u << 20, kStagePiece = 2u << 20;
+int copy_result(wg_engine *eng, void *dst, const void *src, size_t bytes);
 
 // Per-batch work budget: (seed, region) checks per batch and units per batch, and the sizes of
 // the engine's phase-1 work lists.
