@@ -113,15 +113,19 @@ struct Xr32 {
 
 // RNG of octave `p` (index into NoiseSpec octave arrays) of sub `sub` of noise `ns`,
 // given the seed fork (the per-seed createRandomDeriver state).
-__device__ __forceinline__ Xr octave_rng(const NoiseSpec &ns, Xr seed_fork, int sub, int p) {
-    Xr noise = xr_make(ns.name_lo ^ seed_fork.lo, ns.name_hi ^ seed_fork.hi);
+__device__ __forceinline__ Xr octave_rng(uint64_t name_lo, uint64_t name_hi, uint64_t oct_lo, uint64_t oct_hi, Xr seed_fork,
+                                         bool sub) {
+    Xr noise = xr_make(name_lo ^ seed_fork.lo, name_hi ^ seed_fork.hi);
     uint64_t a = xr_next(noise), b = xr_next(noise);
     if (sub) {
         a = xr_next(noise);
         b = xr_next(noise);
     }
     Xr fork = xr_make(a, b);
-    return xr_make(ns.oct_lo[p] ^ fork.lo, ns.oct_hi[p] ^ fork.hi);
+    return xr_make(oct_lo ^ fork.lo, oct_hi ^ fork.hi);
+}
+__device__ __forceinline__ Xr octave_rng(const NoiseSpec &ns, Xr seed_fork, int sub, int p) {
+    return octave_rng(ns.name_lo, ns.name_hi, ns.oct_lo[p], ns.oct_hi[p], seed_fork, sub != 0);
 }
 
 __device__ __forceinline__ Xr seed_fork_of(uint64_t seed) {
@@ -156,20 +160,30 @@ __device__ __forceinline__ uint64_t lcg_long(uint64_t &st) {
     return (hi << 32) + (uint64_t)lo;
 }
 
-// Chunk of the swamp hut in region (rx, rz): spacing 32, separation 8.  Both draws straight on; the
-// JDK's re-draw (a 31-bit value of 2147483640 or more, 8 in 2^31) starts over with the exact loop.
-__device__ __forceinline__ void hut_chunk(uint64_t seed, int rx, int rz, int salt, int &cx, int &cz) {
+// The swamp hut of region (rx, rz), spacing 32, separation 8: the LCG's seed (its low 48 bits matter),
+// linear in rx and rz, and the two draws, the hut's chunk in its region.
+constexpr uint64_t kHutX = 341873128712ULL, kHutZ = 132897987541ULL;
+
+__device__ __forceinline__ uint64_t hut_lcg(uint64_t seed, int rx, int rz, int salt) {
+    return (uint64_t)(int64_t)rx * kHutX + (uint64_t)(int64_t)rz * kHutZ + seed + (uint64_t)(int64_t)salt;
+}
+// Both draws straight on; the JDK's re-draw (a 31-bit value of 2147483640 or more, 8 in 2^31) starts over
+// with the exact loop.
+__device__ __forceinline__ void hut_draws(uint64_t s, int &j, int &k) {
     constexpr uint32_t kLimit = 2147483640u;
-    const uint64_t s = (uint64_t)(int64_t)rx * 341873128712ULL + (uint64_t)(int64_t)rz * 132897987541ULL + seed +
-                       (uint64_t)(int64_t)salt;
-    const uint64_t s1 = (s ^ kLcgMul) * kLcgMul + 0xBULL, s2 = s1 * kLcgMul + 0xBULL;   // low 48 bits matter
+    const uint64_t s1 = (s ^ kLcgMul) * kLcgMul + 0xBULL, s2 = s1 * kLcgMul + 0xBULL;
     const uint32_t u1 = (uint32_t)(s1 >> 17) & 0x7FFFFFFFu, u2 = (uint32_t)(s2 >> 17) & 0x7FFFFFFFu;
-    int j = (int)(u1 % 24u), k = (int)(u2 % 24u);
+    j = (int)(u1 % 24u);
+    k = (int)(u2 % 24u);
     if (u1 >= kLimit || u2 >= kLimit) {
         uint64_t st = (s ^ kLcgMul) & kLcgMask;
         j = lcg_int(st, 24);
         k = lcg_int(st, 24);
     }
+}
+__device__ __forceinline__ void hut_chunk(uint64_t seed, int rx, int rz, int salt, int &cx, int &cz) {
+    int j, k;
+    hut_draws(hut_lcg(seed, rx, rz, salt), j, k);
     cx = rx * 32 + j;
     cz = rz * 32 + k;
 }

@@ -37,6 +37,9 @@ static void fill_slots(int8_t (*dst)[3], const NoiseSpec *specs, const int *nois
     (void)expect;
 }
 
+static void upload_unit_tables(const NoiseSpec *specs, const ClimateStep *const steps[2], const int8_t (*slot_a)[kSlotsA][3],
+                               const int8_t (*slot_c)[kSlotsC][3]);
+
 void upload_tables(const NoiseSpec *specs, const ClimateStep *steps_normal, const ClimateStep *steps_large,
                    const F32Bands *bands) {
     cudaMemcpyToSymbol(c_noise, specs, sizeof(NoiseSpec) * N_NOISE_COUNT);
@@ -58,6 +61,8 @@ void upload_tables(const NoiseSpec *specs, const ClimateStep *steps_normal, cons
     }
     cudaMemcpyToSymbol(c_slot_a, sa, sizeof(sa));
     cudaMemcpyToSymbol(c_slot_c, sc, sizeof(sc));
+    const ClimateStep *const both[2] = {steps_normal, steps_large};
+    upload_unit_tables(specs, both, sa, sc);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1111,12 +1116,12 @@ __device__ __forceinline__ int ent_noise(int i) {
 // order: value = (sum_a + sum_b) * amplitude with sum = sum_p (amp_p * v_p) * per_p, so the error is
 // at most |amplitude| * 2 * sum_p |amp_p * per_p| times the sample bound, plus 1e-12 for the FP64
 // roundings of both sides.
-__device__ double dp_err_f32(int noise) {
-    const NoiseSpec &ns = c_noise[noise];
+__host__ __device__ inline double dp_err_f32(const NoiseSpec &ns) {
     double w = 0.0;
     for (int p = 0; p < ns.npresent; p++) w += fabs(ns.amp[p] * ns.per[p]);
     return 2.0 * fabs(ns.amplitude) * w * (kPerlin3dF32ErrUlps / 16777216.0) + 1e-12;
 }
+__device__ double dp_err_f32(int noise) { return dp_err_f32(c_noise[noise]); }
 
 struct EntranceSmem {
     uint8_t perm[kSlotsB * kPitch];

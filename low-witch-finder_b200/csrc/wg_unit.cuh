@@ -19,11 +19,15 @@
 // The top 24 bits give the lattice cell and a 23-bit fraction (rounded by half a unit added to the
 // base), which costs no FP64 and no conversion instruction.
 //
+// A block costs two barriers: the next block's lattice bases are formed a block ahead, and the pool is
+// looked at only when it is full.  (With six, and the lists packed after each of the erosion steps 4-7:
+// 1.6e9 regions of one seed 55.9 -> 54.2 ms; barriers were 5 % of a CTA's time.)
+//
 // Measured against the three list kernels, which rebuilt a seed's tables for every 2,048-region
-// window, record and candidate: one seed over the whole world (1.37e10 regions) 1,029 -> 472 ms, one seed x
-// 24,964 regions 538 -> 156 us (13 windows in one CTA before), x 400 regions 170 -> 109 us.  Of a
-// large unit's time the hut positions and tier bookkeeping take 18 %, the lattices 9 %, tier 0 13 %,
-// steps 2-3 16 %, the later gates 23 %, the entrance gate 13 %, the ladder 8 %.
+// window, record and candidate: one seed over the whole world (1.37e10 regions) 1,029 -> 425 ms, one seed x
+// 24,964 regions 538 -> 125 us (13 windows in one CTA before), x 400 regions 170 -> 93 us.  Of a large unit's
+// time the table builds take 2 %, the lattices 12 %, hut positions and tier 0 22 %, steps 2-3 16 %, the
+// later gates 21 %, barriers 8 %, the entrance gate 12 %, the ladder 6 %.
 #pragma once
 
 constexpr int kUThreads = 256;
@@ -48,18 +52,78 @@ static_assert(kUClim + kSlotsA <= kUTabs, "climate tables overlay ladder tables"
 constexpr double kPerlinMax = 1.0625;
 constexpr double kSpagSure = 0.29;
 
+// Where a block lies in its lattice tables: its base in lattice coordinates of its first cell, that
+// cell, and the columns per axis (and ceil(2^20 / nx)).
+struct LatBase {
+    uint64_t x[kLatTables], z[kLatTables];
+    int cell_x[kLatTables], cell_z[kLatTables], nx[kLatTables], nz[kLatTables];
+    uint32_t inv[kLatTables];
+};
+
+// What the kernel keeps of the tables' constants (err: FP32 core, bounds of the first entrance test's four
+// noises), and each table's generator (climate tables in step order, then the cave tables).  In global
+// memory: lanes that read different words of constant memory take turns, and in a call of one wave every
+// turn is a miss (the 18 lanes' steps and generators: 10,000 of a CTA's 60,000 cycles, now 2,500).
+struct UnitConst {
+    ClimateSteps steps;
+    uint64_t fstep[kSlotsA];
+    double err[4];
+};
+struct TableRng {
+    uint64_t name_lo, name_hi, oct_lo, oct_hi, sub;
+};
+struct UnitTables {
+    alignas(16) UnitConst c;
+    TableRng rng[kSlotsA + kSlotsC];
+};
+static_assert(sizeof(UnitConst) % 16 == 0, "copied in 16-byte words");
+__device__ UnitTables g_unit_tables[2];        // [large_biomes]
+
+static void upload_unit_tables(const NoiseSpec *specs, const ClimateStep *const steps[2], const int8_t (*slot_a)[kSlotsA][3],
+                               const int8_t (*slot_c)[kSlotsC][3]) {
+    UnitTables host[2];
+    for (int l = 0; l < 2; l++) {
+        UnitTables &u = host[l];
+        auto rng = [&](const int8_t *s) {
+            const NoiseSpec &n = specs[s[0]];
+            return TableRng{n.name_lo, n.name_hi, n.oct_lo[s[2]], n.oct_hi[s[2]], (uint64_t)s[1]};
+        };
+        for (int k = 0; k < kClimateSteps; k++) {
+            const ClimateStep &s = steps[l][k];
+            ClimateSteps &t = u.c.steps;
+            t.sc[k] = s.sc;
+            t.lac[k] = s.lac;
+            t.c1[k] = s.c1;
+            t.c2[k] = s.c2;
+            t.thr[k] = s.thr;
+            t.amp[k] = s.amp;
+            t.slot[k] = s.slot;
+            t.act[k] = s.act;
+            t.tier[k] = s.tier;
+            t.cf[k] = s.cf;
+            t.lo[k] = s.lo;
+            t.hi[k] = s.hi;
+            u.c.fstep[k] = s.fstep;
+            u.rng[k] = rng(slot_a[l][s.slot]);
+        }
+        for (int t = 0; t < kSlotsC; t++) u.rng[kSlotsA + t] = rng(slot_c[l][t]);
+        const int quick[4] = {N_SPAGHETTI_RARITY, N_SPAGHETTI_1, N_SPAGHETTI_2, N_CAVE_ENTRANCE};
+        for (int q = 0; q < 4; q++) u.c.err[q] = dp_err_f32(specs[quick[q]]);
+    }
+    cudaMemcpyToSymbol(g_unit_tables, host, sizeof host);
+}
+
 template <bool F32>
 struct UnitSmem {
     using Real = typename std::conditional<F32, float, double>::type;
     uint8_t tab[kUTabs * kUPitch];
     double org[3 * kUTabs];                    // cave tables' origins [slot][3]
     double cox[kSlotsA], coz[kSlotsA], chy[kSlotsA];   // climate tables, step order
-    uint64_t fx[kSlotsA], fz[kSlotsA], fstep[kSlotsA];
+    uint64_t fx[kSlotsA], fz[kSlotsA];
     float hyf[kSlotsA], fyf[kSlotsA];
     float w0[kLatTables], w1[kLatTables], c0[kLatTables], c1[kLatTables];
     int jy[kSlotsA];
-    uint64_t bx[kLatTables], bz[kLatTables];   // the block's base in lattice coordinates of its first cell
-    int cell_x[kLatTables], cell_z[kLatTables], nx[kLatTables], nz[kLatTables];
+    LatBase lat_base[2];                       // this block's and the next one's
     union {
         struct {
             float4 l0[2][kLat0 * kLat0];
@@ -76,11 +140,10 @@ struct UnitSmem {
     uint32_t und[2 * kUThreads];               // those its first test left open
     uint32_t deep[kUDeep];
     uint32_t n_pool, n_surv, n_und, n_deep, n_total;
-    double err[4];                             // FP32 core: bounds of the first entrance test's noises
     unsigned int hist[P1_KINDS + kTiers];
     uint32_t grad[kGradWords];
     GradF gf;
-    ClimateSteps steps;
+    alignas(16) UnitConst c;
 };
 
 // A survivor word of the unit kernel: the hut's chunk offset from the unit's first chunk, x | z << 16;
@@ -116,7 +179,7 @@ __device__ __forceinline__ uint64_t to_fixed(double v) {
 template <bool F32>
 __device__ __forceinline__ float unit_sample_f32(const UnitSmem<F32> &S, int k, uint32_t dx, uint32_t dz) {
     const uint8_t *P = S.tab + (kUClim + k) * kUPitch;
-    const uint64_t step = S.fstep[k];
+    const uint64_t step = S.c.fstep[k];
     const uint32_t hx = fixed_hi(S.fx[k], step, dx), hz = fixed_hi(S.fz[k], step, dz);
     const float g = fixed_frac(hx), l = fixed_frac(hz);
     const F2 gl = f2(g, l);
@@ -174,7 +237,7 @@ __device__ __forceinline__ void unit_point(const UnitCtx &U, uint32_t e, double 
 }
 template <bool F32>
 __device__ __forceinline__ double unit_sample64(const UnitSmem<F32> &S, int k, double xc, double zc) {
-    const ClimateSteps &st = S.steps;
+    const ClimateSteps &st = S.c.steps;
     const ColTable<1> T{S.tab + (kUClim + k) * kUPitch, S.grad};
     const double sc = st.sc[k], lac = st.lac[k], hy = S.chy[k];
     return perlin_y0(T, S.cox[k], S.coz[k], S.jy[k], hy, fade(hy), keep_precision((xc * sc) * lac),
@@ -183,7 +246,7 @@ __device__ __forceinline__ double unit_sample64(const UnitSmem<F32> &S, int k, d
 // FP64 octave sum of erosion steps [0, k1] in the reference's order.
 template <bool F32>
 __device__ __noinline__ double unit_sum64(const UnitSmem<F32> &S, int k1, double xc, double zc) {
-    const ClimateSteps &st = S.steps;
+    const ClimateSteps &st = S.c.steps;
     double sum = 0.0;
     for (int k = 0; k <= k1; k++) sum += (st.c1[k] * unit_sample64(S, k, xc, zc)) * st.c2[k];
     return sum;
@@ -191,7 +254,7 @@ __device__ __noinline__ double unit_sum64(const UnitSmem<F32> &S, int k1, double
 // FP64 DoublePerlin value of the temperature / ridge noise of steps k0 .. k0 + n - 1.
 template <bool F32>
 __device__ __noinline__ double unit_value64(const UnitSmem<F32> &S, int k0, int n, double xc, double zc) {
-    const ClimateSteps &st = S.steps;
+    const ClimateSteps &st = S.c.steps;
     double sum = 0.0, sum_a = 0.0;
     for (int k = k0; k < k0 + n; k++) {
         sum += (st.c1[k] * unit_sample64(S, k, xc, zc)) * st.c2[k];
@@ -220,15 +283,15 @@ struct WarpCounts {
 // survives the step's tier.
 template <bool F32, bool LAT>
 __device__ __forceinline__ bool unit_step(UnitSmem<F32> &S, const BatchArgs &a, const UnitCtx &U, WarpCounts &W, int k,
-                                          bool all_rechecks, uint32_t e, uint32_t ex, uint32_t ez,
+                                          bool all_rechecks, uint32_t e, const LatBase *B, uint32_t ex, uint32_t ez,
                                           typename UnitSmem<F32>::Real prev, typename UnitSmem<F32>::Real &sum) {
-    const ClimateSteps &st = S.steps;
+    const ClimateSteps &st = S.c.steps;
     bool reject;
     if constexpr (F32) {
         float v;
         if constexpr (LAT) {
-            const uint64_t step = S.fstep[k];
-            v = lat_sample(S.lat.l1[k - 2], S.nx[k], fixed_hi(S.bx[k], step, ex), fixed_hi(S.bz[k], step, ez));
+            const uint64_t step = S.c.fstep[k];
+            v = lat_sample(S.lat.l1[k - 2], B->nx[k], fixed_hi(B->x[k], step, ex), fixed_hi(B->z[k], step, ez));
         } else {
             v = unit_sample_f32(S, k, e & 0xFFFFu, e >> 16);
         }
@@ -254,43 +317,35 @@ __device__ __forceinline__ bool unit_step(UnitSmem<F32> &S, const BatchArgs &a, 
     return !reject;
 }
 
-// Erosion steps 4..7, temperature and ridge for the n <= kList regions in a warp's list; the survivors
-// join the unit's list.
+// Erosion steps 4..7, temperature and ridge for n <= kList pooled regions (words, erosion sums); the
+// survivors join the unit's list.  A region keeps its lane through the four steps: they pass 46 % of what
+// comes in, so lists packed again after each step would take as many rounds for a warp's 64.
 template <bool F32>
-__device__ __forceinline__ void unit_drain(UnitSmem<F32> &S, const BatchArgs &a, const UnitCtx &U, WarpCounts &W, uint32_t n,
-                            bool all_rechecks, int large) {
+__device__ __forceinline__ void unit_drain(UnitSmem<F32> &S, const BatchArgs &a, const UnitCtx &U, WarpCounts &W,
+                                           const uint32_t *words, const typename UnitSmem<F32>::Real *sums, uint32_t n,
+                                           bool all_rechecks, int large) {
     using Real = typename UnitSmem<F32>::Real;
-    const ClimateSteps &st = S.steps;
+    const ClimateSteps &st = S.c.steps;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t *const wl = S.wl[warp];
-    Real *const ws = S.ws[warp];
     const unsigned below = (1u << lane) - 1u;
+    uint32_t n7 = 0;
     __syncwarp();
 #pragma unroll 1
-    for (int k = 4; n && k < 8; k++) {
-        uint32_t nn = 0;
+    for (uint32_t b = 0; b < n; b += 32) {
+        const uint32_t q = b + (uint32_t)lane;
+        bool keep = q < n;
+        const uint32_t e = keep ? words[q] : 0u;
+        Real sum = keep ? sums[q] : Real(0);
 #pragma unroll 1
-        for (uint32_t b = 0; b < n; b += 32) {
-            const uint32_t q = b + (uint32_t)lane;
-            bool keep = false;
-            uint32_t e = 0;
-            Real sum = 0;
-            if (q < n) {
-                e = wl[q];
-                keep = unit_step<F32, false>(S, a, U, W, k, all_rechecks, e, 0, 0, ws[q], sum);
-            }
-            const unsigned m = __ballot_sync(0xFFFFFFFFu, keep);
-            __syncwarp();
-            if (keep) {
-                const uint32_t at = nn + (uint32_t)__popc(m & below);
-                wl[at] = e;
-                ws[at] = sum;
-            }
-            nn += (uint32_t)__popc(m);
-        }
-        __syncwarp();
-        n = nn;
+        for (int k = 4; k < 8; k++)
+            if (keep) keep = unit_step<F32, false>(S, a, U, W, k, all_rechecks, e, nullptr, 0, 0, sum, sum);
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, keep);
+        if (keep) wl[n7 + (uint32_t)__popc(m & below)] = e;
+        n7 += (uint32_t)__popc(m);
     }
+    __syncwarp();
+    n = n7;
     // temperature: four lanes per region, summed in order by the first; then ridge with six
     constexpr int kT0 = 8, kR0 = 12;
     uint32_t nr = 0;
@@ -409,8 +464,8 @@ __device__ __forceinline__ void unit_drain(UnitSmem<F32> &S, const BatchArgs &a,
 // Table t of the unit built by one thread in shared memory: the climate tables (step order) or cave
 // table `slot`; the entries are stored twice and once more by unit_double_tables.
 __device__ __forceinline__ Xr unit_table_rng(int large, bool climate, int idx, const Xr &fork) {
-    const int8_t *s = climate ? c_slot_a[large][c_steps[large][idx].slot] : c_slot_c[large][idx];
-    return octave_rng(c_noise[s[0]], fork, s[1], s[2]);
+    const TableRng t = g_unit_tables[large].rng[climate ? idx : kSlotsA + idx];
+    return octave_rng(t.name_lo, t.name_hi, t.oct_lo, t.oct_hi, fork, t.sub != 0);
 }
 
 // Identity in the first 256 bytes of n tables from table t0 (word by word, whole CTA).
@@ -515,36 +570,20 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
 
     if (tid < P1_KINDS + kTiers) S.hist[tid] = 0;
     if (tid == 0) S.n_pool = S.n_surv = S.n_und = S.n_deep = S.n_total = 0;
-    if (tid < 4)   // the bounds the first entrance test's decisions allow for (exact noises: none)
-        S.err[tid] = F32 ? dp_err_f32(tid == 0 ? N_SPAGHETTI_RARITY
-                                      : tid == 1 ? N_SPAGHETTI_1
-                                      : tid == 2 ? N_SPAGHETTI_2 : N_CAVE_ENTRANCE)
-                         : 0.0;
+    for (int q = kUThreads - 1 - tid; q < (int)(sizeof(UnitConst) / 16); q += kUThreads)   // warps that build nothing
+        reinterpret_cast<uint4 *>(&S.c)[q] = reinterpret_cast<const uint4 *>(&g_unit_tables[large].c)[q];
     fill_grad_table(S.grad, tid);
     fill_grad_table_f32(&S.gf, tid);
-    if (tid < kClimateSteps) {
-        const ClimateStep &c = c_steps[large][tid];
-        S.steps.sc[tid] = c.sc;
-        S.steps.lac[tid] = c.lac;
-        S.steps.c1[tid] = c.c1;
-        S.steps.c2[tid] = c.c2;
-        S.steps.thr[tid] = c.thr;
-        S.steps.amp[tid] = c.amp;
-        S.steps.act[tid] = c.act;
-        S.steps.tier[tid] = c.tier;
-        S.steps.cf[tid] = c.cf;
-        S.steps.lo[tid] = c.lo;
-        S.steps.hi[tid] = c.hi;
-    }
-    unit_init_tables(S.tab, 0, kSlotsB + kSlotsA);
-    __syncthreads();
     // warp 0 builds the climate tables, warp 1 the entrance gate's: one table's 256 dependent steps
     // take about 10 us whatever is beside them
-    if (warp < 2 && lane < kSlotsA) {
-        const bool clim = warp == 0;
-        Xr r = unit_table_rng(large, clim, lane, seed_fork_of(U.seed));
-        double ox, oy, oz;
+    const bool clim = warp == 0, builds = warp < 2 && lane < kSlotsA;
+    Xr r{};
+    if (builds) r = unit_table_rng(large, clim, lane, seed_fork_of(U.seed));
+    unit_init_tables(S.tab, 0, kSlotsB + kSlotsA);
+    __syncthreads();
+    if (builds) {
         const int t = clim ? kUClim + lane : lane;
+        double ox, oy, oz;
         perlin_shuffle<1>(S.tab + t * kUPitch, r, ox, oy, oz);
         if (clim) {
             const int jy = (int)floor(oy);
@@ -555,11 +594,10 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
             S.jy[lane] = jy;
             S.hyf[lane] = __double2float_rn(hy);
             S.fyf[lane] = __double2float_rn(fy);
-            const double sc = S.steps.sc[lane], lac = S.steps.lac[lane];
+            const double sc = S.c.steps.sc[lane], lac = S.c.steps.lac[lane];
             const double xc = (U.ucx * 16 + 8) * 0.25, zc = (U.ucz * 16 + 8) * 0.25;
             S.fx[lane] = to_fixed(keep_precision((xc * sc) * lac) + ox);
             S.fz[lane] = to_fixed(keep_precision((zc * sc) * lac) + oz);
-            S.fstep[lane] = c_steps[large][lane].fstep;
             if (lane < kLatTables) {
                 S.w0[lane] = __double2float_rn(1.0 - fy);
                 S.w1[lane] = __double2float_rn(fy);
@@ -573,40 +611,47 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
         }
     }
     __syncthreads();
-    unit_double_tables(S.tab, 0, kSlotsB + kSlotsA);
-    __syncthreads();
-
-    const ClimateSteps &st = S.steps;
-    WarpCounts W;
     const uint32_t nbx = (U.up.tw + kBlock - 1) / kBlock, nbz = (U.up.th + kBlock - 1) / kBlock;
     const uint32_t bw = (U.up.tw + nbx - 1) / nbx, bh = (U.up.th + nbz - 1) / nbz;
     const uint32_t n_blocks = nbx * nbz;
+    auto lattice_base = [&](uint32_t blk) {   // one thread per table and axis, a block ahead of its use
+        if (tid >= 2 * kLatTables || blk >= n_blocks) return;
+        LatBase &B = S.lat_base[blk & 1u];
+        const int k = tid >> 1;
+        const bool z = tid & 1;
+        const uint32_t at = z ? (blk / nbx) * bh : (blk % nbx) * bw;   // first region of the block, in the unit
+        const uint32_t side = z ? min(bh, U.up.th - at) : min(bw, U.up.tw - at);
+        const uint64_t step = S.c.fstep[k];
+        const uint64_t b = (z ? S.fz[k] : S.fx[k]) + (uint64_t)(at * 32u) * step;
+        const uint64_t b0 = b & 0x00FFFFFFFFFFFFFFull;
+        const int cols = (int)(fixed_hi(b0, step, (side - 1) * 32u + 23u) >> 24) + 2;
+        (z ? B.z : B.x)[k] = b0;
+        (z ? B.cell_z : B.cell_x)[k] = (int)(b >> 56);
+        (z ? B.nz : B.nx)[k] = cols;
+        if (!z) B.inv[k] = ((1u << 20) + (uint32_t)cols - 1) / (uint32_t)cols;
+    };
+    if constexpr (F32) lattice_base(0);
+    unit_double_tables(S.tab, 0, kSlotsB + kSlotsA);
+    __syncthreads();
+
+    const ClimateSteps &st = S.c.steps;
+    WarpCounts W;
     for (uint32_t blk = 0; blk < n_blocks; blk++) {
         const uint32_t x0 = (blk % nbx) * bw, z0 = (blk / nbx) * bh;   // first region of the block, in the unit
         const uint32_t w = min(bw, U.up.tw - x0), h = min(bh, U.up.th - z0), n = w * h;
+        const LatBase &B = S.lat_base[blk & 1u];
         if constexpr (F32) {
             // ---- the block's lattice columns ----
-            if (tid < 2 * kLatTables) {
-                const int k = tid >> 1;
-                const bool z = tid & 1;
-                const uint64_t step = S.fstep[k];
-                const uint64_t b = (z ? S.fz[k] : S.fx[k]) + (uint64_t)((z ? z0 : x0) * 32u) * step;
-                const uint64_t b0 = b & 0x00FFFFFFFFFFFFFFull;
-                const uint32_t last = ((z ? h : w) - 1) * 32u + 23u;
-                (z ? S.bz : S.bx)[k] = b0;
-                (z ? S.cell_z : S.cell_x)[k] = (int)(b >> 56);
-                (z ? S.nz : S.nx)[k] = (int)(fixed_hi(b0, step, last) >> 24) + 2;
-            }
-            __syncthreads();
-            const int m0 = S.nx[0] * S.nz[0], m1 = m0 + S.nx[1] * S.nz[1], m2 = m1 + S.nx[2] * S.nz[2],
-                      m3 = m2 + S.nx[3] * S.nz[3];
+            lattice_base(blk + 1);   // into the other half, which no thread reads before the next block
+            const int m0 = B.nx[0] * B.nz[0], m1 = m0 + B.nx[1] * B.nz[1], m2 = m1 + B.nx[2] * B.nz[2],
+                      m3 = m2 + B.nx[3] * B.nz[3];
             for (int q = tid; q < m3; q += kUThreads) {
                 const int k = (q >= m0) + (q >= m1) + (q >= m2);
                 const int r = q - (k == 0 ? 0 : k == 1 ? m0 : k == 2 ? m1 : m2);
-                const int iz = r / S.nx[k], ix = r - iz * S.nx[k];
+                const int iz = (int)(((uint32_t)r * B.inv[k]) >> 20), ix = r - iz * B.nx[k];   // r < 361, nx <= 19
                 const uint8_t *P = S.tab + (kUClim + k) * kUPitch;
-                const uint8_t *Pj = P + S.jy[k], *Pk = P + ((S.cell_z[k] + iz) & 255);
-                const uint32_t pa = P[(S.cell_x[k] + ix) & 255];
+                const uint8_t *Pj = P + S.jy[k], *Pk = P + ((B.cell_z[k] + iz) & 255);
+                const uint32_t pa = P[(B.cell_x[k] + ix) & 255];
                 const uint32_t h0 = Pk[Pj[pa]] & 15u, h1 = Pk[Pj[pa + 1]] & 15u;
                 const float2 g0 = S.gf.xz[h0], g1 = S.gf.xz[h1];
                 float4 c;
@@ -620,6 +665,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
         }
         // ---- tier 0: this warp's regions of the block, 32 at a time ----
         const uint32_t inv = ((1u << 20) + w - 1) / w;   // q / w = (q * inv) >> 20 for q < 1,024, w <= 32
+        const uint64_t lcg0 = hut_lcg(U.seed, U.up.rx + (int)x0, U.up.rz + (int)z0, a.salt);
         uint32_t n1 = 0;
 #pragma unroll 1
         for (uint32_t b = (uint32_t)warp * 32u; b < n; b += kUThreads) {
@@ -630,17 +676,18 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
             bool pass = false;
             if (valid) {
                 const uint32_t qz = (q * inv) >> 20, qx = q - qz * w;
-                int cx, cz;
-                hut_chunk(U.seed, U.up.rx + (int)(x0 + qx), U.up.rz + (int)(z0 + qz), a.salt, cx, cz);
-                e = (uint32_t)(cx - U.ucx) | ((uint32_t)(cz - U.ucz) << 16);
+                int j, k;
+                hut_draws(lcg0 + qx * kHutX + qz * kHutZ, j, k);
+                const uint32_t ex = qx * 32u + (uint32_t)j, ez = qz * 32u + (uint32_t)k;   // chunks from the block's first
+                e = (x0 * 32u + ex) | ((z0 * 32u + ez) << 16);
                 bool in_band = true;
                 if constexpr (F32) {
-                    const uint32_t ex = (e & 0xFFFFu) - x0 * 32u, ez = (e >> 16) - z0 * 32u;
-                    const uint64_t s0 = S.fstep[0], s1 = S.fstep[1];
-                    sum = __fmul_rn(st.cf[0], lat_sample(S.lat.l0[0], S.nx[0], fixed_hi(S.bx[0], s0, ex),
-                                                         fixed_hi(S.bz[0], s0, ez)));
-                    sum = __fmaf_rn(st.cf[1], lat_sample(S.lat.l0[1], S.nx[1], fixed_hi(S.bx[1], s1, ex),
-                                                         fixed_hi(S.bz[1], s1, ez)), sum);
+                    const uint64_t s0 = S.c.fstep[0], s1 = S.c.fstep[1];
+                    sum = __fmul_rn(st.cf[0],
+                                    lat_sample(S.lat.l0[0], B.nx[0], fixed_hi(B.x[0], s0, ex), fixed_hi(B.z[0], s0, ez)));
+                    sum = __fmaf_rn(st.cf[1],
+                                    lat_sample(S.lat.l0[1], B.nx[1], fixed_hi(B.x[1], s1, ex), fixed_hi(B.z[1], s1, ez)),
+                                    sum);
                     pass = sum >= st.hi[1];
                     in_band = all_rechecks || (!pass && !(sum < st.lo[1]));
                 }
@@ -678,7 +725,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                 Real sum = 0;
                 if (q < n1) {
                     e = S.wl[warp][q];
-                    keep = unit_step<F32, F32>(S, a, U, W, k, all_rechecks, e, (e & 0xFFFFu) - x0 * 32u,
+                    keep = unit_step<F32, F32>(S, a, U, W, k, all_rechecks, e, &B, (e & 0xFFFFu) - x0 * 32u,
                                                (e >> 16) - z0 * 32u, S.ws[warp][q], sum);
                 }
                 const unsigned m = __ballot_sync(0xFFFFFFFFu, keep);
@@ -700,6 +747,8 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
         }
         __syncthreads();   // the block's lattice and the pool are settled
         const bool last_blk = blk + 1 == n_blocks;
+        // nothing to drain yet: the pool and the lists change again only past the next block's barrier
+        if (!last_blk && S.n_pool < kPoolFull) continue;
         for (;;) {
             // ---- the rest of the climate gates for the pool, every warp an equal share of it, so
             // that none waits for another's ----
@@ -710,12 +759,9 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
             if (drain) {
                 const uint32_t share = (take + kUWarps * 32 - 1) / (kUWarps * 32) * 32;
                 const uint32_t from = min(take, (uint32_t)warp * share), cnt = min(take - from, share);
-                for (uint32_t q = (uint32_t)lane; q < cnt; q += 32) {
-                    S.wl[warp][q] = S.pool[np - take + from + q];
-                    S.ws[warp][q] = S.pool_s[np - take + from + q];
-                }
                 if (tid == 0) S.n_pool = np - take;
-                unit_drain<F32>(S, a, U, W, cnt, all_rechecks, large);
+                unit_drain<F32>(S, a, U, W, S.pool + (np - take + from), S.pool_s + (np - take + from), cnt, all_rechecks,
+                                large);
                 __syncthreads();
             }
             const bool last = last_blk && np == take;   // no more climate survivors will come
@@ -742,17 +788,17 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                     if (first) {
                         const double rar = unit_quick(S, N_SPAGHETTI_RARITY, kBaseRarity, (double)(int)((uint32_t)hx * 2u),
                                                       50.0, (double)(int)((uint32_t)hz * 2u));
-                        const double er = S.err[0], sc = tunnel_scale(rar);
+                        const double er = F32 ? S.c.err[0] : 0.0, sc = tunnel_scale(rar);
                         const double px = (double)hx / sc, py = 50.0 / sc, pz = (double)hz / sc;
                         const double l = unit_quick(S, N_SPAGHETTI_1, kBaseSp1, px, py, pz);
                         const double m = unit_quick(S, N_SPAGHETTI_2, kBaseSp2, px, py, pz);
-                        const double sure = kSpagSure + 2.0 * fmax(S.err[1], S.err[2]);
+                        const double sure = kSpagSure + (F32 ? 2.0 * fmax(S.c.err[1], S.c.err[2]) : 0.0);
                         const bool edge = er > 0.0 && (fabs(rar + 0.5) <= er || fabs(rar) <= er || fabs(rar - 0.5) <= er);
                         if (!edge && fmax(fabs(sc * l), fabs(sc * m)) >= sure) {
                             // spaghetti(50) >= 0: the entrance term decides (its depth term is 0 at 50)
                             const double ent = unit_quick(S, N_CAVE_ENTRANCE, kBaseEntrance, (double)hx * 0.75, 25.0,
                                                           (double)hz * 0.75);
-                            if (ent + 0.37 >= S.err[3]) code = P1_ENTRANCE_50;
+                            if (ent + 0.37 >= (F32 ? S.c.err[3] : 0.0)) code = P1_ENTRANCE_50;
                         }
                         if (code < 0) S.und[atomicAdd(&S.n_und, 1u)] = e;
                     } else {
