@@ -42,6 +42,7 @@ constexpr int kList = kBlock * kBlock / kUWarps;   // a warp's regions of a bloc
 constexpr int kPoolFull = kUWarps * 64;       // pooled regions that start a drain: two full rounds a warp
 constexpr int kPool = kPoolFull + kBlock * kBlock;
 constexpr int kUSurv = kUThreads + kUWarps * kList;   // what waited and one drain's
+constexpr int kWide = 2 * kUWarps;            // last survivors that take the entrance gate a warp each
 constexpr int kUDeep = 256;                   // deep candidates finished here; more go to the ladder kernel's list
 static_assert(kUClim + kSlotsA <= kUTabs, "climate tables overlay ladder tables");
 
@@ -129,7 +130,7 @@ struct UnitSmem {
             float4 l0[2][kLat0 * kLat0];
             float4 l1[2][kLat1 * kLat1];
         } lat;
-        double mh[kUWarps][kMhSamples];        // a warp's candidate at maxHeight
+        double mh[kUWarps][2 * kSlotsB];       // a warp's survivor at 50 and 60, or candidate at maxHeight
         LadderVals lad;
     };
     uint32_t wl[kUWarps][kList];               // a warp's list: survivor words and their erosion sums
@@ -549,6 +550,40 @@ __device__ __noinline__ double unit_quick(const UnitSmem<F32> &S, int noise, int
     }
 }
 
+// Entrance at 50 and 60 of one survivor by one warp, a sample a lane: the code that ends it, or -1.
+// unit_entrance's operations; v holds 18 samples of each height.
+template <bool F32>
+__device__ __noinline__ int unit_entrance_warp(const UnitSmem<F32> &S, double *v, int hx, int hz) {
+    const SrcUnit src{S.tab, S.org, S.grad};
+    const int lane = threadIdx.x & 31, h = lane & 1, y = h ? 60 : 50;
+    double *const vh = v + h * kSlotsB;
+    auto sample = [&](int slot, double e) {
+        const int noise = c_slot_c[0][slot][0], sub = c_slot_c[0][slot][1], p = c_slot_c[0][slot][2];
+        double px, py, pz;
+        cave_point(noise, hx, y, hz, e, px, py, pz);
+        vh[slot] = slot_sample_call(src, slot, sub, c_noise[noise].lac[p], px, py, pz);
+    };
+    if (lane < 28) sample(lane < 20 ? lane >> 1 : (lane >> 1) + 4, 1.0);   // all but spaghetti_3d_1 and _2
+    __syncwarp();
+    const double e = tunnel_scale(combine_vals(N_SPAGHETTI_RARITY, vh + kBaseRarity, 1));
+    if (lane < 8) sample(kBaseSp1 + (lane >> 1), e);
+    __syncwarp();
+    const double t = (10.0 + (double)y) / 40.0;
+    const double cl = t < 0.0 ? 0.3 : (t > 1.0 ? 0.0 : lerp(t, 0.3, 0.0));
+    const double cc = combine_vals(N_CAVE_ENTRANCE, vh + kBaseEntrance, 1) + 0.37 + cl;
+    const double tv = combine_vals(N_SPAGHETTI_THICKNESS, vh + kBaseThickness, 1);
+    const double w = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
+    const double m = fabs(e * combine_vals(N_SPAGHETTI_1, vh + kBaseSp1, 1)) - w;
+    const double o = fabs(e * combine_vals(N_SPAGHETTI_2, vh + kBaseSp2, 1)) - w;
+    const double p = clampd(jmax(m, o), -1.0, 1.0);
+    const double mod = combine_vals(N_ROUGHNESS_MODULATOR, vh + kBaseRmod, 1);
+    const double rgh = combine_vals(N_ROUGHNESS, vh + kBaseRough, 1);
+    const double q = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
+    const bool out = jmin(cc, p + q) >= 0;
+    const unsigned b = __ballot_sync(0xFFFFFFFFu, out);   // the barrier also frees v
+    return (b & 1u) ? P1_ENTRANCE_50 : ((b & 2u) ? P1_ENTRANCE_60 : -1);
+}
+
 // One CTA per unit.  F32: the FP32 noise core with the block lattices (small coordinates only), else
 // FP64 samples throughout, in the reference's order.
 template <bool F32>
@@ -768,8 +803,41 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
             // ---- entrance gate.  First test, one survivor per thread: at y = 50 the entrance noise
             // and the two scaled spaghetti noises settle 70 % of the survivors (both terms of the
             // minimum >= 0); the rest take the whole formula at 50 and 60.  Full rounds only. ----
+            auto settle = [&](uint32_t e, int code) {   // ended by the entrance gate, or a candidate (-1)
+                if (code >= 0) {
+                    atomicAdd(&S.hist[code], 1u);
+                    unit_note(a, U, e, code, -1);
+                    return;
+                }
+                const uint32_t q = atomicAdd(&S.n_deep, 1u);
+                if (q < kUDeep) {
+                    S.deep[q] = e;
+                    return;
+                }
+                const uint32_t di = atomicAdd(&a.counters[CNT_DEEP], 1u);
+                if (di < a.cap_deep) {
+                    a.deep[2 * di] = blockIdx.x;
+                    a.deep[2 * di + 1] = region_word(e);
+                } else {
+                    atomicOr(&a.counters[CNT_OVERFLOW], 2u);
+                }
+            };
             for (;;) {
                 const uint32_t ns = S.n_surv, nu = S.n_und;
+                if (last && ns + nu <= kWide) {   // the unit's last few: a warp each
+                    for (uint32_t q = (uint32_t)warp; q < ns + nu; q += kUWarps) {
+                        const uint32_t e = q < ns ? S.surv[q] : S.und[q - ns];
+                        const int code = unit_entrance_warp(S, S.mh[warp], (U.ucx + (int)(e & 0xFFFFu)) * 16 + 3,
+                                                            (U.ucz + (int)(e >> 16)) * 16 + 3);
+                        if (lane == 0) settle(e, code);
+                    }
+                    __syncthreads();
+                    if (tid == 0) {
+                        S.n_total += ns;
+                        S.n_surv = S.n_und = 0;
+                    }
+                    break;
+                }
                 const bool second = nu >= kUThreads || (last && ns == 0 && nu > 0);
                 const bool first = !second && (ns >= kUThreads || (last && ns > 0));
                 __syncthreads();   // every thread has read the counts
@@ -784,8 +852,8 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                 __syncthreads();
                 if (have) {
                     const int hx = (U.ucx + (int)(e & 0xFFFFu)) * 16 + 3, hz = (U.ucz + (int)(e >> 16)) * 16 + 3;
-                    int code = -1;
                     if (first) {
+                        int code = -1;
                         const double rar = unit_quick(S, N_SPAGHETTI_RARITY, kBaseRarity, (double)(int)((uint32_t)hx * 2u),
                                                       50.0, (double)(int)((uint32_t)hz * 2u));
                         const double er = F32 ? S.c.err[0] : 0.0, sc = tunnel_scale(rar);
@@ -801,27 +869,11 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                             if (ent + 0.37 >= (F32 ? S.c.err[3] : 0.0)) code = P1_ENTRANCE_50;
                         }
                         if (code < 0) S.und[atomicAdd(&S.n_und, 1u)] = e;
+                        else settle(e, code);
                     } else {
-                        if (unit_entrance(S, hx, 50, hz) >= 0) code = P1_ENTRANCE_50;
-                        else if (unit_entrance(S, hx, 60, hz) >= 0) code = P1_ENTRANCE_60;
-                        if (code < 0) {
-                            const uint32_t q = atomicAdd(&S.n_deep, 1u);
-                            if (q < kUDeep) {
-                                S.deep[q] = e;
-                            } else {
-                                const uint32_t di = atomicAdd(&a.counters[CNT_DEEP], 1u);
-                                if (di < a.cap_deep) {
-                                    a.deep[2 * di] = blockIdx.x;
-                                    a.deep[2 * di + 1] = region_word(e);
-                                } else {
-                                    atomicOr(&a.counters[CNT_OVERFLOW], 2u);
-                                }
-                            }
-                        }
-                    }
-                    if (code >= 0) {
-                        atomicAdd(&S.hist[code], 1u);
-                        unit_note(a, U, e, code, -1);
+                        settle(e, unit_entrance(S, hx, 50, hz) >= 0   ? P1_ENTRANCE_50
+                                  : unit_entrance(S, hx, 60, hz) >= 0 ? P1_ENTRANCE_60
+                                                                      : -1);
                     }
                 }
                 __syncthreads();
