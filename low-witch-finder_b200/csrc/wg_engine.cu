@@ -45,6 +45,42 @@ bool wg::few_units(uint64_t n_seeds, double n_regions, int sm_count, bool fp32) 
     return (double)n_seeds <= (fp32 ? 6.0 : 3.0) * sm_count * (1.0 + n_regions / 1024.0);
 }
 
+// Tiles of the one-CTA kernel that fill whole waves of its resident CTAs.  A wave lasts as long as its tiles'
+// regions and about 2,000 more (the table builds, the last gates), and a part of a wave, whose CTAs have the
+// SM to themselves, not as long.  The tilings of one to four waves are compared by that.  Against tiles of an
+// eighth of a slot's share (2,048 regions at least), one seed: 400 x 400 regions 100 -> 88 us, 2000 x 2000
+// 429 -> 249 us (3 units a slot, then 1), 6000 x 6000 1.87 -> 1.44 ms; 40 seeds x 600 x 600 1.01 -> 0.59 ms.
+// Requests past four waves of the largest tiles take those, and those of more seeds than four waves one a seed.
+static Tiling wave_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, uint64_t slots) {
+    constexpr uint64_t kWaveRegions = 2000, kMaxSide = 1023;
+    uint64_t best = ~0ull, btw = 0, bth = 0;
+    for (uint64_t waves = 1; waves <= 4; waves++) {
+        const uint64_t m = std::min(waves * slots / n_seeds, (rw * rh + 31) / 32);   // tiles per seed
+        if (m == 0) continue;
+        const double square = std::sqrt((double)m * (double)rw / (double)rh);
+        const uint64_t lo = std::max<uint64_t>(1, (uint64_t)(square * 0.6)), hi = std::min<uint64_t>({rw, m, (uint64_t)(square * 1.7) + 1});
+        for (uint64_t nx = lo; nx <= hi; nx++) {
+            const uint64_t tw = (rw + nx - 1) / nx, nz = std::min(rh, m / ((rw + tw - 1) / tw)), th = (rh + nz - 1) / nz;
+            if (tw > kMaxSide || th > kMaxSide || tw * th > kUnitCtaMax) continue;
+            const uint64_t units = n_seeds * ((rw + tw - 1) / tw) * ((rh + th - 1) / th), part = units % slots;
+            const uint64_t cost = (units / slots) * (tw * th + kWaveRegions) +
+                                  (part ? kWaveRegions + tw * th * (2 * slots + 3 * part) / (5 * slots) : 0);
+            if (cost < best) {
+                best = cost;
+                btw = tw;
+                bth = th;
+            }
+        }
+    }
+    if (best == ~0ull) return tile_rect(rw, rh, kUnitCtaMax);
+    Tiling t;
+    t.tw = (uint32_t)btw;
+    t.th = (uint32_t)bth;
+    t.ntx = (uint32_t)((rw + btw - 1) / btw);
+    t.n_win = t.ntx * ((rh + bth - 1) / bth);
+    return t;
+}
+
 // Whether a request's units take the one-CTA kernel, and its tiles.  Many regions per seed: yes, a
 // tile's two table builds (13,000 warp instructions) are then a small part of it, and the ladder and
 // the entrance gate find the seed's tables built.  Few units (few_units): yes too, in tiles small
@@ -55,10 +91,7 @@ static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, const wg
     const double total = (double)n_seeds * (double)n_regions;
     cta = !single_biome && (n_regions >= kUnitCtaRegions || few_units(n_seeds, (double)n_regions, eng->sm_count, eng->fp32_core != 0));
     if (!cta) return tile_rect(rw, rh, n_regions <= 4096 ? n_regions : 2048);
-    // one tile per resident CTA up to 2,048 regions each, then several waves of larger ones
-    uint64_t target = (uint64_t)(total / (double)slots) + 1;
-    if (target > 2048) target = std::max<uint64_t>(2048, target / 8);
-    return tile_rect(rw, rh, std::min<uint64_t>(std::max<uint64_t>(target, 32), kUnitCtaMax));
+    return wave_tiles(rw, rh, n_seeds, slots);
 }
 
 // Climate evaluation steps (see ClimateStep): the tiered erosion sequence
