@@ -42,7 +42,7 @@ Tiling wg::tile_rect(uint64_t rw, uint64_t rh, uint64_t target) {
 }
 
 bool wg::few_units(uint64_t n_seeds, double n_regions, int sm_count, bool fp32) {
-    return (double)n_seeds <= (fp32 ? 6.0 : 3.0) * sm_count * (1.0 + n_regions / 1024.0);
+    return (double)n_seeds <= (fp32 ? 9.0 + n_regions / 67.0 : 6.5 + n_regions / 138.0) * sm_count;
 }
 
 // Tiles of the one-CTA kernel that fill whole waves of its resident CTAs.  A wave lasts as long as its tiles'
@@ -88,8 +88,9 @@ static Tiling wave_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, uint64_t sl
 // and one evaluation of latency instead of three.  Otherwise 16 units share a CTA.
 static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, const wg_engine *eng, bool single_biome, bool &cta) {
     const uint64_t n_regions = rw * rh, slots = (uint64_t)eng->sm_count * 3;
-    const double total = (double)n_seeds * (double)n_regions;
     cta = !single_biome && (n_regions >= kUnitCtaRegions || few_units(n_seeds, (double)n_regions, eng->sm_count, eng->fp32_core != 0));
+    const uint64_t across = std::min(rw, rh);
+    if (across < kUnitCtaStrip) cta = cta && (double)n_seeds * std::ceil((double)std::max(rw, rh) / 1023.0) <= 4.0 * (double)slots;
     if (!cta) return tile_rect(rw, rh, n_regions <= 4096 ? n_regions : 2048);
     return wave_tiles(rw, rh, n_seeds, slots);
 }

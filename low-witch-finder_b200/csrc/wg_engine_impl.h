@@ -140,9 +140,15 @@ Tiling tile_rect(uint64_t rw, uint64_t rh, uint64_t target);
 // Regions per seed from which a unit takes the one-CTA kernel (launch_unit) however many seeds there
 // are: 8,192 seeds x 2,025 regions take it 1.73 ms and the list kernels 1.41; 3,552 x 4,096 1.07 and 1.99.
 constexpr uint64_t kUnitCtaRegions = 3072;
-// Whether so few units are better off with one CTA each (one wave of sm_count * 3 CTAs takes 70 to
-// 150 us, the fused kernels 100 to 200 whatever the number): 81 regions, 888 seeds 154 us and 162 fused,
-// 1,332 183 and 164; 1,024 regions, 1,776 seeds 337 and 367, 3,552 582 and 477.  FP64 units take longer.
+// A strip of fewer regions across than this makes tiles of few regions (a tile is at most 1,023 long), so it
+// takes the one-CTA kernel only for a few waves of them: 1,000 seeds x 20,000 x 1 3.11 ms and 1.66 fused, x
+// 10,000 x 3 2.44 and 2.36, x 10,000 x 4 2.88 and 2.97; one seed x 1,000,000 x 1 0.21 and 0.54.
+constexpr uint64_t kUnitCtaStrip = 4;
+// Whether so few units are better off with one CTA each (a wave of sm_count * 3 CTAs takes 40 to 120 us,
+// the fused kernels 125 to 450 whatever the number): 64 regions, 1,332 seeds 129 us and 129 fused, 1,776 148
+// and 136; 400 regions, 1,776 seeds 209 and 216, 2,664 286 and 271; 1,600 regions, 2,664 seeds 496 and 626,
+// 5,328 925 and 960.  FP64 units take longer: 64 regions, 888 seeds 107 and 131, 1,332 157 and 129; 400
+// regions, 1,332 seeds 217 and 217; 1,600 regions, 2,664 seeds 711 and 713, 3,552 916 and 780.
 bool few_units(uint64_t n_seeds, double n_regions, int sm_count, bool fp32);
 // Regions per unit of the one-CTA kernel at most.
 constexpr uint64_t kUnitCtaMax = 1ull << 16;
@@ -189,13 +195,18 @@ struct Sink {            // where phase-1 survivors go after each batch
 // 358 and 391 us, 24,576 482 and 467, 131,072 2,030 and 1,650; 1 x 2 regions: 228 and 270, 296 and 297,
 // 1,048 and 679).
 constexpr uint32_t kListUnits = 24576;
+// Strips of one or two regions longer than this keep the fused kernels, whose samples do not need a lattice:
+// 600,000 seeds x 200 x 1 13.8 ms and 14.9 fused, x 100 x 2 13.2 and 14.7; 60,000 x 1,000 x 1 5.17 and 4.58, x
+// 1,000 x 2 8.84 and 8.24.
+constexpr uint32_t kListStrip = 500;
 // The same for the cave gate of one-region units, 1.7 % of which reach it.
 constexpr uint32_t kSpotListUnits = 1u << 19;
 // Allocates the list kernels' lists once per engine.
 int list_buffers(wg_engine *eng);
 // Whether a batch of n_units units takes the list kernels.
 inline bool list_path(const BatchArgs &a, uint32_t n_units) {
-    return !a.unit_cta && a.fp32_core == 1 && a.small_coords && !a.single_biome && n_units >= kListUnits;
+    const bool strip = !a.jobs && std::min(a.tw, a.th) <= 2 && std::max(a.tw, a.th) > kListStrip;
+    return !a.unit_cta && a.fp32_core == 1 && a.small_coords && !a.single_biome && n_units >= kListUnits && !strip;
 }
 // The BatchArgs fields every batch of an engine shares (work lists, counters, rules, salt).
 BatchArgs base_args(wg_engine *eng, const wg_opts &opts, int salt);

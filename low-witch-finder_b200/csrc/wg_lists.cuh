@@ -30,6 +30,14 @@ constexpr int kEWarps = 4, kEThreads = 32 * kEWarps;   // erosion CTAs: three on
 constexpr int kLList = 224;                 // tier-0 survivors a warp carries (a 9 x 9 group has 139 on average)
 constexpr int kLLate = 64;                  // and those past step 3 (28 on average)
 
+// Regions along one side of a tier-0 block of a tile `other` regions wide across it: kLBlock, or in a thin
+// tile as many as the lattice's columns hold (23 for one region; 9 of them left 23 lanes idle).
+__host__ __device__ constexpr uint32_t list_side(uint32_t other) {
+    if (other >= (uint32_t)kLBlock) return kLBlock;
+    const uint32_t s = lattice_side(kLLat * kLLat, other, 255);
+    return s > (uint32_t)kLBlock ? s : kLBlock;
+}
+
 // unit_pos out of line: its divisions and table search would fill the instruction cache.
 __device__ __noinline__ UnitPos unit_pos_call(const BatchArgs &a, uint32_t u) { return unit_pos(a, u); }
 
@@ -300,7 +308,8 @@ __global__ void __launch_bounds__(kEThreads, 4) erosion_kernel(const __grid_cons
             const int rx = __shfl_sync(0xFFFFFFFFu, up.rx, src), rz = __shfl_sync(0xFFFFFFFFu, up.rz, src);
             const uint32_t tw = __shfl_sync(0xFFFFFFFFu, up.tw, src), th = __shfl_sync(0xFFFFFFFFu, up.th, src);
             const uint64_t sd = __shfl_sync(0xFFFFFFFFu, seed, src);
-            const uint32_t nbx = (tw + kLBlock - 1) / kLBlock, nbz = (th + kLBlock - 1) / kLBlock;
+            const uint32_t side_x = list_side(th), side_z = list_side(tw);
+            const uint32_t nbx = (tw + side_x - 1) / side_x, nbz = (th + side_z - 1) / side_z;
             const uint32_t bw = (tw + nbx - 1) / nbx, bh = (th + nbz - 1) / nbz;
             const uint64_t sa = st[0].fstep, sb = st[1].fstep;
 #pragma unroll 1
@@ -345,7 +354,7 @@ __global__ void __launch_bounds__(kEThreads, 4) erosion_kernel(const __grid_cons
                         W.lat[tb ? 1 : 0][i] = v;
                     }
                     __syncwarp();
-                    const uint32_t inv = ((1u << 16) + w - 1) / w;   // q / w = (q * inv) >> 16 for q < 81, w <= 9
+                    const uint32_t inv = ((1u << 16) + w - 1) / w;   // q / w = (q * inv) >> 16 for q < 105, w <= 23
 #pragma unroll 1
                     for (uint32_t b = 0; b < n; b += 32) {
                         const uint32_t q = b + (uint32_t)lane;

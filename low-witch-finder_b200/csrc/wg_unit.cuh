@@ -114,6 +114,20 @@ static void upload_unit_tables(const NoiseSpec *specs, const ClimateStep *const 
     cudaMemcpyToSymbol(g_unit_tables, host, sizeof host);
 }
 
+// Regions along one side of a block of a tile that is `other` regions wide across it: kBlock, or in a thin
+// tile as many as the lattices' columns hold (149 for one region: with 32 a block fed one warp of eight).
+// n regions span at most 0.255 n cells of octave 1/512 and 0.51 n of 1/256, and 3 columns more.
+__host__ __device__ constexpr uint32_t lattice_side(uint32_t columns, uint32_t other, uint32_t per_1000) {
+    return ((columns / (other * per_1000 / 1000 + 3) - 2) * 1000 - 1) / per_1000;
+}
+__host__ __device__ constexpr uint32_t block_side(uint32_t other) {
+    if (other >= (uint32_t)kBlock) return kBlock;
+    const uint32_t a = lattice_side(kLat0 * kLat0, other, 255), b = lattice_side(kLat1 * kLat1, other, 510),
+                   c = kBlock * kBlock / other;
+    const uint32_t s = a < b ? a : b, t = s < c ? s : c;
+    return t > (uint32_t)kBlock ? t : kBlock;
+}
+
 template <bool F32>
 struct UnitSmem {
     using Real = typename std::conditional<F32, float, double>::type;
@@ -646,7 +660,8 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
         }
     }
     __syncthreads();
-    const uint32_t nbx = (U.up.tw + kBlock - 1) / kBlock, nbz = (U.up.th + kBlock - 1) / kBlock;
+    const uint32_t side_x = block_side(U.up.th), side_z = block_side(U.up.tw);
+    const uint32_t nbx = (U.up.tw + side_x - 1) / side_x, nbz = (U.up.th + side_z - 1) / side_z;
     const uint32_t bw = (U.up.tw + nbx - 1) / nbx, bh = (U.up.th + nbz - 1) / nbz;
     const uint32_t n_blocks = nbx * nbz;
     auto lattice_base = [&](uint32_t blk) {   // one thread per table and axis, a block ahead of its use
@@ -683,7 +698,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
             for (int q = tid; q < m3; q += kUThreads) {
                 const int k = (q >= m0) + (q >= m1) + (q >= m2);
                 const int r = q - (k == 0 ? 0 : k == 1 ? m0 : k == 2 ? m1 : m2);
-                const int iz = (int)(((uint32_t)r * B.inv[k]) >> 20), ix = r - iz * B.nx[k];   // r < 361, nx <= 19
+                const int iz = (int)(((uint32_t)r * B.inv[k]) >> 20), ix = r - iz * B.nx[k];   // r < 361, nx <= 120
                 const uint8_t *P = S.tab + (kUClim + k) * kUPitch;
                 const uint8_t *Pj = P + S.jy[k], *Pk = P + ((B.cell_z[k] + iz) & 255);
                 const uint32_t pa = P[(B.cell_x[k] + ix) & 255];
@@ -699,7 +714,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
             __syncthreads();
         }
         // ---- tier 0: this warp's regions of the block, 32 at a time ----
-        const uint32_t inv = ((1u << 20) + w - 1) / w;   // q / w = (q * inv) >> 20 for q < 1,024, w <= 32
+        const uint32_t inv = ((1u << 20) + w - 1) / w;   // q / w = (q * inv) >> 20 for q < 1,024, w <= 149
         const uint64_t lcg0 = hut_lcg(U.seed, U.up.rx + (int)x0, U.up.rz + (int)z0, a.salt);
         uint32_t n1 = 0;
 #pragma unroll 1

@@ -48,9 +48,21 @@ def test_survivors_equal_the_list_kernels(engine, wg):
     assert st["tier_hist"] == whole.stats["tier_hist"]
 
 
+@pytest.mark.parametrize("preset", ["NORMAL", "LARGE_BIOMES"])
+@pytest.mark.parametrize("rect", [(0, 3, -160, 161), (-111, 110, 9, 13), (0, 8, 5, 92), (-60, 57, -40, -9)])
+def test_thin_tiles_equal_the_oracle(engine, port, bind_mod, preset, rect):
+    """Rects less than a block of 32 across, whose blocks are longer: one more region than a block's length."""
+    codes, tiers = engine.phase1_codes(seeds=[41, -8], rect=rect, max_height=-50, preset=preset)
+    for i, s in enumerate([41, -8]):
+        c, t, _, _ = port.phase1_rect(s, bind_mod.rules("1.19.x~26.1", preset), -50, rect)
+        assert np.array_equal(codes[i], c)
+        assert np.array_equal(tiers[i], t)
+
+
 @pytest.mark.parametrize("version,preset", [("1.19.x~26.1", "NORMAL"), ("26.2", "LARGE_BIOMES"), ("1.18.2", "NORMAL")])
 @pytest.mark.parametrize("n,rect", [(24576, (-4, 5, -4, 5)), (24579, (0, 1, 0, 3)), (25001, (7, 17, -30, -21)),
-                                    (24577, (58585, 58594, -58594, -58574))])
+                                    (24577, (58585, 58594, -58594, -58574)), (24576, (-30, 17, 0, 1)),
+                                    (24577, (4, 6, -12, 12)), (24580, (0, 16, 3, 10)), (24576, (0, 501, 0, 1))])
 def test_list_kernels_codes_equal_the_fp64_core(engine, version, preset, n, rect):
     """From 24,576 units of few regions on, the FP32 core takes the list kernels and the FP64 core the
     fused ones: every verdict equal, at unit counts that leave groups of units and records part full."""
