@@ -69,35 +69,29 @@ OPS_3D_SAMPLE = 56 + 192 + 24
 # x2), 24 gradient-component loads, 56 FP32 ops (3 offsets, 8 gradients x3, 3 fades x5, 7 lerps x2)
 OPS_3D_SAMPLE_F32 = 56 + 54 + 24 + 56
 OPS_REGION = 40              # java.util.Random placement (2 x nextInt(24)) + coordinates
-# dram__bytes_read.sum + dram__bytes_write.sum per launch, from ncu on `bench.py --profile 1048576`
-# (one launch of each kernel on 2^20 seeds read from a list in HBM; a 2^24-seed step runs 16 such
-# launches, each over its own 2^20 seeds, so the per-launch figure is the full step's per launch)
-TRAFFIC = {"climate_kernel": 8473088 + 256, "entrance_kernel": 20939520 + 0,
-           "source": "climate: ncu --set full --clock-control none -k regex:climate_kernel -s 1 -c 1 python bench.py "
-                     "--profile 1048576 --warmup 1 --steps 1; entrance: ncu --metrics "
-                     "dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k "
-                     "regex:'climate_kernel|entrance_kernel|ladder_kernel' -s 3 -c 3 python bench.py --profile "
-                     "1048576 --warmup 1 --steps 1 (the timed step's launch; read + write bytes)"}
-# ncu pipe utilisation of the same launches (the --set full captures of one climate and one entrance
-# launch on 2^20 seeds kept under profiles/): the counters behind the issue-rate roofline.  The integer
-# ALU pipe issues 64 lanes per clock per SM, half the 128-lane issue rate the roofline divides by,
-# and carries most of the table builds.
-PIPES = {"climate_kernel": {"issue_active": 0.667, "alu": 0.589, "fma": 0.226, "fp64": 0.021,
-                            "shared_wavefronts": 0.736, "warps_active": 0.275},
-         "entrance_kernel": {"issue_active": 0.574, "alu": 0.553, "fma": 0.153, "fp64": 0.079,
-                             "shared_wavefronts": 0.723, "warps_active": 0.278},
-         "unit": "fraction of peak, ncu --set full of one launch on 2^20 seeds"}
+# Tables that the first stage of the FP32 core builds per seed of 9 x 9 regions: 8 erosion for every seed, 4
+# temperature for the 75 % with a region past erosion, 6 ridge for 58 %, 12 of the cave gates for 53 %.
+LIST_TABLES = 8 + 0.75 * 4 + 0.58 * 6 + 0.53 * 12
+# ncu counters of the erosion kernel, the longest of the step (2^20 seeds, one launch): DRAM read + write bytes
+# and pipe utilisation as fractions of peak.
+TRAFFIC = {"erosion_kernel": 8452608 + 831744, "source": "ncu --clock-control none -k regex:erosion_kernel -s 1 -c 1 "
+                                            "python bench.py --profile 1048576 --warmup 1 --steps 1"}
+PIPES = {"erosion_kernel": {"issue_active": 0.646, "alu": 0.550, "fma": 0.250, "shared_wavefronts": 0.688,
+                            "warps_active": 0.221},
+         "gate_kernel": {"issue_active": 0.635, "alu": 0.679, "fma": 0.182, "shared_wavefronts": 0.732,
+                         "warps_active": 0.243},
+         "unit": "fraction of peak"}
 BYTES_PER_SEED_IN = 8        # the int64 seed read from HBM
 BYTES_PER_RECORD = 12        # (unit, offset, count) per seed with climate survivors
 BYTES_PER_SURVIVOR = 4       # region offset per climate survivor
 
 
-def climate_work(st: dict, n_seeds: int, n_regions: int, fp32: bool) -> tuple[float, float]:
-    """(lane-ops, algorithmic bytes) of the climate kernel over a request, from its funnel."""
+def climate_work(st: dict, n_seeds: int, n_regions: int, fp32: bool, lists: bool) -> tuple[float, float]:
+    """(lane-ops, algorithmic bytes) of the first stage over a request, from its funnel."""
     th = st["tier_hist"]
     rh = st["reject_hist"]
     y0 = sum((t + 2) * th[t] for t in range(7)) + 12 * rh[1] + 18 * (rh[2] + st["climate_survivors"])
-    ops = (18 * n_seeds * OPS_PERLIN_BUILD + y0 * (OPS_Y0_SAMPLE_F32 if fp32 else OPS_Y0_SAMPLE)
+    ops = ((LIST_TABLES if lists else 18) * n_seeds * OPS_PERLIN_BUILD + y0 * (OPS_Y0_SAMPLE_F32 if fp32 else OPS_Y0_SAMPLE)
            + n_seeds * n_regions * OPS_REGION)
     nbytes = n_seeds * BYTES_PER_SEED_IN + st["climate_survivors"] * BYTES_PER_SURVIVOR
     return float(ops), float(nbytes)
@@ -210,6 +204,16 @@ def process_per_seed_baseline(lysh: str, seeds, cores: int) -> dict:
                       f"(hunt.py's CPU mode), {cores} at a time", "seconds": secs}
 
 
+def needs_tables(measure, *args, **kw) -> dict:
+    """A side measurement that needs the game data tables; without them, why it is missing."""
+    try:
+        return measure(*args, **kw)
+    except load_package().EngineError as e:
+        if "game data tables" not in str(e):
+            raise
+        return {"unavailable": str(e)}
+
+
 def phase2_measure(eng, cands, opts, cpu: bool) -> dict:
     """Phase 2 (lysh_eval_hut: biome gate, aquifer flood, carvers, footprint heights) of the step's
     phase-1 survivors through wg_eval_huts, host buffers in and out (wall clock, 3 timed calls
@@ -314,12 +318,15 @@ def deep_measure(eng, opts) -> dict:
     rng = np.random.default_rng(9)
     fin = hits[:1024]
     fin_ws = [((int(u) << 48) | (int(s) & 0xFFFFFFFFFFFF)) for u, s in zip(rng.integers(0, 1 << 16, len(fin)), fin["s48"])]
-    eng.finish_rows(fin_ws[:2], fin["chunk_x"][:2], fin["chunk_z"][:2])
-    frows, fin_s = median_wall(lambda: eng.finish_rows(fin_ws, fin["chunk_x"], fin["chunk_z"]))
-    finisher = {"rows": len(fin_ws), "rows_per_s": len(fin_ws) / fin_s, "ms": 1e3 * fin_s,
+
+    def finisher() -> dict:
+        eng.finish_rows(fin_ws[:2], fin["chunk_x"][:2], fin["chunk_z"][:2])
+        frows, fin_s = median_wall(lambda: eng.finish_rows(fin_ws, fin["chunk_x"], fin["chunk_z"]))
+        return {"rows": len(fin_ws), "rows_per_s": len(fin_ws) / fin_s, "ms": 1e3 * fin_s,
                 "accepted_by_lysh": int(frows["verdict_ok"].sum()), "trees": int((frows["tree_status"] == 0).sum()),
                 "pieces": int(frows["pieces"].sum()),
                 "cpu_baseline": finisher_cpu_baseline(fin_ws[:16], fin["chunk_x"][:16], fin["chunk_z"][:16])}
+
     return {"solver": {"plan": "231564844655014 22 odd", "groups": sst["groups"], "regions": sst["regions"],
                        "tasks": sst["tasks"], "candidates": sst["candidates"], "hits": sst["hits"],
                        "tasks_per_s": sst["tasks"] / solve_s, "groups_per_s": sst["groups"] / solve_s,
@@ -341,7 +348,7 @@ def deep_measure(eng, opts) -> dict:
                             "upper-16-bit world seeds); the terrain stage that expands a match runs at the "
                             "`terrain` rate; the reference's own figure is about 94 M world seeds/s for that "
                             "stage (hunt.py:463-464)")},
-            "finisher": finisher,
+            "finisher": needs_tables(finisher),
             "timing": "wall clock around wg_deep_solve / wg_deep_starts / wg_deep_spots / wg_finish_rows (host "
                       "buffers in and out; the median of three calls each); device time of the solver from its "
                       "CUDA events"}
@@ -737,10 +744,12 @@ def main() -> None:
         max_mhz = float(peaks.get("sm_max_mhz", 1965.0))
         peak_ops = sm_count * 128 * max_mhz * 1e6
         fp32 = args.noise_core in ("fp32", "fp32_caves")
-        ops, nbytes = climate_work(stats, N_SEEDS, n_regions, fp32)
-        launch_ms = kernel_ms[0] / max(1, kernel_launches[0])
-        ops_per_launch = ops / max(1, stats["kernel_launches"][0])
-        bytes_per_launch = nbytes / max(1, stats["kernel_launches"][0])
+        lists = args.noise_core == "fp32"   # the FP32 core's first stage: the list kernels, six a batch
+        ops, nbytes = climate_work(stats, N_SEEDS, n_regions, fp32, lists)
+        batches = max(1, stats["batches"])
+        launch_ms = kernel_ms[0] / args.steps / batches
+        ops_per_launch = ops / batches
+        bytes_per_launch = nbytes / batches
         achieved = ops_per_launch / (launch_ms / 1e3)
         ent_ms = kernel_ms[1] / max(1, kernel_launches[1])
         caves32 = args.noise_core == "fp32_caves"   # the cave samples are FP32 only in that core
@@ -769,32 +778,33 @@ def main() -> None:
             "gpu_launches": sum(kernel_launches),
             "kernel_ms_per_step": [k / args.steps for k in kernel_ms],
             "roofline": {
-                "bound": "issue", "kernel": "climate_kernel", "unit": "Tlane-op/s",
+                "bound": "issue", "kernel": "erosion_kernel + gate_kernel" if lists else "climate_kernel",
+                "unit": "Tlane-op/s",
                 "achieved": achieved / 1e12, "peak": peak_ops / 1e12, "frac": achieved / peak_ops,
                 "peak_source": f"nominal INT32/FP32 issue rate: {sm_count} SMs x 128 lanes x {max_mhz:.0f} MHz "
                                "(sm_max_mhz of MEASURED_PEAKS.json); the kernel is not HBM- or tensor-bound",
                 "ops_per_launch": ops_per_launch, "launch_ms": launch_ms,
-                "ops_model": ("18 Perlin tables per seed x 7,160 lane-ops, per y=0 sample "
+                "ops_model": (f"{LIST_TABLES if lists else 18:.1f} Perlin tables per seed x 7,160 lane-ops, per y=0 sample "
                               f"{OPS_Y0_SAMPLE_F32 if fp32 else OPS_Y0_SAMPLE} lane-ops x the samples the funnel "
                               "implies, 40 per (seed, region) placement"),
-                "traffic": TRAFFIC["climate_kernel"], "traffic_unit": "bytes per launch",
+                "traffic": TRAFFIC["erosion_kernel"], "traffic_unit": "bytes per erosion_kernel launch",
                 "traffic_source": TRAFFIC["source"],
-                "ncu_pipes": dict(PIPES["climate_kernel"], unit=PIPES["unit"]),
+                "ncu_pipes": PIPES,
                 "algorithmic_bytes": bytes_per_launch,
                 "hbm": {"achieved_gbs": bytes_per_launch / (launch_ms / 1e3) / 1e9, "peak_gbs": hbm_peak,
                         "frac": bytes_per_launch / (launch_ms / 1e3) / 1e9 / hbm_peak,
                         "peak_source": "hbm_gbs of MEASURED_PEAKS.json"},
-                "entrance_kernel": {
-                    "bound": "issue", "unit": "Tlane-op/s", "achieved": ent_ops / (ent_ms / 1e3) / 1e12,
-                    "peak": peak_ops / 1e12, "frac": ent_ops / (ent_ms / 1e3) / peak_ops, "ops_per_launch": ent_ops,
-                    "launch_ms": ent_ms, "traffic": TRAFFIC["entrance_kernel"], "traffic_unit": "bytes per launch",
-                    "ncu_pipes": dict(PIPES["entrance_kernel"], unit=PIPES["unit"]),
-                    "ops_model": ("18 Perlin tables per record x 7,160 lane-ops, per climate survivor 36 3-D samples "
-                                  f"x {OPS_3D_SAMPLE_F32 if caves32 else OPS_3D_SAMPLE} lane-ops + 600 for the octave "
-                                  "sums and the decision")},
             },
             "clocks": cs,
         }
+        if not lists:   # the list kernels settle most survivors in their own gates
+            line["roofline"]["entrance_kernel"] = {
+                "bound": "issue", "unit": "Tlane-op/s", "achieved": ent_ops / (ent_ms / 1e3) / 1e12,
+                "peak": peak_ops / 1e12, "frac": ent_ops / (ent_ms / 1e3) / peak_ops, "ops_per_launch": ent_ops,
+                "launch_ms": ent_ms,
+                "ops_model": ("18 Perlin tables per record x 7,160 lane-ops, per climate survivor 36 3-D samples "
+                              f"x {OPS_3D_SAMPLE_F32 if caves32 else OPS_3D_SAMPLE} lane-ops + 600 for the octave "
+                              "sums and the decision")}
         if world == 1:
             nc = noise_core_measure(wg, eng, args, step_device, stream, flush, headline)
             # the output buffer holds the last core measured
@@ -802,10 +812,11 @@ def main() -> None:
             hits_other = sorted_hits(wg, out_dev, nc[other]["found"])
             nc["same_hits_and_funnel"] = bool(nc["same_hits_and_funnel"] and np.array_equal(hits_other, hits_headline))
             line["noise_core"] = nc
-        line["phase2"] = phase2_measure(eng, res.candidates, opts, cpu=(world == 1 and not args.no_cpu_baseline))
+        line["phase2"] = needs_tables(phase2_measure, eng, res.candidates, opts,
+                                      cpu=(world == 1 and not args.no_cpu_baseline))
         line["whole_world"] = whole_world_measure(eng, opts)
         line["deep_dive"] = deep_measure(eng, opts)
-        line["biome_map"] = biome_measure(eng)
+        line["biome_map"] = needs_tables(biome_measure, eng)
         if world == 1 and not args.no_jobs:
             line["jobs"] = jobs_measure(wg, eng)
             line["serving"] = serving_measure(wg)

@@ -396,7 +396,7 @@ __device__ __forceinline__ double perlin_3d(const T &P, double ox, double oy, do
 //      |err| <= max(err a, err b) + |t err| * |b - a| + 2 u, with |b - a| <= 4
 //      x lerps: 3 u + 4 * 4 u + 2 u = 21 u;  y lerps: 21 u + 4 * u/2 + 2 u = 25 u;
 //      z lerp: 25 u + 4 * 4 u + 2 u = 43 u   (T slightly above 1 after rounding: x 1.0001)
-// So |FP32 sample - exact| <= 44 u = 2.62e-6 (kPerlinF32ErrUlps), and |sample| <= 2.  The
+// So |FP32 sample - exact| <= 44 u = 2.62e-6 (under kPerlinF32ErrUlps), and |sample| <= 2.  The
 // FP64 sample of the reference order is within ~1e-14 of the exact value; the gates add that
 // and the sums' own roundings (build_climate_steps).  No FMA contraction is left to the
 // compiler: every FP32 operation below is an explicit intrinsic.

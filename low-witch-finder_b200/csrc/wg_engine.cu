@@ -269,7 +269,7 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
         float ms = 0.f;
         cudaEventElapsedTime(&ms, eng->kev[k], eng->kev[k + 1]);
         st.kernel_ms[k] += ms;
-        st.kernel_launches[k]++;
+        st.kernel_launches[k] += k == 0 && lists ? kListKernels : 1;
     }
     if (eng->h_counters[CNT_OVERFLOW]) {
         if (n_units <= (a.unit_cta ? 1u : 32u)) return eng->fail(WG_ERR_CAPACITY, "phase-1 work list full even for the smallest batch");

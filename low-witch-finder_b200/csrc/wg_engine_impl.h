@@ -201,6 +201,7 @@ constexpr uint32_t kListUnits = 24576;
 constexpr uint32_t kListStrip = 500;
 // The same for the cave gate of one-region units, 1.7 % of which reach it.
 constexpr uint32_t kSpotListUnits = 1u << 19;
+constexpr int kListKernels = 6;   // launches of launch_lists
 // Allocates the list kernels' lists once per engine.
 int list_buffers(wg_engine *eng);
 // Whether a batch of n_units units takes the list kernels.

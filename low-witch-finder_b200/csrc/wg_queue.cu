@@ -232,7 +232,10 @@ int run_queue(wg_engine *eng, const BatchArgs &proto, uint64_t total_units, uint
     st.records += (int64_t)h.records;
     st.batches += (int64_t)h.slices;
     st.retries += (int64_t)h.retries;
-    for (int k = 0; k < 3; k++) st.kernel_launches[k] += (int64_t)(h.slices + h.retries);
+    const int64_t runs = (int64_t)(h.slices + h.retries);   // the unit kernel has no entrance kernel beside it
+    st.kernel_launches[0] += lists ? kListKernels * runs : runs;
+    st.kernel_launches[1] += a.unit_cta ? 0 : runs;
+    st.kernel_launches[2] += runs;
     st.kernel_ms[0] += ms;   // one graph: its time is booked on the climate kernel's line
     return WG_OK;
 }

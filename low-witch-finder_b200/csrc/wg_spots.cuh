@@ -6,7 +6,8 @@
 // each step samples only its own octave.  So the stage runs breadth first over lists in HBM:
 // tier 0 for every unit, then one kernel per erosion step over the survivors of the step before
 // (one table per item, the partial sum carried in the item), then temperature and ridge for the
-// erosion survivors; ridge survivors become unit records for the entrance kernel as usual.
+// erosion survivors; ridge survivors become unit records for the entrance kernel, or in batches of 2^19
+// units and more go through the cave gates of wg_lists.cuh first.
 // A lane owns one byte column of its warp's table area and builds one table at a time there; the warps
 // of a block wait for no other (24 warps an SM).  Measured, 256 spots (1.7e7 world seeds), the whole
 // stage: columns initialised byte by byte in 272-byte rows of a 256-thread block 20.4 ms, by the warp in
