@@ -15,7 +15,8 @@
 // and what the last three leave open (3 % of the climate survivors) goes to the entrance kernel,
 // which decides in FP64 at 50 and 60.  A warp owns its 32 tables (one byte column per lane, 32-byte
 // rows) and waits for no other warp, so the warps of an SM drift apart and one's build fills the issue
-// slots another's sampling leaves free.  Measured on 2^24 seeds x 9 x 9: see launch_lists.
+// slots another's sampling leaves free.  Measured on 2^24 seeds x 9 x 9: these six kernels 174 ms and the
+// entrance kernel's rest 6; the fused climate kernel 160 and the entrance kernel 74.
 //
 // Tier 0 takes its samples from lattice columns as the unit kernel does (wg_unit.cuh): a 9 x 9 block
 // spans 2.2 cells of octave 1/512, so 25 columns per table replace 81 three-dimensional samples.
@@ -26,7 +27,7 @@ constexpr int kRows = 257;                  // row 256 = row 0 (ColTableF)
 constexpr int kLBlock = 9;                  // regions per side of a tier-0 block
 constexpr int kLLat = 5;                    // its lattice columns per axis (2.2 cells)
 constexpr int kLUnits = 4;                  // units of a warp in the erosion kernel
-constexpr int kEWarps = 4, kEThreads = 32 * kEWarps;   // erosion CTAs: three on an SM, 18 warps, 12.2 KB a warp
+constexpr int kEWarps = 4, kEThreads = 32 * kEWarps;   // erosion CTAs: four on an SM, 16 warps at 128 registers
 constexpr int kLList = 224;                 // tier-0 survivors a warp carries (a 9 x 9 group has 139 on average)
 constexpr int kLLate = 64;                  // and those past step 3 (28 on average)
 
@@ -697,8 +698,6 @@ __global__ void __launch_bounds__(kLThreads, 5) gate_kernel(const __grid_constan
 }
 
 static unsigned long long g_smem_done_ero = 0, g_smem_done_gate[5] = {0, 0, 0, 0, 0};
-static int g_list_sms = 0, g_ero_per_sm = 0, g_gate_per_sm = 0;   // resident CTAs per SM
-
 static void prepare_list_launches() {
     allow_dynamic_smem(erosion_kernel, sizeof(ErosionSmem), g_smem_done_ero);
     allow_dynamic_smem(gate_kernel<G_TEMPERATURE>, sizeof(GateSmem), g_smem_done_gate[0]);
@@ -706,25 +705,34 @@ static void prepare_list_launches() {
     allow_dynamic_smem(gate_kernel<G_SCALED>, sizeof(GateSmem), g_smem_done_gate[2]);
     allow_dynamic_smem(gate_kernel<G_ENTRANCE>, sizeof(GateSmem), g_smem_done_gate[3]);
     allow_dynamic_smem(gate_kernel<G_ROUGH>, sizeof(GateSmem), g_smem_done_gate[4]);
-    if (!g_list_sms) {
-        int dev = 0;
+}
+
+// Grids of the resident CTAs; asked for once, by whichever thread comes first (after prepare_list_launches).
+struct ListGrids {
+    int erosion = 1, gate = 1;
+    ListGrids() {
+        int dev = 0, sms = 1, ero = 0, g = 8;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_list_sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_ero_per_sm, erosion_kernel, kEThreads, sizeof(ErosionSmem));
-        g_gate_per_sm = 8;
-        auto least = [](auto kernel) {
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ero, erosion_kernel, kEThreads, sizeof(ErosionSmem));
+        auto least = [&](auto kernel) {
             int n = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kLThreads, sizeof(GateSmem));
-            if (n < g_gate_per_sm) g_gate_per_sm = n;
+            if (n < g) g = n;
         };
         least(gate_kernel<G_TEMPERATURE>);
         least(gate_kernel<G_RIDGE>);
         least(gate_kernel<G_SCALED>);
         least(gate_kernel<G_ENTRANCE>);
         least(gate_kernel<G_ROUGH>);
-        if (g_ero_per_sm < 1) g_ero_per_sm = 1;
-        if (g_gate_per_sm < 1) g_gate_per_sm = 1;
+        erosion = sms * (ero < 1 ? 1 : ero);
+        gate = sms * (g < 1 ? 1 : g);
     }
+};
+static const ListGrids &list_grids() {
+    prepare_list_launches();
+    static const ListGrids grids;
+    return grids;
 }
 
 static RegionList stage_list(const BatchArgs &a, int list, int cnt) {
@@ -735,8 +743,7 @@ static RegionList stage_list(const BatchArgs &a, int list, int cnt) {
 
 // The first entrance tests for the climate survivors in lists[0].
 static void launch_cave_lists(const BatchArgs &a, cudaStream_t s) {
-    prepare_list_launches();
-    const int gate = g_list_sms * g_gate_per_sm;
+    const int gate = list_grids().gate;
     const RegionList none{}, open = stage_list(a, 2, CNT_RECORDS);
     gate_kernel<G_SCALED><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 0, CNT_CLIMATE_LIST),
                                                                     stage_list(a, 1, CNT_SCALED_LIST), open);
@@ -748,11 +755,10 @@ static void launch_cave_lists(const BatchArgs &a, cudaStream_t s) {
 // The climate and entrance stages of a batch: grids of the resident CTAs, whose warps take groups of
 // units or records in turn.  lists[0], lists[1] alternate; lists[2] is the entrance kernel's input.
 void launch_lists(const BatchArgs &a, cudaStream_t s) {
-    prepare_list_launches();
-    const int gate = g_list_sms * g_gate_per_sm;
+    const int gate = list_grids().gate;
     BatchArgs b = a;
     b.lists[0].cnt = CNT_EROSION_LIST;
-    erosion_kernel<<<g_list_sms * g_ero_per_sm, kEThreads, sizeof(ErosionSmem), s>>>(b);
+    erosion_kernel<<<list_grids().erosion, kEThreads, sizeof(ErosionSmem), s>>>(b);
     const RegionList none{};
     gate_kernel<G_TEMPERATURE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 0, CNT_EROSION_LIST), stage_list(a, 1, CNT_TEMP_LIST), none);
     gate_kernel<G_RIDGE><<<gate, kLThreads, sizeof(GateSmem), s>>>(a, stage_list(a, 1, CNT_TEMP_LIST), stage_list(a, 0, CNT_CLIMATE_LIST), none);

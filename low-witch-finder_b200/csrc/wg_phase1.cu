@@ -1768,7 +1768,7 @@ void prepare_phase1_launches() {
     allow_dynamic_smem(entrance_kernel<false>, sizeof(EntranceSmem), g_smem_done_ent);
     allow_dynamic_smem(entrance_kernel<true>, sizeof(EntranceSmem), g_smem_done_ent32);
     prepare_unit_launches();
-    prepare_list_launches();
+    list_grids();
     ladder_geometry();
 }
 
