@@ -711,8 +711,10 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                 c.w = 0.0f;
                 (k < 2 ? S.lat.l0[k] : S.lat.l1[k - 2])[r] = c;
             }
-            __syncthreads();
         }
+        // Both cores: the lattice is complete, and every thread has read the last block's pool count (below)
+        // before a warp of this block adds to it.
+        __syncthreads();
         // ---- tier 0: this warp's regions of the block, 32 at a time ----
         const uint32_t inv = ((1u << 20) + w - 1) / w;   // q / w = (q * inv) >> 20 for q < 1,024, w <= 149
         const uint64_t lcg0 = hut_lcg(U.seed, U.up.rx + (int)x0, U.up.rz + (int)z0, a.salt);
@@ -797,7 +799,8 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
         }
         __syncthreads();   // the block's lattice and the pool are settled
         const bool last_blk = blk + 1 == n_blocks;
-        // nothing to drain yet: the pool and the lists change again only past the next block's barrier
+        // nothing to drain yet: the pool and the lists change again only past the barrier at the head of the next
+        // block's tier 0, which both cores have
         if (!last_blk && S.n_pool < kPoolFull) continue;
         for (;;) {
             // ---- the rest of the climate gates for the pool, every warp an equal share of it, so

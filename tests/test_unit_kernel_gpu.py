@@ -74,3 +74,28 @@ def test_list_kernels_codes_equal_the_fp64_core(engine, version, preset, n, rect
         engine.set_noise_core("fp32")
     assert np.array_equal(a[0], b[0])
     assert np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("core", ["fp64", "fp32"])
+@pytest.mark.parametrize("x0,z0", [(-128, -127), (2_999_900, -3_000_000)])
+def test_pools_drained_many_times_equal_the_oracle(engine, port, bind_mod, core, x0, z0):
+    """One tile of 65,536 regions a seed (64 blocks of 32 x 32): its pool fills and drains about ten times, in the
+    FP64 instance too (the FP64 core, and the FP32 core beyond its small coordinates)."""
+    rect, seeds = (x0, x0 + 256, z0, z0 + 256), [1473884015873122059, 11, -5]
+    engine.set_noise_core(core)
+    engine.set_tuning([0, 0, 0, 65536])
+    try:
+        per, st = engine.seed_check_jobs([{"seeds": seeds, "rect": rect, "max_height": 40}])
+    finally:
+        engine.set_tuning()
+        engine.set_noise_core("fp32")
+    assert st["kernel_launches"][1] == 0   # the unit kernel: no entrance kernel beside it
+    hist, tier, rows = np.zeros(len(st["reject_hist"]), np.int64), np.zeros(len(st["tier_hist"]), np.int64), []
+    for i, s in enumerate(seeds):
+        c, t, _, _ = port.phase1_rect(s, bind_mod.rules("1.19.x~26.1", "NORMAL"), 40, rect)
+        hist += np.bincount(c, minlength=len(hist))
+        tier += np.bincount(t[t >= 0], minlength=len(tier))
+        rows += [(i, x0 + int(r) % 256, z0 + int(r) // 256) for r in np.flatnonzero(c == len(hist) - 1)]
+    assert st["reject_hist"] == list(hist)
+    assert st["tier_hist"] == list(tier)
+    assert [(int(r["seed_index"]), int(r["rx"]), int(r["rz"])) for r in per[0]] == rows
