@@ -847,7 +847,10 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                         const uint32_t e = q < ns ? S.surv[q] : S.und[q - ns];
                         const int code = unit_entrance_warp(S, S.mh[warp], (U.ucx + (int)(e & 0xFFFFu)) * 16 + 3,
                                                             (U.ucz + (int)(e >> 16)) * 16 + 3);
-                        if (lane == 0) settle(e, code);
+                        if (lane == 0) {
+                            W.rechecks += all_rechecks;
+                            settle(e, code);
+                        }
                     }
                     __syncthreads();
                     if (tid == 0) {
@@ -886,9 +889,11 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                                                           (double)hz * 0.75);
                             if (ent + 0.37 >= (F32 ? S.c.err[3] : 0.0)) code = P1_ENTRANCE_50;
                         }
+                        if (all_rechecks) code = -1;   // the check mode: the whole formula in FP64 for every survivor
                         if (code < 0) S.und[atomicAdd(&S.n_und, 1u)] = e;
                         else settle(e, code);
                     } else {
+                        W.rechecks += all_rechecks;
                         settle(e, unit_entrance(S, hx, 50, hz) >= 0   ? P1_ENTRANCE_50
                                   : unit_entrance(S, hx, 60, hz) >= 0 ? P1_ENTRANCE_60
                                                                       : -1);

@@ -99,3 +99,23 @@ def test_pools_drained_many_times_equal_the_oracle(engine, port, bind_mod, core,
     assert st["reject_hist"] == list(hist)
     assert st["tier_hist"] == list(tier)
     assert [(int(r["seed_index"]), int(r["rx"]), int(r["rz"])) for r in per[0]] == rows
+
+
+@pytest.mark.parametrize("rect", [(-16, 16, -16, 16), (-150, 150, -150, 150)])
+def test_check_mode_takes_every_gate_again(engine, rect):
+    """fp32_recheck_all: one FP64 decision for each region at tier 0, for each that reaches one of the six
+    erosion steps after it, temperature and ridge, and for each climate survivor at the entrance gate."""
+    engine.set_noise_core("fp32_recheck_all")
+    try:
+        st = engine.seed_check(seeds=[1473884015873122059], rect=rect, max_height=-50).stats
+    finally:
+        engine.set_noise_core("fp32")
+    assert st["kernel_launches"][1] == 0 and st["climate_survivors"] > 0
+    tier, left = st["tier_hist"], st["scanned"]
+    want = left
+    for t in tier[:-1]:
+        left -= t
+        want += left
+    left -= tier[-1]
+    want += left + (left - st["reject_hist"][1]) + st["climate_survivors"]
+    assert st["rechecks"] == want
