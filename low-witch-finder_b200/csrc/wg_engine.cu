@@ -379,7 +379,7 @@ int copy_result(wg_engine *eng, void *dst, const void *src, size_t bytes) {
 
 int list_buffers(wg_engine *eng) {
     if (eng->list_block) return WG_OK;
-    const size_t rec = sizeof(uint32_t) * kCapRec, reg = sizeof(uint32_t) * kCapSurv, one = 3 * rec + 2 * reg;
+    const size_t rec = sizeof(uint32_t) * kCapRec, reg = sizeof(uint32_t) * kCapSurv, one = 3 * rec + 3 * reg;
     WG_CUDA(cudaMalloc(&eng->list_block, 2 * one), "alloc lists");
     for (int k = 0; k < 2; k++) {
         char *p = static_cast<char *>(eng->list_block) + k * one;
@@ -388,7 +388,7 @@ int list_buffers(wg_engine *eng) {
         L.off = reinterpret_cast<uint32_t *>(p + rec);
         L.rcnt = reinterpret_cast<uint32_t *>(p + 2 * rec);
         L.surv = reinterpret_cast<uint32_t *>(p + 3 * rec);
-        L.pay = reinterpret_cast<float *>(p + 3 * rec + reg);
+        L.pay = reinterpret_cast<double *>(p + 3 * rec + reg);
         L.cap_rec = kCapRec;
         L.cap_surv = kCapSurv;
         L.cnt = 0;

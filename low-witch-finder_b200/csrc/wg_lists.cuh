@@ -13,7 +13,8 @@
 //   rough caves  half of those              6 tables (thickness, roughness and its modulator), 5 per warp
 //
 // and what the last three leave open (3 % of the climate survivors) goes to the entrance kernel,
-// which decides in FP64 at 50 and 60.  A warp owns its 32 tables (one byte column per lane, 32-byte
+// which decides at 50 and 60.  The cave stages sample in FP64, as the entrance kernel does (in FP32, as
+// WG_NOISE_FP32_CAVES would have it, 2^24 seeds x 9 x 9 took 0.6 % less).  A warp owns its 32 tables (one byte column per lane, 32-byte
 // rows) and waits for no other warp, so the warps of an SM drift apart and one's build fills the issue
 // slots another's sampling leaves free.  Measured on 2^24 seeds x 9 x 9: these six kernels 174 ms and the
 // entrance kernel's rest 6; the fused climate kernel 160 and the entrance kernel 74.
@@ -142,7 +143,7 @@ __device__ __noinline__ double col_value64(const uint8_t *tab, int col, const ui
 // Appends n <= 32 regions (one per lane, of ascending record ids) to a list as records, one per run of
 // equal ids.  On a full list only the overflow flag is set; every later kernel of the batch then ends.
 __device__ __forceinline__ void list_emit(const BatchArgs &a, const RegionList &L, int lane, uint32_t n, uint32_t id,
-                                          uint32_t unit, uint32_t word, float pay) {
+                                          uint32_t unit, uint32_t word, double pay) {
     if (!n) return;
     const unsigned below = (1u << lane) - 1u;
     const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, id, 1);
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(kEThreads, 4) erosion_kernel(const __grid_cons
         uint32_t n1 = 0, n_out = 0;
         auto flush = [&](uint32_t n) {   // the first n <= 32 survivors to the list
             const uint32_t e = (uint32_t)lane < n ? W.out[lane] : 0u;
-            list_emit(a, a.lists[0], lane, n, e >> 30, u0 + (e >> 30), entry_word(e), 0.0f);
+            list_emit(a, a.lists[0], lane, n, e >> 30, u0 + (e >> 30), entry_word(e), 0.0);
         };
         // erosion steps 2..7 breadth first over the warp's list
         auto drain = [&]() {
@@ -442,7 +443,7 @@ struct GateWarp {
     uint32_t unit[8], off[8], first[9];   // first: the records' prefix of region counts
     uint32_t out[2][64];                  // regions not yet in the lists: their record here, offset word and value
     uint32_t word[2][64];
-    float pay[64];
+    double pay[64];
 };
 static_assert(sizeof(GateWarp) % 16 == 0, "warp_build writes 16 bytes at a time");
 struct GateSmem {
@@ -480,19 +481,6 @@ __global__ void __launch_bounds__(kLThreads, 5) gate_kernel(const __grid_constan
     const NoiseSpec &ns = c_noise[sl[0]];
     const int sub = sl[1], oct = sl[2];
     const uint64_t step = GateShape<G>::climate ? c_steps[large][k0 + my_p].fstep : 0;
-    // error bounds of the stage's FP32 DoublePerlin values
-    double er0 = 0.0, er1 = 0.0, er2 = 0.0;
-    if constexpr (G == G_SCALED) {
-        er0 = dp_err_f32(N_SPAGHETTI_RARITY);
-        er1 = fmax(dp_err_f32(N_SPAGHETTI_1), dp_err_f32(N_SPAGHETTI_2));
-    } else if constexpr (G == G_ENTRANCE) {
-        er0 = dp_err_f32(N_CAVE_ENTRANCE);
-        er1 = fmax(dp_err_f32(N_SPAGHETTI_1), dp_err_f32(N_SPAGHETTI_2));
-    } else if constexpr (G == G_ROUGH) {
-        er0 = dp_err_f32(N_SPAGHETTI_THICKNESS);
-        er1 = dp_err_f32(N_ROUGHNESS_MODULATOR);
-        er2 = dp_err_f32(N_ROUGHNESS);
-    }
     uint32_t rechecks = 0, rejected = 0;
     const uint32_t n_rec = min(a.counters[in.cnt], in.cap_rec);
     const uint32_t groups = (n_rec + R - 1) / R;
@@ -540,7 +528,7 @@ __global__ void __launch_bounds__(kLThreads, 5) gate_kernel(const __grid_constan
         uint32_t n_out[2] = {0, 0};
         auto flush = [&](int which, uint32_t n) {
             const uint32_t id = (uint32_t)lane < n ? W.out[which][lane] : 0u;
-            const float pay = which == 0 && (uint32_t)lane < n ? W.pay[lane] : 0.0f;
+            const double pay = which == 0 && (uint32_t)lane < n ? W.pay[lane] : 0.0;
             list_emit(a, which ? open : out, lane, n, id, W.unit[id], W.word[which][lane], pay);
         };
 #pragma unroll 1
@@ -551,7 +539,7 @@ __global__ void __launch_bounds__(kLThreads, 5) gate_kernel(const __grid_constan
             for (int q = 1; q < R; q++) r += i >= W.first[q] ? 1 : 0;
             uint32_t word = 0;
             int cx = 0, cz = 0;
-            float in_pay = 0.0f;
+            double in_pay = 0.0;
             if (have) {
                 const uint32_t at = W.off[r] + (i - W.first[r]);
                 word = in.surv[at];
@@ -560,7 +548,7 @@ __global__ void __launch_bounds__(kLThreads, 5) gate_kernel(const __grid_constan
             }
             const int col = r * K + my_p;
             bool keep = false, is_open = false;
-            float pay = 0.0f;
+            double pay = 0.0;
             int code = -1;
             if constexpr (GateShape<G>::climate) {
                 float v = 0.0f;
@@ -591,56 +579,51 @@ __global__ void __launch_bounds__(kLThreads, 5) gate_kernel(const __grid_constan
                 }
             } else {
                 const int hx = cx * 16 + 3, hz = cz * 16 + 3;
-                const ColTableF<32> T{W.tab + col, &S.gf};
-                const double scale = sub ? kDblScale : 1.0, lac = ns.lac[oct];
+                // FP64 samples in the reference's order, as everywhere in the default core's cave gates: what is
+                // decided here is the reference's decision.
+                const ColTable<32> T{W.tab + col, S.grad};
+                const double scale = sub ? kDblScale : 1.0, lac = ns.lac[oct], amp = ns.amp[oct], per = ns.per[oct];
                 auto sample = [&](double x, double y, double z) {
-                    return (double)perlin_3d_f32(T, W.org.x[col], W.org.y[col], W.org.z[col], keep_precision((x * scale) * lac),
-                                                 keep_precision((y * scale) * lac), keep_precision((z * scale) * lac)) *
-                           (ns.amp[oct] * ns.per[oct]);
+                    return (amp * perlin_3d(T, W.org.x[col], W.org.y[col], W.org.z[col], keep_precision((x * scale) * lac),
+                                            keep_precision((y * scale) * lac), keep_precision((z * scale) * lac))) *
+                           per;
                 };
-                // the DoublePerlin value of the noise whose tables are columns p and p + 1 of the region
+                // the DoublePerlin value of the noise whose 2 np tables are columns p, p + 1, .. of the region
                 const int lead = lane - my_p;
-                auto pair_sum = [&](double v, int p) {
-                    return (__shfl_sync(0xFFFFFFFFu, v, (lead + p) & 31) + __shfl_sync(0xFFFFFFFFu, v, (lead + p + 1) & 31));
+                auto value = [&](int noise, double v, int p, int np) {
+                    double s0 = 0.0, s1 = 0.0;
+                    for (int q = 0; q < np; q++) s0 += __shfl_sync(0xFFFFFFFFu, v, (lead + p + q) & 31);
+                    for (int q = 0; q < np; q++) s1 += __shfl_sync(0xFFFFFFFFu, v, (lead + p + np + q) & 31);
+                    return (s0 + s1) * c_noise[noise].amplitude;
                 };
                 if constexpr (G == G_SCALED) {
                     double v = 0.0;
                     if (have && my_p < 2) v = sample((double)(int)((uint32_t)hx * 2u), 50.0, (double)(int)((uint32_t)hz * 2u));
-                    const double rar = pair_sum(v, 0) * c_noise[N_SPAGHETTI_RARITY].amplitude;
-                    const double sc = tunnel_scale(rar);
+                    const double sc = tunnel_scale(value(N_SPAGHETTI_RARITY, v, 0, 1));
                     if (have && my_p >= 2) v = sample((double)hx / sc, 50.0 / sc, (double)hz / sc);
-                    const double l = pair_sum(v, 2) * c_noise[N_SPAGHETTI_1].amplitude,
-                                 m = pair_sum(v, 4) * c_noise[N_SPAGHETTI_2].amplitude;
-                    if (have && my_p == 0) {
-                        is_open = fabs(rar + 0.5) <= er0 || fabs(rar) <= er0 || fabs(rar - 0.5) <= er0;
-                        keep = !is_open;
-                        pay = (float)fmax(fabs(sc * l), fabs(sc * m));
-                    }
+                    const double l = value(N_SPAGHETTI_1, v, 2, 1), m = value(N_SPAGHETTI_2, v, 4, 1);
+                    keep = have && my_p == 0;
+                    pay = fmax(fabs(sc * l), fabs(sc * m));
                 } else if constexpr (G == G_ENTRANCE) {
                     const double v = have ? sample((double)hx * 0.75, 25.0, (double)hz * 0.75) : 0.0;
-                    const double ent = (pair_sum(v, 0) + pair_sum(v, 2) + pair_sum(v, 4)) * c_noise[N_CAVE_ENTRANCE].amplitude;
+                    const double ent = value(N_CAVE_ENTRANCE, v, 0, 3);
                     if (have && my_p == 0) {
                         // the entrance term's depth part is 0 at 50
-                        if (ent + 0.37 < er0) is_open = true;
-                        else if ((double)in_pay >= kSpagSure + 2.0 * er1 + 1e-6) code = P1_ENTRANCE_50;
+                        if (ent + 0.37 < 0) is_open = true;
+                        else if (in_pay >= kSpagSure) code = P1_ENTRANCE_50;
                         else keep = true;
                         pay = in_pay;
                     }
                 } else {
                     const double v = have ? sample((double)hx, 50.0, (double)hz) : 0.0;
-                    const double tv = pair_sum(v, 0) * c_noise[N_SPAGHETTI_THICKNESS].amplitude,
-                                 mod = pair_sum(v, 2) * c_noise[N_ROUGHNESS_MODULATOR].amplitude,
-                                 rgh = pair_sum(v, 4) * c_noise[N_ROUGHNESS].amplitude;
+                    const double tv = value(N_SPAGHETTI_THICKNESS, v, 0, 1), mod = value(N_ROUGHNESS_MODULATOR, v, 2, 1),
+                                 rgh = value(N_ROUGHNESS, v, 4, 1);
                     if (have && my_p == 0) {
                         const double h = lerp((tv - -1.0) / (1.0 - -1.0), 0.065, 0.088);
-                        const double p = clampd((double)in_pay - h, -1.0, 1.0);
+                        // the larger of the two differences is the larger term's: a rounded difference is monotone
+                        const double p = clampd(in_pay - h, -1.0, 1.0);
                         const double q = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
-                        // the bound of p + q: the scaled noises at the largest scale 2 (and the stored
-                        // float's rounding), the thickness with slope 0.0115, q as in the entrance kernel
-                        const double bound = (2.0 * fmax(dp_err_f32(N_SPAGHETTI_1), dp_err_f32(N_SPAGHETTI_2)) + 1e-6 + 0.0115 * er0 +
-                                              0.05 * er1 * (fabs(-0.4 + fabs(rgh)) + er2) + 0.05 * (1.0 + fabs(mod) + er1) * er2) *
-                                                 1.000001 + 1e-12;
-                        if (p + q >= bound) code = P1_ENTRANCE_50;
+                        if (p + q >= 0) code = P1_ENTRANCE_50;
                         else is_open = true;
                     }
                 }
@@ -674,7 +657,7 @@ __global__ void __launch_bounds__(kLThreads, 5) gate_kernel(const __grid_constan
                 flush(q, 32);
                 __syncwarp();
                 const uint32_t id = W.out[q][32 + lane], wd = W.word[q][32 + lane];
-                const float py = q == 0 ? W.pay[32 + lane] : 0.0f;
+                const double py = q == 0 ? W.pay[32 + lane] : 0.0;
                 __syncwarp();
                 W.out[q][lane] = id;
                 W.word[q][lane] = wd;

@@ -86,7 +86,7 @@ __host__ __device__ inline uint32_t climate_records(const uint32_t *c) {
 struct RegionList {
     uint32_t *unit, *off, *rcnt;   // per record: batch-local unit, first region, regions (<= 32)
     uint32_t *surv;                // per region: its offset in the unit's tile (dx | dz << 16)
-    float *pay;                    // per region: the value a later stage needs, or null
+    double *pay;                   // per region: the value a later stage needs, or null
     uint32_t cap_rec, cap_surv;
     int cnt;                       // its counters
 };

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kSpotThreads) spot_steps_kernel(const __grid_c
                 const unsigned m = __ballot_sync(0xFFFFFFFFu, passed);
                 const int src = (int)__fns(m, 0, (int)(threadIdx.x & 31) + 1) & 31;
                 const uint32_t unit = __shfl_sync(0xFFFFFFFFu, it.unit, src);
-                list_emit(a, a.lists[0], (int)(threadIdx.x & 31), (uint32_t)__popc(m), threadIdx.x & 31, unit, 0u, 0.0f);
+                list_emit(a, a.lists[0], (int)(threadIdx.x & 31), (uint32_t)__popc(m), threadIdx.x & 31, unit, 0u, 0.0);
             }
         }
         if (alive) {

@@ -61,8 +61,8 @@ struct LatBase {
     uint32_t inv[kLatTables];
 };
 
-// What the kernel keeps of the tables' constants (err: FP32 core, bounds of the first entrance test's four
-// noises), and each table's generator (climate tables in step order, then the cave tables).  In global
+// What the kernel keeps of the tables' constants (err: bounds of the first entrance test's four noises in
+// FP32), and each table's generator (climate tables in step order, then the cave tables).  In global
 // memory: lanes that read different words of constant memory take turns, and in a call of one wave every
 // turn is a miss (the 18 lanes' steps and generators: 10,000 of a CTA's 60,000 cycles, now 2,500).
 struct UnitConst {
@@ -540,11 +540,12 @@ __device__ __noinline__ double unit_entrance(const UnitSmem<F32> &S, int x, int 
     const double q = (-0.05 + (-0.05 * mod)) * (-0.4 + fabs(rgh));
     return jmin(cc, p + q);
 }
-// A DoublePerlin of the first entrance test: FP32 samples summed in FP64 (F32; within dp_err_f32 of
-// the reference's value), or the reference's.
+// A DoublePerlin of the first entrance test: the reference's, or where the caller chose FP32 cave samples
+// (cave32) those summed in FP64 (within dp_err_f32 of the reference's value).
 template <bool F32>
-__device__ __noinline__ double unit_quick(const UnitSmem<F32> &S, int noise, int base, double x, double y, double z) {
-    if constexpr (!F32) {
+__device__ __noinline__ double unit_quick(const UnitSmem<F32> &S, bool cave32, int noise, int base, double x, double y,
+                                          double z) {
+    if (!F32 || !cave32) {
         return unit_dbl(S.tab, S.org, S.grad, noise, base, x, y, z);
     } else {
         const NoiseSpec &ns = c_noise[noise];
@@ -610,6 +611,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
     const unsigned below = (1u << lane) - 1u;
     const int large = a.large_biomes ? 1 : 0;
     const bool all_rechecks = F32 && a.fp32_core == 2;
+    const bool cave32 = F32 && a.fp32_core >= 2;   // FP32 cave samples: WG_NOISE_FP32_CAVES and the check mode
     UnitCtx U;
     U.up = unit_pos(a, blockIdx.x);
     U.g = U.up.g;
@@ -875,19 +877,19 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                     const int hx = (U.ucx + (int)(e & 0xFFFFu)) * 16 + 3, hz = (U.ucz + (int)(e >> 16)) * 16 + 3;
                     if (first) {
                         int code = -1;
-                        const double rar = unit_quick(S, N_SPAGHETTI_RARITY, kBaseRarity, (double)(int)((uint32_t)hx * 2u),
+                        const double rar = unit_quick(S, cave32, N_SPAGHETTI_RARITY, kBaseRarity, (double)(int)((uint32_t)hx * 2u),
                                                       50.0, (double)(int)((uint32_t)hz * 2u));
-                        const double er = F32 ? S.c.err[0] : 0.0, sc = tunnel_scale(rar);
+                        const double er = cave32 ? S.c.err[0] : 0.0, sc = tunnel_scale(rar);
                         const double px = (double)hx / sc, py = 50.0 / sc, pz = (double)hz / sc;
-                        const double l = unit_quick(S, N_SPAGHETTI_1, kBaseSp1, px, py, pz);
-                        const double m = unit_quick(S, N_SPAGHETTI_2, kBaseSp2, px, py, pz);
-                        const double sure = kSpagSure + (F32 ? 2.0 * fmax(S.c.err[1], S.c.err[2]) : 0.0);
+                        const double l = unit_quick(S, cave32, N_SPAGHETTI_1, kBaseSp1, px, py, pz);
+                        const double m = unit_quick(S, cave32, N_SPAGHETTI_2, kBaseSp2, px, py, pz);
+                        const double sure = kSpagSure + (cave32 ? 2.0 * fmax(S.c.err[1], S.c.err[2]) : 0.0);
                         const bool edge = er > 0.0 && (fabs(rar + 0.5) <= er || fabs(rar) <= er || fabs(rar - 0.5) <= er);
                         if (!edge && fmax(fabs(sc * l), fabs(sc * m)) >= sure) {
                             // spaghetti(50) >= 0: the entrance term decides (its depth term is 0 at 50)
-                            const double ent = unit_quick(S, N_CAVE_ENTRANCE, kBaseEntrance, (double)hx * 0.75, 25.0,
+                            const double ent = unit_quick(S, cave32, N_CAVE_ENTRANCE, kBaseEntrance, (double)hx * 0.75, 25.0,
                                                           (double)hz * 0.75);
-                            if (ent + 0.37 >= (F32 ? S.c.err[3] : 0.0)) code = P1_ENTRANCE_50;
+                            if (ent + 0.37 >= (cave32 ? S.c.err[3] : 0.0)) code = P1_ENTRANCE_50;
                         }
                         if (all_rechecks) code = -1;   // the check mode: the whole formula in FP64 for every survivor
                         if (code < 0) S.und[atomicAdd(&S.n_und, 1u)] = e;
