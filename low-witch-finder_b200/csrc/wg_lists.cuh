@@ -80,10 +80,10 @@ __device__ __forceinline__ void clim_col(ClimCols &C, int col, const ClimateStep
 // One y = 0 sample of a column at chunk offset (dx, dz) from its unit's first chunk.
 __device__ __forceinline__ float col_sample(const uint8_t *tab, const ClimCols &C, const GradF &gf, int col, uint64_t step,
                                             uint32_t dx, uint32_t dz) {
-    const uint32_t hx = fixed_hi(C.fx[col], step, dx), hz = fixed_hi(C.fz[col], step, dz);
+    const uint64_t cx = fixed_at(C.fx[col], step, dx), cz = fixed_at(C.fz[col], step, dz);
     const ColTableF<32> T{tab + col, &gf};
-    return perlin_y0_cell_f32(T, (int)(hx >> 24), C.jy[col], (int)(hz >> 24), fixed_frac(hx), fixed_frac(hz), C.hyf[col],
-                              C.fyf[col]);
+    return perlin_y0_cell_f32(T, (int)fixed_cell(cx), C.jy[col], (int)fixed_cell(cz), fixed_frac(cx), fixed_frac(cz),
+                              C.hyf[col], C.fyf[col]);
 }
 
 // The FP64 sample of climate step k of `seed`, for the decisions an FP32 sum leaves open: the origins
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kEThreads, 4) erosion_kernel(const __grid_cons
                         const uint64_t f = (z ? W.col.fz[c] : W.col.fx[c]) + (uint64_t)((z ? bz : bx) * 32u) * step;
                         W.base[lane] = f & kFrac;
                         cell0 = (uint32_t)(f >> 56);
-                        cells = (fixed_hi(f & kFrac, step, ((z ? h : w) - 1) * 32u + 23u) >> 24) + 2;
+                        cells = fixed_cell(fixed_at(f & kFrac, step, ((z ? h : w) - 1) * 32u + 23u)) + 2;
                     }
                     const int nax = (int)__shfl_sync(0xFFFFFFFFu, cells, 0), naz = (int)__shfl_sync(0xFFFFFFFFu, cells, 1),
                               nbx2 = (int)__shfl_sync(0xFFFFFFFFu, cells, 2), nbz2 = (int)__shfl_sync(0xFFFFFFFFu, cells, 3);
@@ -370,10 +370,10 @@ __global__ void __launch_bounds__(kEThreads, 4) erosion_kernel(const __grid_cons
                             const uint32_t dx = (uint32_t)(cx - rx * 32), dz = (uint32_t)(cz - rz * 32);
                             e = ((uint32_t)u << 30) | (dz << 15) | dx;
                             const uint32_t ex = dx - bx * 32u, ez = dz - bz * 32u;
-                            sum = __fmul_rn(st[0].cf, lat_sample(W.lat[0], nax, fixed_hi(W.base[0], sa, ex),
-                                                                 fixed_hi(W.base[1], sa, ez)));
-                            sum = __fmaf_rn(st[1].cf, lat_sample(W.lat[1], nbx2, fixed_hi(W.base[2], sb, ex),
-                                                                 fixed_hi(W.base[3], sb, ez)), sum);
+                            sum = __fmul_rn(st[0].cf, lat_sample(W.lat[0], nax, fixed_at(W.base[0], sa, ex),
+                                                                 fixed_at(W.base[1], sa, ez)));
+                            sum = __fmaf_rn(st[1].cf, lat_sample(W.lat[1], nbx2, fixed_at(W.base[2], sb, ex),
+                                                                 fixed_at(W.base[3], sb, ez)), sum);
                             pass = sum >= st[1].hi;
                             if (!pass && !(sum < st[1].lo)) {
                                 rechecks++;

@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "wg_device.cuh"
+#include "wg_fixed.h"
 #include "wg_phase1.cuh"
 
 namespace wg {

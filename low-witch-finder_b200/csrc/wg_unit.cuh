@@ -14,10 +14,8 @@
 // memory, and a sample is four 16-byte loads and about 30 operations instead of 14 table lookups,
 // 8 gradients and a 3-D blend (about 170).
 //
-// Coordinates are 8.56 fixed point, mod 256 (the tables' period): base of the unit per table and
-// axis, plus the hut's chunk offset times the table's step, exact to 2^-40 of a cell over a unit.
-// The top 24 bits give the lattice cell and a 23-bit fraction (rounded by half a unit added to the
-// base), which costs no FP64 and no conversion instruction.
+// Coordinates are 8.56 fixed point (wg_fixed.h): base of the unit per table and axis, plus the hut's chunk
+// offset times the table's step, which costs no FP64.
 //
 // A block costs two barriers: the next block's lattice bases are formed a block ahead, and the pool is
 // looked at only when it is full.  (With six, and the lists packed after each of the erosion steps 4-7:
@@ -175,34 +173,21 @@ __device__ __forceinline__ void unit_note(const BatchArgs &a, const UnitCtx &U, 
     if (a.codes) note_code(a, U.g, U.up.region(region_word(e)), code, tier);
 }
 
-// High word of base + d * step (8.56 fixed point).
-__device__ __forceinline__ uint32_t fixed_hi(uint64_t base, uint64_t step, uint32_t d) {
-    return (uint32_t)((base + (uint64_t)d * (uint32_t)step) >> 32) + d * (uint32_t)(step >> 32);
-}
-// Its fraction in [0, 1), 23 bits.
-__device__ __forceinline__ float fixed_frac(uint32_t hi) {
-    return __fadd_rn(__uint_as_float(((hi >> 1) & 0x7FFFFFu) | 0x3F800000u), -1.0f);
-}
-// A coordinate of a table as 8.56 fixed point, rounded so that fixed_frac rounds to nearest.
-__device__ __forceinline__ uint64_t to_fixed(double v) {
-    return (uint64_t)((v - 256.0 * floor(v * (1.0 / 256.0))) * 72057594037927936.0) + (1ull << 32);
-}
-
 // One y = 0 sample of climate step k in FP32 from the table itself (perlin_y0_f32's operations
-// with the fixed-point coordinates: the fractions lie within u of the exact ones, G - 1 and L - 1
-// are exact, so a corner dot stays within 3 u and the bound above perlin_y0_f32 holds).
+// with the fixed-point coordinates: the fractions lie within u / 2 of the exact ones as there, so the
+// bound above perlin_y0_f32 holds).
 template <bool F32>
 __device__ __forceinline__ float unit_sample_f32(const UnitSmem<F32> &S, int k, uint32_t dx, uint32_t dz) {
     const uint8_t *P = S.tab + (kUClim + k) * kUPitch;
     const uint64_t step = S.c.fstep[k];
-    const uint32_t hx = fixed_hi(S.fx[k], step, dx), hz = fixed_hi(S.fz[k], step, dz);
-    const float g = fixed_frac(hx), l = fixed_frac(hz);
+    const uint64_t cx = fixed_at(S.fx[k], step, dx), cz = fixed_at(S.fz[k], step, dz);
+    const float g = fixed_frac(cx), l = fixed_frac(cz);
     const F2 gl = f2(g, l);
     float g1, l1;
     f2_split(f2_add(gl, f2(-1.0f, -1.0f)), g1, l1);
     const float hyf = S.hyf[k], hy1 = __fsub_rn(hyf, 1.0f), fyf = S.fyf[k];
-    const uint8_t *Pj = P + S.jy[k], *Pk = P + (hz >> 24);
-    const uint32_t i = hx >> 24;
+    const uint8_t *Pj = P + S.jy[k], *Pk = P + fixed_cell(cz);
+    const uint32_t i = fixed_cell(cx);
     const uint32_t a = P[i], b = P[i + 1];
     const uint32_t c = Pj[a], d = Pj[a + 1], e = Pj[b], f = Pj[b + 1];
     auto grad = [&](uint32_t hash, float x, float y, float z) {
@@ -224,14 +209,14 @@ __device__ __forceinline__ float unit_sample_f32(const UnitSmem<F32> &S, int k, 
 
 // The same sample from the block's lattice columns (table k < 4): corner values A x + B z + C, then
 // the x and z blends.  Bound, u = 2^-24: A, B, C within 1.5 u each (rounded weights, one rounded
-// sum, magnitude <= 1); fractions within u; two FMAs of values <= 2: corner 1.5 * 3 u + 2 u + 2 u = 8.5 u;
+// sum, magnitude <= 1); fractions, and those less 1, within u; two FMAs of values <= 2: corner 1.5 * 3 u + 2 u + 2 u = 8.5 u;
 // x blend 8.5 u + 4 * 4 u + 2 u = 26.5 u; z blend 26.5 u + 4 * 4 u + 2 u = 44.5 u, under kPerlinF32ErrUlps.
-__device__ __forceinline__ float lat_sample(const float4 *L, int nx, uint32_t hx, uint32_t hz) {
-    const float g = fixed_frac(hx), l = fixed_frac(hz);
+__device__ __forceinline__ float lat_sample(const float4 *L, int nx, uint64_t cx, uint64_t cz) {
+    const float g = fixed_frac(cx), l = fixed_frac(cz);
     const F2 gl = f2(g, l);
     float g1, l1;
     f2_split(f2_add(gl, f2(-1.0f, -1.0f)), g1, l1);
-    const float4 *p = L + (hz >> 24) * (uint32_t)nx + (hx >> 24);
+    const float4 *p = L + fixed_cell(cz) * (uint32_t)nx + fixed_cell(cx);
     const float4 q00 = p[0], q10 = p[1], q01 = p[nx], q11 = p[nx + 1];
     const float v00 = __fmaf_rn(q00.x, g, __fmaf_rn(q00.y, l, q00.z));
     const float v10 = __fmaf_rn(q10.x, g1, __fmaf_rn(q10.y, l, q10.z));
@@ -306,7 +291,7 @@ __device__ __forceinline__ bool unit_step(UnitSmem<F32> &S, const BatchArgs &a, 
         float v;
         if constexpr (LAT) {
             const uint64_t step = S.c.fstep[k];
-            v = lat_sample(S.lat.l1[k - 2], B->nx[k], fixed_hi(B->x[k], step, ex), fixed_hi(B->z[k], step, ez));
+            v = lat_sample(S.lat.l1[k - 2], B->nx[k], fixed_at(B->x[k], step, ex), fixed_at(B->z[k], step, ez));
         } else {
             v = unit_sample_f32(S, k, e & 0xFFFFu, e >> 16);
         }
@@ -676,7 +661,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
         const uint64_t step = S.c.fstep[k];
         const uint64_t b = (z ? S.fz[k] : S.fx[k]) + (uint64_t)(at * 32u) * step;
         const uint64_t b0 = b & 0x00FFFFFFFFFFFFFFull;
-        const int cols = (int)(fixed_hi(b0, step, (side - 1) * 32u + 23u) >> 24) + 2;
+        const int cols = (int)fixed_cell(fixed_at(b0, step, (side - 1) * 32u + 23u)) + 2;
         (z ? B.z : B.x)[k] = b0;
         (z ? B.cell_z : B.cell_x)[k] = (int)(b >> 56);
         (z ? B.nz : B.nx)[k] = cols;
@@ -738,9 +723,9 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                 if constexpr (F32) {
                     const uint64_t s0 = S.c.fstep[0], s1 = S.c.fstep[1];
                     sum = __fmul_rn(st.cf[0],
-                                    lat_sample(S.lat.l0[0], B.nx[0], fixed_hi(B.x[0], s0, ex), fixed_hi(B.z[0], s0, ez)));
+                                    lat_sample(S.lat.l0[0], B.nx[0], fixed_at(B.x[0], s0, ex), fixed_at(B.z[0], s0, ez)));
                     sum = __fmaf_rn(st.cf[1],
-                                    lat_sample(S.lat.l0[1], B.nx[1], fixed_hi(B.x[1], s1, ex), fixed_hi(B.z[1], s1, ez)),
+                                    lat_sample(S.lat.l0[1], B.nx[1], fixed_at(B.x[1], s1, ex), fixed_at(B.z[1], s1, ez)),
                                     sum);
                     pass = sum >= st.hi[1];
                     in_band = all_rechecks || (!pass && !(sum < st.lo[1]));
