@@ -41,8 +41,8 @@ Tiling wg::tile_rect(uint64_t rw, uint64_t rh, uint64_t target) {
     return t;
 }
 
-bool wg::few_units(uint64_t n_seeds, double n_regions, int sm_count, bool fp32) {
-    return (double)n_seeds <= (fp32 ? 9.0 + n_regions / 67.0 : 6.5 + n_regions / 138.0) * sm_count;
+bool wg::few_units(double n_units, double n_regions, int sm_count, bool fp32) {
+    return n_units <= (fp32 ? 9.0 + n_regions / 67.0 : 6.5 + n_regions / 138.0) * sm_count;
 }
 
 // Tiles of the one-CTA kernel that fill whole waves of its resident CTAs.  A wave lasts as long as its tiles'
@@ -84,13 +84,17 @@ static Tiling wave_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, uint64_t sl
 // Whether a request's units take the one-CTA kernel, and its tiles.  Many regions per seed: yes, a
 // tile's two table builds (13,000 warp instructions) are then a small part of it, and the ladder and
 // the entrance gate find the seed's tables built.  Few units (few_units): yes too, in tiles small
-// enough to give every one of the sm_count * 3 resident CTAs one, since the call then takes one build
+// enough to give every one of the resident CTAs one, since the call then takes one build
 // and one evaluation of latency instead of three.  Otherwise 16 units share a CTA.
-static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, const wg_engine *eng, bool single_biome, bool &cta) {
-    const uint64_t n_regions = rw * rh, slots = (uint64_t)eng->sm_count * 3;
-    cta = !single_biome && (n_regions >= kUnitCtaRegions || few_units(n_seeds, (double)n_regions, eng->sm_count, eng->fp32_core != 0));
+static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, const wg_engine *eng, bool single_biome, bool f32, bool &cta) {
+    const uint64_t n_regions = rw * rh, slots = (uint64_t)eng->sm_count * (uint64_t)eng->unit_per_sm[f32 ? 1 : 0];
     const uint64_t across = std::min(rw, rh);
-    if (across < kUnitCtaStrip) cta = cta && (double)n_seeds * std::ceil((double)std::max(rw, rh) / 1023.0) <= 4.0 * (double)slots;
+    const bool strip = across < kUnitCtaStrip;
+    const Tiling large = tile_rect(rw, rh, kUnitCtaMax);   // FP64 units that are not whole seeds count as its tiles
+    const bool few = f32 || n_regions <= 4096 ? few_units((double)n_seeds, (double)n_regions, eng->sm_count, f32)
+                                              : few_units((double)n_seeds * (double)large.n_win, (double)large.win(), eng->sm_count, f32);
+    cta = !single_biome && (few || (strip ? n_regions >= kUnitCtaRegions : unit_rect(rw, rh, f32)));
+    if (strip) cta = cta && (double)n_seeds * std::ceil((double)std::max(rw, rh) / 1023.0) <= 4.0 * (double)slots;
     if (!cta) return tile_rect(rw, rh, n_regions <= 4096 ? n_regions : 2048);
     return wave_tiles(rw, rh, n_seeds, slots);
 }
@@ -401,8 +405,11 @@ int run_request(wg_engine *eng, const Request &rq, Sink &sink, wg_scan_stats &st
     const uint64_t rw = (uint64_t)((int64_t)rq.rx1 - rq.rx0), rh = (uint64_t)((int64_t)rq.rz1 - rq.rz0);
     const uint64_t n_regions = rw * rh;
     const bool spot = spot_path(false, n_regions, rq.d_codes != nullptr, rq.opts.single_biome != 0);
+    // spots shift the rect by their own regions: only plain requests are proved small
+    const bool small = !rq.d_spot_s48 && coords_small(std::min(rq.rx0, rq.rz0), std::max(rq.rx1, rq.rz1) - 1ll);
     bool cta = false;
-    const Tiling tiles = spot ? tile_rect(rw, rh, 1) : request_tiles(rw, rh, rq.n_seeds, eng, rq.opts.single_biome != 0, cta);
+    const Tiling tiles = spot ? tile_rect(rw, rh, 1)
+                              : request_tiles(rw, rh, rq.n_seeds, eng, rq.opts.single_biome != 0, eng->fp32_core && small, cta);
     const uint64_t n_win = tiles.n_win, win = tiles.win();
     const uint64_t units = rq.n_seeds * n_win;
 
@@ -425,8 +432,7 @@ int run_request(wg_engine *eng, const Request &rq, Sink &sink, wg_scan_stats &st
     a.spot_s48 = rq.d_spot_s48;
     a.spot_rx = rq.d_spot_rx;
     a.spot_rz = rq.d_spot_rz;
-    // spots shift the rect by their own regions: only plain requests are proved small
-    a.small_coords = !rq.d_spot_s48 && coords_small(std::min(rq.rx0, rq.rz0), std::max(rq.rx1, rq.rz1) - 1ll) ? 1 : 0;
+    a.small_coords = small ? 1 : 0;
 
     // the one-CTA kernel keeps no work lists in HBM, so its batches are eight times as large
     uint64_t per_batch = std::min<uint64_t>(kMaxUnits, std::max<uint64_t>(32, kWorkPerBatch * (cta ? 8 : 1) / win));
@@ -573,6 +579,8 @@ int wg_engine_open(int device, wg_engine **out) {
         for (int k = 0; k < 4; k++) WG_CUDA(cudaEventCreate(&eng->kev[k]), "event");
         upload_phase1_tables();
         WG_CUDA(cudaGetLastError(), "upload tables");
+        for (int f32 = 0; f32 < 2; f32++) eng->unit_per_sm[f32] = unit_ctas_per_sm(f32 != 0);
+        WG_CUDA(cudaGetLastError(), "unit kernel");
         WG_CUDA(cudaMalloc(&eng->rec_unit, sizeof(uint32_t) * kCapRec), "alloc");
         WG_CUDA(cudaMalloc(&eng->rec_off, sizeof(uint32_t) * kCapRec), "alloc");
         WG_CUDA(cudaMalloc(&eng->rec_cnt, sizeof(uint32_t) * kCapRec), "alloc");

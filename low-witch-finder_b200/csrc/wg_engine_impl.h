@@ -22,6 +22,7 @@ struct QueueRes;
 struct wg_engine {
     int device = 0;
     int sm_count = 148;
+    int unit_per_sm[2] = {1, 1};   // unit_ctas_per_sm of the FP64 and the FP32 instance
     int fp32_core = 1;   // 1 FP32 core with FP64 rechecks, 3 also the cave samples, 0 FP64, 2 as 3 re-taking every gate
     int job_queue = 1;   // wg_seed_check_jobs through the device work queue (1) or the host batch loop (0)
     // autotuned job settings (wg_engine_tune): regions per unit per job class (0 = window_for's
@@ -140,18 +141,31 @@ Tiling tile_rect(uint64_t rw, uint64_t rh, uint64_t target);
 // Regions per seed from which a unit takes the one-CTA kernel (launch_unit) however many seeds there
 // are: 8,192 seeds x 2,025 regions take it 1.73 ms and the list kernels 1.41; 3,552 x 4,096 1.07 and 1.99.
 constexpr uint64_t kUnitCtaRegions = 3072;
+// The same for its FP64 instance, whose regions take twice as long: a rect of at most 4,096 regions, which the
+// fused kernels walk as one unit (18,000 seeds x 3,249 regions 5.93 ms and 5.41 fused, x 3,364 5.83 and 5.59,
+// 16,666 x 3,600 5.67 and 5.92, 14,648 x 4,096 5.11 and 6.25), and the regions per tile of a larger one (6e7
+// regions in all, rects of tiles of 2,732 regions 6.83 and 5.11, 4,000 5.89 and 5.10, 4,098 5.59 and 5.11, 4,225
+// 5.44 and 6.19, 4,500 5.32 and 5.53, 5,000 4.95 and 5.10, 16,384 4.1 and 6.0).
+constexpr uint64_t kUnitCtaRegions64 = 3600, kUnitCtaTile64 = 4200;
 // A strip of fewer regions across than this makes tiles of few regions (a tile is at most 1,023 long), so it
 // takes the one-CTA kernel only for a few waves of them: 1,000 seeds x 20,000 x 1 3.11 ms and 1.66 fused, x
 // 10,000 x 3 2.44 and 2.36, x 10,000 x 4 2.88 and 2.97; one seed x 1,000,000 x 1 0.21 and 0.54.
 constexpr uint64_t kUnitCtaStrip = 4;
-// Whether so few units are better off with one CTA each (a wave of sm_count * 3 CTAs takes 40 to 120 us,
+// Whether so few units are better off with one CTA each (a wave of resident CTAs, 3 an SM, takes 40 to 120 us,
 // the fused kernels 125 to 450 whatever the number): 64 regions, 1,332 seeds 129 us and 129 fused, 1,776 148
 // and 136; 400 regions, 1,776 seeds 209 and 216, 2,664 286 and 271; 1,600 regions, 2,664 seeds 496 and 626,
 // 5,328 925 and 960.  FP64 units take longer: 64 regions, 888 seeds 107 and 131, 1,332 157 and 129; 400
 // regions, 1,332 seeds 217 and 217; 1,600 regions, 2,664 seeds 711 and 713, 3,552 916 and 780.
-bool few_units(uint64_t n_seeds, double n_regions, int sm_count, bool fp32);
+bool few_units(double n_units, double n_regions, int sm_count, bool fp32);
 // Regions per unit of the one-CTA kernel at most.
 constexpr uint64_t kUnitCtaMax = 1ull << 16;
+// Whether seeds of a rw x rh rect take the one-CTA kernel however many they are (rects kUnitCtaStrip across
+// and more); f32: its FP32 instance.
+inline bool unit_rect(uint64_t rw, uint64_t rh, bool f32) {
+    const uint64_t n = rw * rh;
+    if (f32) return n >= kUnitCtaRegions;
+    return n <= 4096 ? n >= kUnitCtaRegions64 : tile_rect(rw, rh, kUnitCtaMax).win() >= kUnitCtaTile64;
+}
 
 // Job classes of the autotuner by regions per seed: <= 16, <= 256, <= 4096, more.
 constexpr uint64_t kJobClassMax[4] = {16, 256, 4096, ~0ull};

@@ -40,9 +40,9 @@ bool candidate_order(const Candidate &x, const Candidate &y) {
     return x.rx < y.rx;
 }
 
-// Whether a batch of so few units takes the one-CTA kernel.
-bool small_batch(const wg_engine *eng, const SchedJob &lead, uint64_t units, uint64_t work) {
-    return !lead.opts.single_biome && few_units(units, (double)work / (double)units, eng->sm_count, eng->fp32_core != 0);
+// Whether a batch of so few units takes the one-CTA kernel; f32: its FP32 instance.
+bool small_batch(const wg_engine *eng, const SchedJob &lead, uint64_t units, uint64_t work, bool f32) {
+    return !lead.opts.single_biome && few_units((double)units, (double)work / (double)units, eng->sm_count, f32);
 }
 
 // Whether a job's climate coordinates are proved inside maintainPrecision's identity range.
@@ -65,7 +65,8 @@ int sched_job_init(SchedJob &j, const wg_job &spec, const wg_engine *eng) {
     j.rw = (int)rw;
     j.rh = (int)rh;
     j.n_regions = rw * rh;
-    j.unit_cta = j.n_regions >= kUnitCtaRegions && std::min(rw, rh) >= kUnitCtaStrip && !spec.opts.single_biome;
+    j.unit_cta = std::min(rw, rh) >= kUnitCtaStrip && !spec.opts.single_biome &&
+                 unit_rect(rw, rh, (!eng || eng->fp32_core) && job_small(j));
     j.tiles = tile_rect(rw, rh, std::min<uint64_t>(job_window(eng, j.n_regions), j.unit_cta ? kUnitCtaMax : 4096));
     if (spec.n_seeds > ~0ull / j.tiles.n_win) return WG_ERR_ARG;
     j.units = spec.n_seeds * j.tiles.n_win;
@@ -257,9 +258,9 @@ int Scheduler::step(std::vector<SchedJob *> &finished, std::vector<SchedJob *> &
     a.seeds = d_arena_;
     a.jobs = d_table_;
     a.n_jobs = (uint32_t)table.size();
-    a.unit_cta = lead.unit_cta || small_batch(eng_, lead, units, step_work_ - budget) ? 1 : 0;
     a.small_coords = 1;
     for (const SchedJob *j : members) a.small_coords &= job_small(*j) ? 1 : 0;
+    a.unit_cta = lead.unit_cta || small_batch(eng_, lead, units, step_work_ - budget, a.fp32_core && a.small_coords) ? 1 : 0;
     found_.clear();
     Sink sink;
     sink.host = &found_;
@@ -390,9 +391,9 @@ int jobs_on_device_queue(wg_engine *eng, std::vector<SchedJob> &js, uint64_t tot
             a.seeds = d_seeds;
             a.jobs = d_table;
             a.n_jobs = (uint32_t)table.size();
-            a.unit_cta = js[lead].unit_cta || small_batch(eng, js[lead], units, work) ? 1 : 0;
             a.small_coords = 1;
             for (size_t k : member) a.small_coords &= job_small(js[k]) ? 1 : 0;
+            a.unit_cta = js[lead].unit_cta || small_batch(eng, js[lead], units, work, a.fp32_core && a.small_coords) ? 1 : 0;
             std::vector<Candidate> found;
             const uint64_t slice = js[lead].opts.single_biome ? std::min<uint64_t>(budget, kCapSurv / 2) : budget;
             int r = run_queue(eng, a, units, max_units, slice, found, st);

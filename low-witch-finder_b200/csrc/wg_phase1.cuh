@@ -229,6 +229,8 @@ void launch_ladder(const BatchArgs &a, int grid, cudaStream_t s);
 void launch_lists(const BatchArgs &a, cudaStream_t s);
 // All of phase 1, one CTA per unit; deep candidates past a CTA's own list go to the ladder kernel's.
 void launch_unit(const BatchArgs &a, cudaStream_t s);
+// CTAs of launch_unit's kernel that an SM of the current device holds at once (f32: its FP32 instance).
+int unit_ctas_per_sm(bool f32);
 // Sets the kernels' shared-memory limits and the ladder's resident-block count on the current
 // device, so that the launch functions make no further runtime calls (a stream capture may follow).
 void prepare_phase1_launches();

@@ -126,22 +126,34 @@ __host__ __device__ constexpr uint32_t block_side(uint32_t other) {
     return t > (uint32_t)kBlock ? t : kBlock;
 }
 
+// What only the FP32 instance keeps: the climate tables' fixed-point constants, the lattice columns and
+// where they lie.
 template <bool F32>
-struct UnitSmem {
+struct UnitFixed {
+    uint64_t fx[kSlotsA], fz[kSlotsA];
+    float hyf[kSlotsA], fyf[kSlotsA];
+    float w0[kLatTables], w1[kLatTables], c0[kLatTables], c1[kLatTables];
+    LatBase lat_base[2];                       // this block's and the next one's
+};
+template <>
+struct UnitFixed<false> {};
+template <bool F32>
+struct UnitLattice {
+    float4 l0[2][kLat0 * kLat0];
+    float4 l1[2][kLat1 * kLat1];
+};
+template <>
+struct UnitLattice<false> {};
+
+template <bool F32>
+struct UnitSmem : UnitFixed<F32> {
     using Real = typename std::conditional<F32, float, double>::type;
     uint8_t tab[kUTabs * kUPitch];
     double org[3 * kUTabs];                    // cave tables' origins [slot][3]
     double cox[kSlotsA], coz[kSlotsA], chy[kSlotsA];   // climate tables, step order
-    uint64_t fx[kSlotsA], fz[kSlotsA];
-    float hyf[kSlotsA], fyf[kSlotsA];
-    float w0[kLatTables], w1[kLatTables], c0[kLatTables], c1[kLatTables];
     int jy[kSlotsA];
-    LatBase lat_base[2];                       // this block's and the next one's
     union {
-        struct {
-            float4 l0[2][kLat0 * kLat0];
-            float4 l1[2][kLat1 * kLat1];
-        } lat;
+        UnitLattice<F32> lat;
         double mh[kUWarps][2 * kSlotsB];       // a warp's survivor at 50 and 60, or candidate at maxHeight
         LadderVals lad;
     };
@@ -628,17 +640,19 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
             S.coz[lane] = oz;
             S.chy[lane] = hy;
             S.jy[lane] = jy;
-            S.hyf[lane] = __double2float_rn(hy);
-            S.fyf[lane] = __double2float_rn(fy);
-            const double sc = S.c.steps.sc[lane], lac = S.c.steps.lac[lane];
-            const double xc = (U.ucx * 16 + 8) * 0.25, zc = (U.ucz * 16 + 8) * 0.25;
-            S.fx[lane] = to_fixed(keep_precision((xc * sc) * lac) + ox);
-            S.fz[lane] = to_fixed(keep_precision((zc * sc) * lac) + oz);
-            if (lane < kLatTables) {
-                S.w0[lane] = __double2float_rn(1.0 - fy);
-                S.w1[lane] = __double2float_rn(fy);
-                S.c0[lane] = __double2float_rn((1.0 - fy) * hy);
-                S.c1[lane] = __double2float_rn(fy * (hy - 1.0));
+            if constexpr (F32) {
+                S.hyf[lane] = __double2float_rn(hy);
+                S.fyf[lane] = __double2float_rn(fy);
+                const double sc = S.c.steps.sc[lane], lac = S.c.steps.lac[lane];
+                const double xc = (U.ucx * 16 + 8) * 0.25, zc = (U.ucz * 16 + 8) * 0.25;
+                S.fx[lane] = to_fixed(keep_precision((xc * sc) * lac) + ox);
+                S.fz[lane] = to_fixed(keep_precision((zc * sc) * lac) + oz);
+                if (lane < kLatTables) {
+                    S.w0[lane] = __double2float_rn(1.0 - fy);
+                    S.w1[lane] = __double2float_rn(fy);
+                    S.c0[lane] = __double2float_rn((1.0 - fy) * hy);
+                    S.c1[lane] = __double2float_rn(fy * (hy - 1.0));
+                }
             }
         } else {
             S.org[3 * lane] = ox;
@@ -652,22 +666,24 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
     const uint32_t bw = (U.up.tw + nbx - 1) / nbx, bh = (U.up.th + nbz - 1) / nbz;
     const uint32_t n_blocks = nbx * nbz;
     auto lattice_base = [&](uint32_t blk) {   // one thread per table and axis, a block ahead of its use
-        if (tid >= 2 * kLatTables || blk >= n_blocks) return;
-        LatBase &B = S.lat_base[blk & 1u];
-        const int k = tid >> 1;
-        const bool z = tid & 1;
-        const uint32_t at = z ? (blk / nbx) * bh : (blk % nbx) * bw;   // first region of the block, in the unit
-        const uint32_t side = z ? min(bh, U.up.th - at) : min(bw, U.up.tw - at);
-        const uint64_t step = S.c.fstep[k];
-        const uint64_t b = (z ? S.fz[k] : S.fx[k]) + (uint64_t)(at * 32u) * step;
-        const uint64_t b0 = b & 0x00FFFFFFFFFFFFFFull;
-        const int cols = (int)fixed_cell(fixed_at(b0, step, (side - 1) * 32u + 23u)) + 2;
-        (z ? B.z : B.x)[k] = b0;
-        (z ? B.cell_z : B.cell_x)[k] = (int)(b >> 56);
-        (z ? B.nz : B.nx)[k] = cols;
-        if (!z) B.inv[k] = ((1u << 20) + (uint32_t)cols - 1) / (uint32_t)cols;
+        if constexpr (F32) {
+            if (tid >= 2 * kLatTables || blk >= n_blocks) return;
+            LatBase &B = S.lat_base[blk & 1u];
+            const int k = tid >> 1;
+            const bool z = tid & 1;
+            const uint32_t at = z ? (blk / nbx) * bh : (blk % nbx) * bw;   // first region of the block, in the unit
+            const uint32_t side = z ? min(bh, U.up.th - at) : min(bw, U.up.tw - at);
+            const uint64_t step = S.c.fstep[k];
+            const uint64_t b = (z ? S.fz[k] : S.fx[k]) + (uint64_t)(at * 32u) * step;
+            const uint64_t b0 = b & 0x00FFFFFFFFFFFFFFull;
+            const int cols = (int)fixed_cell(fixed_at(b0, step, (side - 1) * 32u + 23u)) + 2;
+            (z ? B.z : B.x)[k] = b0;
+            (z ? B.cell_z : B.cell_x)[k] = (int)(b >> 56);
+            (z ? B.nz : B.nx)[k] = cols;
+            if (!z) B.inv[k] = ((1u << 20) + (uint32_t)cols - 1) / (uint32_t)cols;
+        }
     };
-    if constexpr (F32) lattice_base(0);
+    lattice_base(0);
     unit_double_tables(S.tab, 0, kSlotsB + kSlotsA);
     __syncthreads();
 
@@ -676,9 +692,10 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
     for (uint32_t blk = 0; blk < n_blocks; blk++) {
         const uint32_t x0 = (blk % nbx) * bw, z0 = (blk / nbx) * bh;   // first region of the block, in the unit
         const uint32_t w = min(bw, U.up.tw - x0), h = min(bh, U.up.th - z0), n = w * h;
-        const LatBase &B = S.lat_base[blk & 1u];
+        const LatBase *Bp = nullptr;
         if constexpr (F32) {
             // ---- the block's lattice columns ----
+            const LatBase &B = *(Bp = &S.lat_base[blk & 1u]);
             lattice_base(blk + 1);   // into the other half, which no thread reads before the next block
             const int m0 = B.nx[0] * B.nz[0], m1 = m0 + B.nx[1] * B.nz[1], m2 = m1 + B.nx[2] * B.nz[2],
                       m3 = m2 + B.nx[3] * B.nz[3];
@@ -721,6 +738,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                 e = (x0 * 32u + ex) | ((z0 * 32u + ez) << 16);
                 bool in_band = true;
                 if constexpr (F32) {
+                    const LatBase &B = *Bp;
                     const uint64_t s0 = S.c.fstep[0], s1 = S.c.fstep[1];
                     sum = __fmul_rn(st.cf[0],
                                     lat_sample(S.lat.l0[0], B.nx[0], fixed_at(B.x[0], s0, ex), fixed_at(B.z[0], s0, ez)));
@@ -764,7 +782,7 @@ __global__ void __launch_bounds__(kUThreads, 3) unit_kernel(const __grid_constan
                 Real sum = 0;
                 if (q < n1) {
                     e = S.wl[warp][q];
-                    keep = unit_step<F32, F32>(S, a, U, W, k, all_rechecks, e, &B, (e & 0xFFFFu) - x0 * 32u,
+                    keep = unit_step<F32, F32>(S, a, U, W, k, all_rechecks, e, Bp, (e & 0xFFFFu) - x0 * 32u,
                                                (e >> 16) - z0 * 32u, S.ws[warp][q], sum);
                 }
                 const unsigned m = __ballot_sync(0xFFFFFFFFu, keep);
@@ -964,6 +982,14 @@ static unsigned long long g_smem_done_u32 = 0, g_smem_done_u64 = 0;
 static void prepare_unit_launches() {
     allow_dynamic_smem(unit_kernel<true>, sizeof(UnitSmem<true>), g_smem_done_u32);
     allow_dynamic_smem(unit_kernel<false>, sizeof(UnitSmem<false>), g_smem_done_u64);
+}
+
+int unit_ctas_per_sm(bool f32) {
+    prepare_unit_launches();
+    int n = 0;
+    if (f32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, unit_kernel<true>, kUThreads, sizeof(UnitSmem<true>));
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, unit_kernel<false>, kUThreads, sizeof(UnitSmem<false>));
+    return n < 1 ? 1 : n;
 }
 
 void launch_unit(const BatchArgs &a, cudaStream_t s) {

@@ -119,3 +119,22 @@ def test_check_mode_takes_every_gate_again(engine, rect):
     left -= tier[-1]
     want += left + (left - st["reject_hist"][1]) + st["climate_survivors"]
     assert st["rechecks"] == want
+
+
+@pytest.mark.parametrize("n,rect,unit", [(400, (0, 56, 0, 56), True), (6000, (0, 56, 0, 56), False),
+                                         (5000, (-30, 30, -30, 30), True), (200, (-2000, 2000, 0, 4), True),
+                                         (1500, (-2000, 2000, 0, 4), False), (600, (-80, 80, -80, 80), True)])
+def test_fp64_routes_equal_the_fp32_core(engine, n, rect, unit):
+    """The FP64 core on both sides of its rules for the unit kernel (regions of a seed or of a tile, few units)
+    against the FP32 core, whose unit kernel takes all of these."""
+    a = engine.seed_check(gen=(n, n), rect=rect, max_height=40)
+    engine.set_noise_core("fp64")
+    try:
+        b = engine.seed_check(gen=(n, n), rect=rect, max_height=40)
+    finally:
+        engine.set_noise_core("fp32")
+    assert a.stats["kernel_launches"][1] == 0
+    assert (b.stats["kernel_launches"][1] == 0) == unit
+    assert len(a.candidates) and np.array_equal(a.candidates, b.candidates)
+    assert a.stats["reject_hist"] == b.stats["reject_hist"]
+    assert a.stats["tier_hist"] == b.stats["tier_hist"]
