@@ -21,64 +21,8 @@
 
 using namespace wg;
 
-Tiling wg::tile_rect(uint64_t rw, uint64_t rh, uint64_t target) {
-    constexpr uint64_t kMaxSide = 1023;   // a hut's chunk offset in its tile stays below 2^15
-    target = std::max<uint64_t>(target, 1);
-    uint64_t tw = rw, th = rh;
-    if (rw > target / rh || rw > kMaxSide || rh > kMaxSide) {
-        const uint64_t side = std::max<uint64_t>(1, (uint64_t)std::sqrt((double)target));
-        tw = std::min<uint64_t>({rw, side, kMaxSide});
-        th = std::min<uint64_t>({rh, std::max<uint64_t>(1, target / tw), kMaxSide});
-        tw = std::min<uint64_t>({rw, std::max<uint64_t>(1, target / th), kMaxSide});   // a low rect: wider tiles
-        tw = (rw + (rw + tw - 1) / tw - 1) / ((rw + tw - 1) / tw);                     // of equal size
-        th = (rh + (rh + th - 1) / th - 1) / ((rh + th - 1) / th);
-    }
-    Tiling t;
-    t.tw = (uint32_t)tw;
-    t.th = (uint32_t)th;
-    t.ntx = (uint32_t)((rw + tw - 1) / tw);
-    t.n_win = t.ntx * ((rh + th - 1) / th);
-    return t;
-}
-
 bool wg::few_units(double n_units, double n_regions, int sm_count, bool fp32) {
     return n_units <= (fp32 ? 9.0 + n_regions / 67.0 : 6.5 + n_regions / 138.0) * sm_count;
-}
-
-// Tiles of the one-CTA kernel that fill whole waves of its resident CTAs.  A wave lasts as long as its tiles'
-// regions and about 2,000 more (the table builds, the last gates), and a part of a wave, whose CTAs have the
-// SM to themselves, not as long.  The tilings of one to four waves are compared by that.  Against tiles of an
-// eighth of a slot's share (2,048 regions at least), one seed: 400 x 400 regions 100 -> 88 us, 2000 x 2000
-// 429 -> 249 us (3 units a slot, then 1), 6000 x 6000 1.87 -> 1.44 ms; 40 seeds x 600 x 600 1.01 -> 0.59 ms.
-// Requests past four waves of the largest tiles take those, and those of more seeds than four waves one a seed.
-static Tiling wave_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, uint64_t slots) {
-    constexpr uint64_t kWaveRegions = 2000, kMaxSide = 1023;
-    uint64_t best = ~0ull, btw = 0, bth = 0;
-    for (uint64_t waves = 1; waves <= 4; waves++) {
-        const uint64_t m = std::min(waves * slots / n_seeds, (rw * rh + 31) / 32);   // tiles per seed
-        if (m == 0) continue;
-        const double square = std::sqrt((double)m * (double)rw / (double)rh);
-        const uint64_t lo = std::max<uint64_t>(1, (uint64_t)(square * 0.6)), hi = std::min<uint64_t>({rw, m, (uint64_t)(square * 1.7) + 1});
-        for (uint64_t nx = lo; nx <= hi; nx++) {
-            const uint64_t tw = (rw + nx - 1) / nx, nz = std::min(rh, m / ((rw + tw - 1) / tw)), th = (rh + nz - 1) / nz;
-            if (tw > kMaxSide || th > kMaxSide || tw * th > kUnitCtaMax) continue;
-            const uint64_t units = n_seeds * ((rw + tw - 1) / tw) * ((rh + th - 1) / th), part = units % slots;
-            const uint64_t cost = (units / slots) * (tw * th + kWaveRegions) +
-                                  (part ? kWaveRegions + tw * th * (2 * slots + 3 * part) / (5 * slots) : 0);
-            if (cost < best) {
-                best = cost;
-                btw = tw;
-                bth = th;
-            }
-        }
-    }
-    if (best == ~0ull) return tile_rect(rw, rh, kUnitCtaMax);
-    Tiling t;
-    t.tw = (uint32_t)btw;
-    t.th = (uint32_t)bth;
-    t.ntx = (uint32_t)((rw + btw - 1) / btw);
-    t.n_win = t.ntx * ((rh + bth - 1) / bth);
-    return t;
 }
 
 // Whether a request's units take the one-CTA kernel, and its tiles.  Many regions per seed: yes, a
@@ -95,8 +39,12 @@ static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, const wg
                                               : few_units((double)n_seeds * (double)large.n_win, (double)large.win(), eng->sm_count, f32);
     cta = !single_biome && (few || (strip ? n_regions >= kUnitCtaRegions : unit_rect(rw, rh, f32)));
     if (strip) cta = cta && (double)n_seeds * std::ceil((double)std::max(rw, rh) / 1023.0) <= 4.0 * (double)slots;
-    if (!cta) return tile_rect(rw, rh, n_regions <= 4096 ? n_regions : 2048);
-    return wave_tiles(rw, rh, n_seeds, slots);
+    // Long strips of one or two regions stay with the fused kernels, whose tiles may be longer: fewer table builds,
+    // if there are units enough for six waves of those kernels all the same (10,000 x 1, tiles of 1,000 and of
+    // 2,000 regions: 500 seeds 0.63 and 0.73 ms, 2,000 1.67 and 1.72, 3,000 2.37 and 2.36, 12,000 8.85 and 8.25).
+    if (cta) return wave_tiles(rw, rh, n_seeds, slots);
+    const bool many = (double)n_seeds * (double)n_regions >= 2048.0 * 100.0 * eng->sm_count;
+    return tile_rect(rw, rh, n_regions <= 4096 ? n_regions : 2048, across <= 2 && many ? 4096 : kTileSide);
 }
 
 // Climate evaluation steps (see ClimateStep): the tiered erosion sequence

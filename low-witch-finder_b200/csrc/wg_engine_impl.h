@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/witchgpu.h"
+#include "wg_tiling.h"
 #include "wg_phase1.cuh"
 
 namespace wg {
@@ -129,15 +130,6 @@ inline bool spot_path(bool jobs, uint64_t win, bool codes, bool single_biome) {
     return !jobs && win == 1 && !codes && !single_biome;
 }
 
-// How a rect is cut into units (tiles of regions, wg_phase1.cuh).
-struct Tiling {
-    uint32_t tw = 1, th = 1, ntx = 1;
-    uint64_t n_win = 1;           // tiles per seed
-    uint64_t win() const { return (uint64_t)tw * th; }   // regions per tile at most
-};
-// Tiles of at most `target` regions (at least one), near square, of equal size up to rounding.
-Tiling tile_rect(uint64_t rw, uint64_t rh, uint64_t target);
-
 // Regions per seed from which a unit takes the one-CTA kernel (launch_unit) however many seeds there
 // are: 8,192 seeds x 2,025 regions take it 1.73 ms and the list kernels 1.41; 3,552 x 4,096 1.07 and 1.99.
 constexpr uint64_t kUnitCtaRegions = 3072;
@@ -157,8 +149,6 @@ constexpr uint64_t kUnitCtaStrip = 4;
 // 5,328 925 and 960.  FP64 units take longer: 64 regions, 888 seeds 107 and 131, 1,332 157 and 129; 400
 // regions, 1,332 seeds 217 and 217; 1,600 regions, 2,664 seeds 711 and 713, 3,552 916 and 780.
 bool few_units(double n_units, double n_regions, int sm_count, bool fp32);
-// Regions per unit of the one-CTA kernel at most.
-constexpr uint64_t kUnitCtaMax = 1ull << 16;
 // Whether seeds of a rw x rh rect take the one-CTA kernel however many they are (rects kUnitCtaStrip across
 // and more); f32: its FP32 instance.
 inline bool unit_rect(uint64_t rw, uint64_t rh, bool f32) {
@@ -213,6 +203,7 @@ constexpr uint32_t kListUnits = 24576;
 // 600,000 seeds x 200 x 1 13.8 ms and 14.9 fused, x 100 x 2 13.2 and 14.7; 60,000 x 1,000 x 1 5.17 and 4.58, x
 // 1,000 x 2 8.84 and 8.24.
 constexpr uint32_t kListStrip = 500;
+static_assert(kListStrip < kTileSide, "only strips that stay out of the list kernels have longer tiles");
 // The same for the cave gate of one-region units, 1.7 % of which reach it.
 constexpr uint32_t kSpotListUnits = 1u << 19;
 constexpr int kListKernels = 6;   // launches of launch_lists
