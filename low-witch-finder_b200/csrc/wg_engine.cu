@@ -165,12 +165,12 @@ int run_batch(wg_engine *eng, const BatchArgs &proto, uint64_t unit0, uint32_t n
     a.unit0 = unit0;
     a.n_units = n_units;
     const bool spots = !a.unit_cta && spot_path(a.jobs != nullptr, (uint64_t)a.tw * a.th, a.codes != nullptr, a.single_biome != 0);
-    const bool lists = !spots && list_path(a, n_units);
+    bool lists = !spots && list_path(a, n_units);
     // one-region units: their climate stage is its own, the cave gate's list kernels from kSpotListUnits on
     const bool spot_lists = spots && a.fp32_core == 1 && n_units >= kSpotListUnits;
-    if (lists || spot_lists) {
-        int rc = list_buffers(eng);
-        if (rc) return rc;
+    if ((lists || spot_lists) && !list_buffers(eng)) {
+        lists = false;   // no memory for the lists: the fused kernels and the entrance kernel, which need none
+    } else if (lists || spot_lists) {
         a.lists[0] = eng->lists[0];
         a.lists[1] = eng->lists[1];
         if (spot_lists) a.lists[0].cnt = CNT_CLIMATE_LIST;
@@ -329,10 +329,14 @@ int copy_result(wg_engine *eng, void *dst, const void *src, size_t bytes) {
     return WG_OK;
 }
 
-int list_buffers(wg_engine *eng) {
-    if (eng->list_block) return WG_OK;
+bool list_buffers(wg_engine *eng) {
+    if (eng->list_block) return true;
     const size_t rec = sizeof(uint32_t) * kCapRec, reg = sizeof(uint32_t) * kCapSurv, one = 3 * rec + 3 * reg;
-    WG_CUDA(cudaMalloc(&eng->list_block, 2 * one), "alloc lists");
+    if (cudaMalloc(&eng->list_block, 2 * one) != cudaSuccess) {
+        cudaGetLastError();   // the caller does without them; the next batch asks again
+        eng->list_block = nullptr;
+        return false;
+    }
     for (int k = 0; k < 2; k++) {
         char *p = static_cast<char *>(eng->list_block) + k * one;
         RegionList &L = eng->lists[k];
@@ -345,7 +349,7 @@ int list_buffers(wg_engine *eng) {
         L.cap_surv = kCapSurv;
         L.cnt = 0;
     }
-    return WG_OK;
+    return true;
 }
 
 int run_request(wg_engine *eng, const Request &rq, Sink &sink, wg_scan_stats &st) {

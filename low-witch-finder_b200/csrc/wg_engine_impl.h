@@ -207,8 +207,8 @@ static_assert(kListStrip < kTileSide, "only strips that stay out of the list ker
 // The same for the cave gate of one-region units, 1.7 % of which reach it.
 constexpr uint32_t kSpotListUnits = 1u << 19;
 constexpr int kListKernels = 6;   // launches of launch_lists
-// Allocates the list kernels' lists once per engine.
-int list_buffers(wg_engine *eng);
+// Allocates the list kernels' lists (228 MB) once per engine; false where there is no memory for them.
+bool list_buffers(wg_engine *eng);
 // Whether a batch of n_units units takes the list kernels.
 inline bool list_path(const BatchArgs &a, uint32_t n_units) {
     const bool strip = !a.jobs && std::min(a.tw, a.th) <= 2 && std::max(a.tw, a.th) > kListStrip;

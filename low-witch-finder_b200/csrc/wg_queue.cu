@@ -167,10 +167,8 @@ int run_queue(wg_engine *eng, const BatchArgs &proto, uint64_t total_units, uint
     a.unit0 = 0;
     a.n_units = max_units;   // the launch geometry; the slice range comes from dyn
     a.dyn = R.q->dyn;
-    const bool lists = list_path(a, max_units);
+    const bool lists = list_path(a, max_units) && list_buffers(eng);
     if (lists) {
-        int rc = list_buffers(eng);
-        if (rc) return rc;
         a.lists[0] = eng->lists[0];
         a.lists[1] = eng->lists[1];
     }

@@ -138,3 +138,25 @@ def test_fp64_routes_equal_the_fp32_core(engine, n, rect, unit):
     assert len(a.candidates) and np.array_equal(a.candidates, b.candidates)
     assert a.stats["reject_hist"] == b.stats["reject_hist"]
     assert a.stats["tier_hist"] == b.stats["tier_hist"]
+
+
+def test_no_memory_for_the_lists(wg, engine):
+    """A call that would take the list kernels, with less device memory free than their lists need (228 MB):
+    the fused kernels serve it, with the same survivors and funnel."""
+    import torch
+    want = engine.seed_check(gen=(5, 24576), rect=(-4, 5, -4, 5), max_height=40)
+    assert want.stats["kernel_launches"][0] == 6 * want.stats["batches"]
+    with wg.Engine(0) as e:
+        e.seed_check(gen=(1, 20000), rect=(-4, 5, -4, 5), max_height=40)   # its kernels are loaded
+        torch.cuda.synchronize()
+        full = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (160 << 20)), dtype=torch.uint8, device="cuda")
+        try:
+            got = e.seed_check(gen=(5, 24576), rect=(-4, 5, -4, 5), max_height=40)
+        finally:
+            del full
+            torch.cuda.empty_cache()
+        assert got.stats["kernel_launches"][0] == got.stats["batches"]
+        assert len(want.candidates) and np.array_equal(got.candidates, want.candidates)
+        assert got.stats["reject_hist"] == want.stats["reject_hist"]
+        again = e.seed_check(gen=(5, 24576), rect=(-4, 5, -4, 5), max_height=40)
+        assert again.stats["kernel_launches"][0] == 6 * again.stats["batches"]
