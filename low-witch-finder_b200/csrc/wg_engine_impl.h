@@ -164,12 +164,25 @@ inline int job_class(uint64_t n_regions) {
     while (c < 3 && n_regions > kJobClassMax[c]) c++;
     return c;
 }
-// Regions per unit of a job: the engine's tuned value for its class, else the whole rect up to
-// 4,096 regions and 16,384-region tiles above.
-inline uint64_t job_window(const wg_engine *eng, uint64_t n_regions) {
+// Regions per unit of a job: the engine's tuned value for its class, else the whole rect up to 4,096 regions, and
+// above that tiles of 16,384 for the one-CTA kernel and of 2,048 for the fused kernels.
+inline uint64_t job_window(const wg_engine *eng, uint64_t n_regions, bool unit) {
     const uint64_t w = eng ? eng->tuned_win[job_class(n_regions)] : 0u;
-    if (!w) return n_regions <= 4096 ? n_regions : 16384u;
+    if (!w) return n_regions <= 4096 ? n_regions : (unit ? 16384u : 2048u);
     return n_regions < w ? n_regions : w;
+}
+// Whether a job takes the one-CTA kernel, and its tiles.  A tuned window (the tuner tries 2,048 to 16,384) may make
+// them smaller than that kernel pays for: 16 jobs of 256 seeds x 129 x 129 regions in windows of 512, 1,024 and
+// 2,048 took it 14.0, 11.2 and 7.0 ms, the fused kernels 6.4, 5.7 and 5.6.
+inline Tiling job_tiles(const wg_engine *eng, uint64_t rw, uint64_t rh, bool single_biome, bool f32, bool &unit) {
+    const uint64_t n = rw * rh, least = f32 ? kUnitCtaRegions : n <= 4096 ? kUnitCtaRegions64 : kUnitCtaTile64;
+    if (!single_biome && std::min(rw, rh) >= kUnitCtaStrip) {
+        const Tiling t = tile_rect(rw, rh, std::min(job_window(eng, n, true), kUnitCtaMax));
+        unit = t.win() >= least;
+        if (unit) return t;
+    }
+    unit = false;
+    return tile_rect(rw, rh, std::min<uint64_t>(job_window(eng, n, false), 4096));
 }
 
 // One phase-1 request over one rect (wg_engine.cu).

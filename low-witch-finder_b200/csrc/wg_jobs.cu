@@ -65,9 +65,7 @@ int sched_job_init(SchedJob &j, const wg_job &spec, const wg_engine *eng) {
     j.rw = (int)rw;
     j.rh = (int)rh;
     j.n_regions = rw * rh;
-    j.unit_cta = std::min(rw, rh) >= kUnitCtaStrip && !spec.opts.single_biome &&
-                 unit_rect(rw, rh, (!eng || eng->fp32_core) && job_small(j));
-    j.tiles = tile_rect(rw, rh, std::min<uint64_t>(job_window(eng, j.n_regions), j.unit_cta ? kUnitCtaMax : 4096));
+    j.tiles = job_tiles(eng, rw, rh, spec.opts.single_biome != 0, (!eng || eng->fp32_core) && job_small(j), j.unit_cta);
     if (spec.n_seeds > ~0ull / j.tiles.n_win) return WG_ERR_ARG;
     j.units = spec.n_seeds * j.tiles.n_win;
     try {

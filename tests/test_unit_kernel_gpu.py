@@ -160,3 +160,21 @@ def test_no_memory_for_the_lists(wg, engine):
         assert got.stats["reject_hist"] == want.stats["reject_hist"]
         again = e.seed_check(gen=(5, 24576), rect=(-4, 5, -4, 5), max_height=40)
         assert again.stats["kernel_launches"][0] == 6 * again.stats["batches"]
+
+
+@pytest.mark.parametrize("queue", [True, False])
+@pytest.mark.parametrize("window,unit", [(0, True), (512, False), (2048, False), (4096, False), (8192, True)])
+def test_tuned_windows_choose_the_kernel(engine, queue, window, unit):
+    """Jobs of more than 4,096 regions in tuned windows: small ones take the fused kernels, with the same results."""
+    jobs = [{"gen": (7, 900), "rect": (-64, 65, -64, 65), "max_height": 40}]
+    want, st0 = engine.seed_check_jobs(jobs)
+    engine.set_tuning([0, 0, 0, window])
+    engine.set_job_queue(queue)
+    try:
+        got, st = engine.seed_check_jobs(jobs)
+    finally:
+        engine.set_job_queue(True)
+        engine.set_tuning()
+    assert (st["kernel_launches"][1] == 0) == unit
+    assert len(want[0]) and np.array_equal(got[0], want[0])
+    assert st["reject_hist"] == st0["reject_hist"] and st["tier_hist"] == st0["tier_hist"]
