@@ -22,7 +22,14 @@
 using namespace wg;
 
 bool wg::few_units(double n_units, double n_regions, int sm_count, bool fp32) {
-    return n_units <= (fp32 ? 9.0 + n_regions / 67.0 : 6.5 + n_regions / 138.0) * sm_count;
+    static constexpr double kLine[2][4][2] = {   // [fp32][round - 1]: units per SM, and regions per further unit
+        {{8.6, 230.0}, {11.5, 160.0}, {18.0, 125.0}, {-45.0, 30.0}},
+        {{9.0, 180.0}, {12.0, 140.0}, {18.0, 88.0}, {-30.0, 30.0}}};
+    const double per_sm = n_units / sm_count;
+    const int round = (int)std::ceil(std::min(per_sm, 1e6) / kUnits);
+    if (round > 4) return false;
+    const double *l = kLine[fp32 ? 1 : 0][round > 0 ? round - 1 : 0];
+    return per_sm <= l[0] + n_regions / l[1];
 }
 
 // Whether a request's units take the one-CTA kernel, and its tiles.  Many regions per seed: yes, a
@@ -34,9 +41,12 @@ static Tiling request_tiles(uint64_t rw, uint64_t rh, uint64_t n_seeds, const wg
     const uint64_t n_regions = rw * rh, slots = (uint64_t)eng->sm_count * (uint64_t)eng->unit_per_sm[f32 ? 1 : 0];
     const uint64_t across = std::min(rw, rh);
     const bool strip = across < kUnitCtaStrip;
-    const Tiling large = tile_rect(rw, rh, kUnitCtaMax);   // FP64 units that are not whole seeds count as its tiles
-    const bool few = f32 || n_regions <= 4096 ? few_units((double)n_seeds, (double)n_regions, eng->sm_count, f32)
-                                              : few_units((double)n_seeds * (double)large.n_win, (double)large.win(), eng->sm_count, f32);
+    // FP64 units that are not whole seeds: their tiles of `large` against the fused kernels' 2,048-region windows
+    // (tiles of 4,000 regions: 20 an SM 1.23 and 1.38 ms, 24 1.45 and 1.43, 50 2.99 and 2.81).
+    const Tiling large = tile_rect(rw, rh, kUnitCtaMax);
+    const bool few = f32 || n_regions <= 4096
+                         ? few_units((double)n_seeds, (double)n_regions, eng->sm_count, f32)
+                         : (double)n_seeds * (double)large.n_win <= (6.5 + (double)large.win() / 200.0) * eng->sm_count;
     cta = !single_biome && (few || (strip ? n_regions >= kUnitCtaRegions : unit_rect(rw, rh, f32)));
     if (strip) cta = cta && (double)n_seeds * std::ceil((double)std::max(rw, rh) / 1023.0) <= 4.0 * (double)slots;
     // Long strips of one or two regions stay with the fused kernels, whose tiles may be longer: fewer table builds,

@@ -143,11 +143,13 @@ constexpr uint64_t kUnitCtaRegions64 = 3600, kUnitCtaTile64 = 4200;
 // takes the one-CTA kernel only for a few waves of them: 1,000 seeds x 20,000 x 1 3.11 ms and 1.66 fused, x
 // 10,000 x 3 2.44 and 2.36, x 10,000 x 4 2.88 and 2.97; one seed x 1,000,000 x 1 0.21 and 0.54.
 constexpr uint64_t kUnitCtaStrip = 4;
-// Whether so few units are better off with one CTA each (a wave of resident CTAs, 3 an SM, takes 40 to 120 us,
-// the fused kernels 125 to 450 whatever the number): 64 regions, 1,332 seeds 129 us and 129 fused, 1,776 148
-// and 136; 400 regions, 1,776 seeds 209 and 216, 2,664 286 and 271; 1,600 regions, 2,664 seeds 496 and 626,
-// 5,328 925 and 960.  FP64 units take longer: 64 regions, 888 seeds 107 and 131, 1,332 157 and 129; 400
-// regions, 1,332 seeds 217 and 217; 1,600 regions, 2,664 seeds 711 and 713, 3,552 916 and 780.
+// Whether so few units are better off with one CTA each.  The fused kernels put 16 in a CTA, so their time goes up
+// with every round of 16 units an SM (a second round shares the SM with the first, a third follows), the unit
+// kernel's with every unit; the line of each round lies where they meet.  Measured, FP32, unit kernel's time in
+// fused kernels' times at 444, 1,332, 2,331, 2,400, 4,620 and 4,842 units of 148 SMs: 81 regions 0.55, 0.93, 1.38, 1.32,
+// 1.95, 1.81; 400 regions 0.43, 0.83, 1.26, 1.09, 1.72, 1.49; 1,600 regions 0.28, 0.61, 0.97, 0.79, 1.29, 0.97; 2,500
+// regions 0.21, 0.49, 0.69, 0.61, 1.00, 0.77; FP64 0.54, 1.01, 1.45, 1.32, 2.08, 1.87; 0.47, 0.87, 1.32, 1.16, 1.77, 1.51;
+// 0.30, 0.68, 1.10, 0.86, 1.45, 1.10; 0.23, 0.55, 0.83, 0.68, 1.13, 0.89.
 bool few_units(double n_units, double n_regions, int sm_count, bool fp32);
 // Whether seeds of a rw x rh rect take the one-CTA kernel however many they are (rects kUnitCtaStrip across
 // and more); f32: its FP32 instance.

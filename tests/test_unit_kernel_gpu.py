@@ -121,7 +121,7 @@ def test_check_mode_takes_every_gate_again(engine, rect):
     assert st["rechecks"] == want
 
 
-@pytest.mark.parametrize("n,rect,unit", [(400, (0, 56, 0, 56), True), (6000, (0, 56, 0, 56), False),
+@pytest.mark.parametrize("n,rect,unit", [(400, (0, 56, 0, 56), True), (12000, (0, 56, 0, 56), False),
                                          (5000, (-30, 30, -30, 30), True), (200, (-2000, 2000, 0, 4), True),
                                          (1500, (-2000, 2000, 0, 4), False), (600, (-80, 80, -80, 80), True)])
 def test_fp64_routes_equal_the_fp32_core(engine, n, rect, unit):
