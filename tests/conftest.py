@@ -24,6 +24,21 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (runs on the B200 box)")
 
 
+# Tests of what needs the game data tables (phase 2, the finisher, the biome map): a library built without them
+# (no reference sources, NO_GAMEDATA=1) fails these.  They run last, so that a run which stops at its first
+# failure has run everything else.
+NEEDS_TABLES = ("test_biome_map_gpu.py", "test_finish_gpu.py", "test_phase2_gpu.py",
+                "test_hut_lookup_gpu.py::test_finish_command", "test_worker_gpu.py::test_worker_protocol",
+                "test_worker_gpu.py::test_single_shot_cli",
+                "test_worker_gpu.py::test_exact_hits_follow_the_phase2_ceiling",
+                "test_worker_gpu.py::test_self_test_passes",
+                "test_world_gpu.py::test_whole_world_worker_equals_reference_hit_list")
+
+
+def pytest_collection_modifyitems(items):
+    items.sort(key=lambda item: item.nodeid.split("/")[-1].startswith(NEEDS_TABLES))
+
+
 def load_package():
     name = "low_witch_finder_b200"
     if name in sys.modules:
