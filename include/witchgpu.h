@@ -61,7 +61,8 @@ typedef struct {
     double gpu_ms;                /* device time of the whole call, CUDA events on its stream */
     double wall_ms;               /* host wall time of the call */
     int64_t rechecks;             /* FP32 noise core: climate gate decisions re-taken in FP64 */
-    int64_t records;              /* seed units with climate survivors (tables the entrance kernel builds / 18) */
+    int64_t records;              /* seed units with climate survivors; batches of the list kernels count a unit's
+                                     survivors in records of at most 32, so a unit may count more than once */
 } wg_scan_stats;
 
 /* Create an engine on CUDA device `device`: context binding, stream, noise tables and work
@@ -77,7 +78,7 @@ const char *wg_engine_error(const wg_engine *e);
 
 /* Noise core of the phase-1 gates.
  *   WG_NOISE_FP32 (the default): the climate gates' samples (erosion tiers, temperature, ridge)
- *     in FP32 after an FP64 coordinate reduction, gates decided from the FP32 sums outside a
+ *     in FP32 after an FP64 or fixed-point coordinate reduction, gates decided from the FP32 sums outside a
  *     derived error band and re-taken in FP64 inside it, so every verdict equals the FP64 path's;
  *     wg_scan_stats.rechecks counts the re-takes.  The cave gates sample in FP64.
  *   WG_NOISE_FP64: every sample in FP64 in the reference's operation order.
@@ -466,7 +467,8 @@ typedef struct {
 int wg_engine_tune(wg_engine *e, wg_tune_report *report);
 
 /* Sets the job settings directly (e.g. from a saved tuning): window[4] regions per unit per class
- * (NULL or 0 = the default rule: a whole seed up to 4,096 regions, else 2,048), budget checks per
+ * (NULL or 0 = the default rule: a whole seed up to 4,096 regions, else 16,384 or, where those take the
+ * fused kernels, 2,048), budget checks per
  * slice (0 = 2^27). */
 int wg_engine_set_tuning(wg_engine *e, const uint32_t *window, uint64_t budget);
 

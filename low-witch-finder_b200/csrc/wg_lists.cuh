@@ -30,7 +30,6 @@ constexpr int kLLat = 5;                    // its lattice columns per axis (2.2
 constexpr int kLUnits = 4;                  // units of a warp in the erosion kernel
 constexpr int kEWarps = 4, kEThreads = 32 * kEWarps;   // erosion CTAs: four on an SM, 16 warps at 128 registers
 constexpr int kLList = 224;                 // tier-0 survivors a warp carries (a 9 x 9 group has 139 on average)
-constexpr int kLLate = 64;                  // and those past step 3 (28 on average)
 
 // Regions along one side of a tier-0 block of a tile `other` regions wide across it: kLBlock, or in a thin
 // tile as many as the lattice's columns hold (23 for one region; 9 of them left 23 lanes idle).
@@ -209,7 +208,7 @@ __global__ void __launch_bounds__(kEThreads, 4) erosion_kernel(const __grid_cons
     __syncthreads();
     const ClimateStep *const st = c_steps[large];
     const int my_k = lane & 7;
-    uint32_t tiers[3] = {0, 0, 0};   // rejections of tiers 0 to 2; the few others go straight to the histogram
+    uint32_t tiers[2] = {0, 0};   // rejections of tiers 0 and 1; the others go straight to the histogram
     uint32_t rechecks = 0;
     const uint32_t groups = (n_units + kLUnits - 1) / kLUnits;
     for (uint32_t grp = blockIdx.x * kEWarps + (uint32_t)warp; grp < groups; grp += gridDim.x * kEWarps) {
@@ -401,7 +400,7 @@ __global__ void __launch_bounds__(kEThreads, 4) erosion_kernel(const __grid_cons
         flush(n_out);
     }
     {
-        for (int t = 0; t < 3; t++) {
+        for (int t = 0; t < 2; t++) {
             const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, tiers[t]);
             if (lane == 0 && n) atomicAdd(&S.hist[P1_KINDS + st[1 + t].tier], n);
         }

@@ -3,10 +3,11 @@
 //
 // Phase 1 restates lysh_phase1_check_ex (engine/tools/lysh/src/phase1.c:130-200) per
 // (seed, region) and takes one of three forms, chosen by the number of units and of regions per seed
-// (wg_engine_impl.h): the unit kernel (wg_unit.cuh), one CTA for all of a tile; the list kernels
-// (wg_lists.cuh), breadth first over regions, one table set per warp and stage; or, for few units of few
-// regions, the FP64 core, SINGLE_BIOME and the check modes, three fused kernels by how often each stage is
-// reached (the last two also finish what the list kernels leave open):
+// (wg_engine_impl.h): the unit kernel (wg_unit.cuh), one CTA for all of a tile, for few units and for many
+// regions per seed; the list kernels (wg_lists.cuh), breadth first over regions, one table set per warp and
+// stage, for the default core's many units; or three fused kernels by how often each stage is reached, for
+// what lies between, the other cores' many units, SINGLE_BIOME and long strips (the last two also finish what
+// the list kernels leave open):
 //
 //   climate  every seed     builds the 18 climate Perlins of 16 units per CTA in shared
 //                           memory, runs the tiered erosion / temperature / ridge gates for

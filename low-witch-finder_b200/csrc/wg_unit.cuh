@@ -1,7 +1,7 @@
 // The unit kernel: all of phase 1 for one unit (a tile of one seed's regions) in one CTA.  Included by
 // wg_phase1.cu (it uses its constant tables and cave formulas).
 //
-// (SINGLE_BIOME requests, whose every region passes the climate stage, take the list kernels.)
+// (SINGLE_BIOME requests, whose every region passes the climate stage, take the fused kernels.)
 // For units of many regions, and for calls too small to fill the GPU with 16-unit CTAs.  The seed's
 // 18 climate tables and the entrance gate's 18 tables are built once per CTA, side by side (one
 // thread each), so nothing is rebuilt per record or per candidate; the ladder's other 36 are built
@@ -21,7 +21,7 @@
 // looked at only when it is full.  (With six, and the lists packed after each of the erosion steps 4-7:
 // 1.6e9 regions of one seed 55.9 -> 54.2 ms; barriers were 5 % of a CTA's time.)
 //
-// Measured against the three list kernels, which rebuilt a seed's tables for every 2,048-region
+// Measured against the three fused kernels, which rebuilt a seed's tables for every 2,048-region
 // window, record and candidate: one seed over the whole world (1.37e10 regions) 1,029 -> 425 ms, one seed x
 // 24,964 regions 538 -> 125 us (13 windows in one CTA before), x 400 regions 170 -> 93 us.  Of a large unit's
 // time the table builds take 2 %, the lattices 12 %, hut positions and tier 0 22 %, steps 2-3 16 %, the
