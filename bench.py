@@ -589,9 +589,16 @@ def noise_core_measure(wg, eng, args, step_device, stream, flush, headline: dict
 
 
 def run_reference(args) -> None:
-    """--impl reference: the reference's CPU scanner on the host cores, same metric."""
+    """--impl reference: the reference's CPU scanner (oracle/_ref, built from its sources) on the host cores, same
+    metric.  Without those sources there is no reference arm: the C restatement in oracle/ is not the reference."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import bind
+    if not os.path.exists(bind.REF_LIB):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref is not built: the reference's sources are "
+                                                              "not on this machine"}), flush=True)
         return
     n_sample = 1 << 18
     for _ in range(args.warmup):
