@@ -69,17 +69,27 @@ OPS_3D_SAMPLE = 56 + 192 + 24
 # x2), 24 gradient-component loads, 56 FP32 ops (3 offsets, 8 gradients x3, 3 fades x5, 7 lerps x2)
 OPS_3D_SAMPLE_F32 = 56 + 54 + 24 + 56
 OPS_REGION = 40              # java.util.Random placement (2 x nextInt(24)) + coordinates
+# The list kernels' sample from a table: fixed-point coordinates (6 integer ops, 2 conversions of 3) in place of
+# the FP64 reduction; and from four lattice columns: the same coordinates and 2 offsets, 4 loads of 16 bytes (x2),
+# 8 FMAs, 2 fades x5, 3 lerps x2, the running sum.
+OPS_Y0_SAMPLE_FIXED = 56 + 12 + 24 + 51 + 1
+OPS_LATTICE_SAMPLE = 12 + 4 + 8 + 8 + 10 + 6 + 1
+# One lattice column (5 lookups x4, 2 gradients of 3 loads, 6 FP32 ops, a store and its place), and the columns of
+# a 9 x 9 block: on average 4.18^2 and 4.22^2 in the two tables of tier 0.
+OPS_LATTICE_COLUMN = 20 + 6 + 6 + 8
+LATTICE_COLUMNS = 4.18 ** 2 + 4.22 ** 2
 # Tables that the first stage of the FP32 core builds per seed of 9 x 9 regions: 8 erosion for every seed, 4
-# temperature for the 75 % with a region past erosion, 6 ridge for 58 %, 12 of the cave gates for 53 %.
+# temperature for the 75 % with a region past erosion, 6 ridge for 58 %, 12 of the cave gates for 53 % (shares
+# measured on the headline's seeds; the funnel counts regions, not seeds).
 LIST_TABLES = 8 + 0.75 * 4 + 0.58 * 6 + 0.53 * 12
 # ncu counters of the erosion kernel, the longest of the step (2^20 seeds, one launch): DRAM read + write bytes
 # and pipe utilisation as fractions of peak.
-TRAFFIC = {"erosion_kernel": 8452608 + 831744, "source": "ncu --clock-control none -k regex:erosion_kernel -s 1 -c 1 "
+TRAFFIC = {"erosion_kernel": 8451840 + 3154944, "source": "ncu --clock-control none -k regex:erosion_kernel -s 1 -c 1 "
                                             "python bench.py --profile 1048576 --warmup 1 --steps 1"}
-PIPES = {"erosion_kernel": {"issue_active": 0.646, "alu": 0.550, "fma": 0.250, "shared_wavefronts": 0.688,
+PIPES = {"erosion_kernel": {"issue_active": 0.646, "alu": 0.543, "fma": 0.254, "shared_wavefronts": 0.689,
                             "warps_active": 0.221},
-         "gate_kernel": {"issue_active": 0.635, "alu": 0.679, "fma": 0.182, "shared_wavefronts": 0.732,
-                         "warps_active": 0.243},
+         "gate_kernel": {"issue_active": 0.635, "alu": 0.676, "fma": 0.183, "shared_wavefronts": 0.731,
+                         "warps_active": 0.244},
          "unit": "fraction of peak"}
 BYTES_PER_SEED_IN = 8        # the int64 seed read from HBM
 BYTES_PER_RECORD = 12        # (unit, offset, count) per seed with climate survivors
@@ -91,8 +101,13 @@ def climate_work(st: dict, n_seeds: int, n_regions: int, fp32: bool, lists: bool
     th = st["tier_hist"]
     rh = st["reject_hist"]
     y0 = sum((t + 2) * th[t] for t in range(7)) + 12 * rh[1] + 18 * (rh[2] + st["climate_survivors"])
-    ops = ((LIST_TABLES if lists else 18) * n_seeds * OPS_PERLIN_BUILD + y0 * (OPS_Y0_SAMPLE_F32 if fp32 else OPS_Y0_SAMPLE)
-           + n_seeds * n_regions * OPS_REGION)
+    if lists:   # tier 0 from lattice columns, the later gates from the tables; the cave samples (3 % more) left out
+        tier0 = 2 * n_seeds * n_regions
+        samples = (tier0 * OPS_LATTICE_SAMPLE + n_seeds * LATTICE_COLUMNS * OPS_LATTICE_COLUMN
+                   + (y0 - tier0) * OPS_Y0_SAMPLE_FIXED)
+    else:
+        samples = y0 * (OPS_Y0_SAMPLE_F32 if fp32 else OPS_Y0_SAMPLE)
+    ops = (LIST_TABLES if lists else 18) * n_seeds * OPS_PERLIN_BUILD + samples + n_seeds * n_regions * OPS_REGION
     nbytes = n_seeds * BYTES_PER_SEED_IN + st["climate_survivors"] * BYTES_PER_SURVIVOR
     return float(ops), float(nbytes)
 
@@ -791,9 +806,11 @@ def main() -> None:
                 "peak_source": f"nominal INT32/FP32 issue rate: {sm_count} SMs x 128 lanes x {max_mhz:.0f} MHz "
                                "(sm_max_mhz of MEASURED_PEAKS.json); the kernel is not HBM- or tensor-bound",
                 "ops_per_launch": ops_per_launch, "launch_ms": launch_ms,
-                "ops_model": (f"{LIST_TABLES if lists else 18:.1f} Perlin tables per seed x 7,160 lane-ops, per y=0 sample "
-                              f"{OPS_Y0_SAMPLE_F32 if fp32 else OPS_Y0_SAMPLE} lane-ops x the samples the funnel "
-                              "implies, 40 per (seed, region) placement"),
+                "ops_model": (f"{LIST_TABLES if lists else 18:.1f} Perlin tables per seed x 7,160 lane-ops, "
+                              + (f"{OPS_LATTICE_SAMPLE} per tier-0 sample from lattice columns and "
+                                 f"{OPS_Y0_SAMPLE_FIXED} per later y=0 sample" if lists else
+                                 f"{OPS_Y0_SAMPLE_F32 if fp32 else OPS_Y0_SAMPLE} per y=0 sample")
+                              + " x the samples the funnel implies, 40 per (seed, region) placement"),
                 "traffic": TRAFFIC["erosion_kernel"], "traffic_unit": "bytes per erosion_kernel launch",
                 "traffic_source": TRAFFIC["source"],
                 "ncu_pipes": PIPES,

@@ -16,7 +16,7 @@
 // which decides at 50 and 60.  The cave stages sample in FP64, as the entrance kernel does (in FP32, as
 // WG_NOISE_FP32_CAVES would have it, 2^24 seeds x 9 x 9 took 0.6 % less).  A warp owns its 32 tables (one byte column per lane, 32-byte
 // rows) and waits for no other warp, so the warps of an SM drift apart and one's build fills the issue
-// slots another's sampling leaves free.  Measured on 2^24 seeds x 9 x 9: these six kernels 174 ms and the
+// slots another's sampling leaves free.  Measured on 2^24 seeds x 9 x 9: these six kernels 175 ms and the
 // entrance kernel's rest 6; the fused climate kernel 160 and the entrance kernel 74.
 //
 // Tier 0 takes its samples from lattice columns as the unit kernel does (wg_unit.cuh): a 9 x 9 block

@@ -22,10 +22,11 @@
 // 1.6e9 regions of one seed 55.9 -> 54.2 ms; barriers were 5 % of a CTA's time.)
 //
 // Measured against the three fused kernels, which rebuilt a seed's tables for every 2,048-region
-// window, record and candidate: one seed over the whole world (1.37e10 regions) 1,029 -> 425 ms, one seed x
-// 24,964 regions 538 -> 125 us (13 windows in one CTA before), x 400 regions 170 -> 93 us.  Of a large unit's
+// window, record and candidate (whole calls): one seed over the whole world (1.37e10 regions) 939 -> 425 ms, one
+// seed x 24,964 regions 529 -> 105 us (13 windows in one CTA before), x 400 regions 170 -> 82 us.  Of a large unit's
 // time the table builds take 2 %, the lattices 12 %, hut positions and tier 0 22 %, steps 2-3 16 %, the
-// later gates 21 %, barriers 8 %, the entrance gate 12 %, the ladder 6 %.
+// later gates 21 %, barriers 8 %, the entrance gate 12 % (its first test then in FP32; in FP64 a large unit takes
+// 2 % longer), the ladder 6 %.
 #pragma once
 
 constexpr int kUThreads = 256;
